@@ -77,9 +77,13 @@ _SIGNATURES = {
         "ps_rms_norm_pair": [_P, _I, _I, _P, _P, _F, _P, _P, _I, _P],
         "ps_layernorm": [_P, _P, _I, _I, _P, _P, _F, _I, _P, _I, _P],
         "ps_gemm_simt": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "ps_gemm_f32_rows": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "ps_kv_append": [_P, _P, _I, _P, _P, _P, _I, _P, _P, _L, _I, _I, _I, _I, _I, _P],
         "ps_paged_attention_simt": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P,
                                     _I, _I, _I, _P],
+        "ps_prompt_attention_f32": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P,
+                                    _I, _P],
+        "ps_token_attention_f32": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _I, _P],
         "ps_rotary_cache_write": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _P, _L, _I, _I, _I, _I, _I,
                                   _I, _P],
         "ps_token_shift_mix": [_P, _I, _P, _I, _P, _L, _I, _P, _P, _P, _P, _L, _I, _I, _I, _I, _P],
@@ -372,6 +376,32 @@ class Ops:
                "gemm_simt")
         return out
 
+    F32_FEW_ROWS = 16             # most rows of a float32 product that run on the kernel that streams the weights once
+
+    def linear_f32_rows(self, a, w, bias, out, act=None, accumulate=False):
+        """The float32 product of at most F32_FEW_ROWS rows (csrc/gemm_simt.cu: gemm_f32_rows_kernel)."""
+        M, K = a.shape
+        N = w.shape[0]
+        if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
+            raise KernelError("linear_f32_rows: shapes do not match")
+        for name, tensor in (("a", a), ("w", w), ("out", out)):
+            _require(tensor, name, torch.float32)
+            if tensor.stride(1) != 1:
+                raise KernelError("linear_f32_rows: innermost stride must be 1")
+        if bias is not None:
+            _require(bias, "bias", torch.float32)
+            if bias.numel() != N:
+                raise KernelError("linear_f32_rows: bias length")
+        self.launches += 1
+        _check(self.core.ps_gemm_f32_rows(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(bias), _ptr(out), out.stride(0),
+                                          M, N, K, _ACT_CODE[act], int(accumulate), _stream()), "gemm_f32_rows")
+        return out
+
+    def _f32_rows_ok(self, a, w, out):
+        return (a.shape[0] <= self.F32_FEW_ROWS and a.shape[1] % 4 == 0 and a.dtype == w.dtype == out.dtype == torch.float32
+                and a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1 and a.stride(0) % 4 == 0
+                and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
     def linear_skinny(self, a, w, bias, out, act=None, accumulate=False, kv=None):
         """Weight-streaming product for at most 64 rows of ``a`` (bfloat16 operands).  ``kv`` =
         (ctx, layer, q_width, kv_width, head_dim) sends the key and value columns of a packed q|k|v
@@ -641,6 +671,8 @@ class Ops:
                 return self.linear_skinny_fused(a, w, bias, out, act, accumulate)
             a = a.materialize()
         if self.dtype == torch.float32:
+            if self._f32_rows_ok(a, w, out):
+                return self.linear_f32_rows(a, w, bias, out, act, accumulate)
             return self.linear_simt(a, w, bias, out, act, accumulate)
         from pagedserve_b200.kernels import tensorcore
 
