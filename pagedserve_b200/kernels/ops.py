@@ -728,6 +728,42 @@ class Ops:
         return out
 
     @staticmethod
+    def attention_f32_ok(q, out, k_pool, v_pool, page_stride, head_dim):
+        """Whether the float32 kernels of csrc/attention_f32.cu take these rows: 16-byte pieces, head sizes up to 128."""
+        return (q.dtype == out.dtype == k_pool.dtype == torch.float32 and head_dim % 4 == 0 and head_dim <= 128
+                and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0 and page_stride % 4 == 0
+                and all(t.data_ptr() % 16 == 0 for t in (q, out, k_pool, v_pool)))
+
+    def attention_f32(self, q, out, ctx, layer, n_heads, n_kv_heads, head_dim, window, scale, softcap=None, sink=None,
+                      all_values=False):
+        """The step's attention in float32: short entries token by token, prompt portions in blocks of 64 queries (the
+        step's flat batch holds the short entries first).  Arguments as in :meth:`paged_attention_simt`."""
+        for name, tensor in (("q", q), ("out", out)):
+            _require(tensor, name, torch.float32)
+            if tensor.stride(1) != 1:
+                raise KernelError("attention: innermost stride must be 1")
+        if sink is not None:
+            _require(sink, "sink", torch.float32)
+            if sink.numel() != n_heads:
+                raise KernelError("attention: one sink per query head")
+        pools = (_ptr(layer.k_pool), _ptr(layer.v_pool), layer.page_stride)
+        table = (_ptr(layer.block_table), layer.block_table.stride(0))
+        rest = (n_heads, n_kv_heads, head_dim, layer.page_size, window or 0, scale, float(softcap or 0.0), _ptr(sink),
+                1 if all_values else 0, _stream())
+        if ctx.num_short_tokens:
+            self.launches += 1
+            _check(self.core.ps_token_attention_f32(_ptr(q), q.stride(0), _ptr(out), out.stride(0), *pools, _ptr(ctx.token_slot),
+                                                    _ptr(ctx.positions), *table, ctx.num_short_tokens, *rest),
+                   "token_attention_f32")
+        long_items = ctx.num_items - ctx.num_short_items
+        if long_items:
+            self.launches += 1
+            _check(self.core.ps_prompt_attention_f32(_ptr(q), q.stride(0), _ptr(out), out.stride(0), *pools, _ptr(ctx.q_start),
+                                                     _ptr(ctx.kv_len), *table, _ptr(ctx.item_slot), ctx.num_short_items,
+                                                     long_items, ctx.num_long_blocks, *rest), "prompt_attention_f32")
+        return out
+
+    @staticmethod
     def attention_chunk_keys(head_dim, page_size):
         """Keys per shared-memory chunk of the split attention kernel (mirrors the CUDA side)."""
         keys = 128 if head_dim <= 64 else 64 if head_dim <= 128 else 32
@@ -958,8 +994,13 @@ class Ops:
 
         if self.dtype == torch.float32 or head_dim % 16 != 0 or head_dim > 256:
             # the CUDA-core kernel takes every head size (up to 1,024); the tensor-core kernels want multiples of 16
-            # up to 256
+            # up to 256, the float32 ones multiples of 4 up to 128
             every = out if mix is None else self.empty((q.shape[0], n_heads * n_kv_heads * head_dim), self.dtype, q.device)
+            if (self.attention_f32_ok(q, every, layer.k_pool, layer.v_pool, layer.page_stride, head_dim)
+                    and ctx.num_long_blocks <= 65535):
+                self.attention_f32(q, every, ctx, layer, n_heads, n_kv_heads, head_dim, window, scale, softcap, sink,
+                                   all_values=mix is not None)
+                return out if mix is None else self.head_mix(every, mix, out, n_heads, n_kv_heads, head_dim)
             self.paged_attention_simt(q, every, layer.k_pool, layer.v_pool, layer.page_stride, ctx.token_slot,
                                       ctx.positions, layer.block_table, n_heads, n_kv_heads, head_dim, layer.page_size,
                                       window, scale, softcap, sink, all_values=mix is not None)

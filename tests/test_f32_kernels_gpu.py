@@ -74,3 +74,106 @@ def test_tiles(M, N, K):
         assert float((out.cpu().double() - want).abs().max()) < sum_bound(K) * 8 * float(want.abs().max())
         outs.append(out)
     assert torch.equal(outs[0], outs[1])                         # however the rows lie: the same sums in the same order
+
+
+class Step:
+    """Requests with pages in no order, each with some keys cached and some queries at its end; the short ones come first."""
+
+    def __init__(self, entries, n_heads, n_kv_heads, head_dim, page, seed):
+        g = torch.Generator().manual_seed(seed)
+        entries = sorted(entries, key=lambda entry: entry[1] >= 16)
+        self.lengths = [length for length, _ in entries]
+        pages = [-(-length // page) for length in self.lengths]
+        order = torch.randperm(sum(pages) + 2, generator=g).tolist()
+        table = torch.full((len(entries) + 1, max(pages)), -1, dtype=torch.int32)
+        rows = torch.randperm(len(entries) + 1, generator=g)[:len(entries)]
+        pool = torch.full((sum(pages) + 2, 2, n_kv_heads, page, head_dim), float("nan"))
+        self.k = [torch.randn(length, n_kv_heads, head_dim, generator=g) for length in self.lengths]
+        self.v = [torch.randn(length, n_kv_heads, head_dim, generator=g) for length in self.lengths]
+        for r, count in enumerate(pages):
+            for i in range(count):
+                p = order.pop()
+                table[rows[r], i] = p
+                here = self.k[r][i * page:(i + 1) * page], self.v[r][i * page:(i + 1) * page]
+                for which in (0, 1):
+                    pool[p, which, :, :len(here[which])] = here[which].transpose(0, 1)
+        pool = pool.to(DEV)
+        counts = [count for _, count in entries]
+        self.q = [torch.randn(count, n_heads, head_dim, generator=g) for count in counts]
+        as_ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+        starts = [sum(counts[:i]) for i in range(len(counts) + 1)]
+        short = sum(count < 16 for count in counts)
+        self.ctx = SimpleNamespace(
+            num_items=len(counts), num_short_items=short, num_short_tokens=starts[short],
+            num_long_blocks=sum(-(-count // 64) for count in counts[short:]) + 2, q_start=as_ints(starts),
+            kv_len=as_ints(self.lengths), item_slot=as_ints(rows.tolist()),
+            token_slot=as_ints([int(rows[r]) for r, count in enumerate(counts) for _ in range(count)]),
+            positions=as_ints([length - count + i for length, count in entries for i in range(count)]))
+        self.layer = SimpleNamespace(k_pool=pool[:, 0], v_pool=pool[:, 1], page_stride=pool.stride(0), page_size=page,
+                                     block_table=table.to(DEV))
+
+
+def plain(step, scale, window, softcap, sink, all_values):
+    out = []
+    for q, k, v in zip(step.q, step.k, step.v):
+        q, k, v = q.double(), k.double(), v.double()
+        H, G = q.shape[1], k.shape[1]
+        at = torch.arange(len(k) - len(q), len(k))[:, None]
+        key = torch.arange(len(k))[None]
+        seen = key <= at
+        if window > 0:
+            seen &= at - key < window
+        elif window < 0:
+            seen &= at // -window == key // -window
+        for_heads = []
+        for h in range(H):
+            s = q[:, h] @ k[:, h // (H // G)].T * scale
+            if softcap:
+                s = softcap * torch.tanh(s / softcap)
+            s = s.masked_fill(~seen, float("-inf"))
+            if sink is not None:
+                s = torch.cat([s, sink[h].double().expand(len(q), 1)], 1)
+            p = torch.softmax(s, -1)[:, :len(k)]
+            for_heads += [p @ v[:, other] for other in (range(G) if all_values else [h // (H // G)])]
+        out.append(torch.cat(for_heads, -1))
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("n_heads,n_kv_heads,head_dim", [(3, 3, 64), (4, 2, 128), (4, 1, 36), (2, 2, 4), (2, 1, 100)])
+@pytest.mark.parametrize("window,softcap,with_sink,all_values", [(0, 0.0, False, False), (19, 5.0, True, False), (-40, 0.0, True, True),
+                                                                 (64, 0.0, False, False)])
+def test_attention(n_heads, n_kv_heads, head_dim, window, softcap, with_sink, all_values):
+    entries = [(1, 1), (700, 1), (33, 5), (16, 16), (64, 64), (129, 65), (200, 17), (331, 200), (65, 1)]
+    step = Step(entries, n_heads, n_kv_heads, head_dim, page=8, seed=head_dim + n_heads)
+    ops, scale = ops_for(), head_dim ** -0.5
+    sink = torch.randn(n_heads, generator=torch.Generator().manual_seed(3)) if with_sink else None
+    q = torch.cat([rows.reshape(len(rows), -1) for rows in step.q]).to(DEV)
+    columns = n_heads * (n_kv_heads if all_values else 1) * head_dim
+    out = torch.full((len(q), columns), float("nan"), device=DEV)
+    layer = step.layer
+    assert ops.attention_f32_ok(q, out, layer.k_pool, layer.v_pool, layer.page_stride, head_dim)
+    ops.attention_f32(q, out, step.ctx, layer, n_heads, n_kv_heads, head_dim, window, scale, softcap,
+                      None if sink is None else sink.to(DEV), all_values)
+    want = plain(step, scale, window, softcap, sink, all_values)
+    # scores of order one: a score is off by at most (head_dim + 3) 2^-24 of a few, the sums of up to 700 weights by 700 * 2^-24
+    assert float((out.cpu().double() - want).abs().max()) < 1e-5
+    # the general kernel, which these calls ran on before
+    general = torch.full_like(out, float("nan"))
+    ops.paged_attention_simt(q, general, layer.k_pool, layer.v_pool, layer.page_stride, step.ctx.token_slot, step.ctx.positions,
+                             layer.block_table, n_heads, n_kv_heads, head_dim, layer.page_size, window, scale, softcap,
+                             None if sink is None else sink.to(DEV), all_values=all_values)
+    assert float((out - general).abs().max()) < 2e-5
+
+
+def test_attention_keeps_a_later_infinity_out():
+    """An infinity in a later token's key and value stays out of the earlier queries of its block of queries."""
+    step = Step([(80, 80)], 2, 2, 64, page=16, seed=5)
+    ops, layer = ops_for(), step.layer
+    q = step.q[0].reshape(80, -1).to(DEV)
+    clean, out = torch.empty(80, 128, device=DEV), torch.empty(80, 128, device=DEV)
+    ops.attention_f32(q, clean, step.ctx, layer, 2, 2, 64, 0, 0.125)
+    page, place = int(layer.block_table[int(step.ctx.item_slot[0]), 70 // 16]), 70 % 16
+    layer.v_pool[page, :, place] = float("inf")
+    layer.k_pool[page, :, place] = float("nan")
+    ops.attention_f32(q, out, step.ctx, layer, 2, 2, 64, 0, 0.125)
+    assert torch.equal(out[:70], clean[:70]) and bool(torch.isnan(out[70:]).all())
