@@ -307,8 +307,8 @@ inline bool ensure_dynamic_smem(const void* kernel, size_t smem, size_t (&raised
 // Launch with the programmatic-stream-serialization attribute (kept when a stream is captured into a
 // CUDA graph, where it becomes a programmatic dependency edge).
 template <typename... KArgs, typename... Args>
-inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                              int cluster_z, Args... args) {
+inline int launch_pdl_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                               dim3 cluster, Args... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
@@ -325,17 +325,24 @@ inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
         attribute[count].val.programmaticStreamSerializationAllowed = 1;
         ++count;
     }
-    if (cluster_z > 1) {             // thread-block clusters of (1, 1, cluster_z) CTAs
+    if (cluster.x * cluster.y * cluster.z > 1) {
         attribute[count].id = cudaLaunchAttributeClusterDimension;
-        attribute[count].val.clusterDim.x = 1;
-        attribute[count].val.clusterDim.y = 1;
-        attribute[count].val.clusterDim.z = (unsigned)cluster_z;
+        attribute[count].val.clusterDim.x = cluster.x;
+        attribute[count].val.clusterDim.y = cluster.y;
+        attribute[count].val.clusterDim.z = cluster.z;
         ++count;
     }
     config.attrs = attribute;
     config.numAttrs = count;
     cudaError_t e = cudaLaunchKernelEx(&config, kernel, KArgs(args)...);
     return e == cudaSuccess ? PS_OK : PS_ERR_LAUNCH;
+}
+
+// thread-block clusters of (1, 1, cluster_z) CTAs
+template <typename... KArgs, typename... Args>
+inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              int cluster_z, Args... args) {
+    return launch_pdl_clusters(kernel, grid, block, smem, stream, dim3(1, 1, (unsigned)cluster_z), args...);
 }
 
 template <typename... KArgs, typename... Args>

@@ -31,6 +31,7 @@ namespace tc {
 constexpr int BM = 128;
 constexpr int BK = 64;                 // bf16 elements per k-block = 128 bytes
 constexpr int THREADS = 320;           // TMA warp, MMA warp, two teams of four epilogue warps
+constexpr int PAIR_256 = 512;          // in place of a tile's columns: tiles of 256 x 256 on pairs of CTAs
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -58,14 +59,25 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     return t;
 }
 constexpr uint64_t WAIT_LIMIT_NS = 200ull * 1000 * 1000;      // 0.2 s: far beyond any legitimate wait here
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {      // arrivals of other CTAs too
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
 // false: the wait ran out, or another role of this CTA gave up (abort flag set)
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
+    auto done = [&]() { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+    if (done()) return true;
     const uint64_t start = global_timer_ns();
     while (true) {
 #pragma unroll 1
         for (int spin = 0; spin < 64; ++spin)
-            if (mbar_try_wait(bar, parity)) return true;
+            if (done()) return true;
         if (*abort_flag) return false;
         if (global_timer_ns() - start > WAIT_LIMIT_NS) { *abort_flag = 1; return false; }
     }
@@ -95,6 +107,33 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                  ::"r"(smem_u32(bar)) : "memory");
+}
+// The same for a pair of CTAs (PAIR below): one MMA of 256 rows, of which each CTA holds 128 with their accumulators and half of
+// the columns' operand; the first CTA of the pair issues.
+__device__ __forceinline__ uint32_t in_first_cta(const void* p) {         // the same place in the first CTA's shared memory
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(smem_u32(p)));
+    return remote;
+}
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                               uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {         // arrives at this place in both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
@@ -147,9 +186,10 @@ struct ColumnGroups {
     int out_cols;
 };
 
-template <int BN> struct Config {
-    static constexpr int STAGE_BYTES = BM * BK * 2 + BN * BK * 2;
-    static constexpr int STAGES = BN > 128 ? 4 : (BN >= 96 ? 5 : 6);
+template <int BN, bool PAIR> struct Config {
+    static constexpr int W_ROWS = PAIR ? BN / 2 : BN;              // rows of W in a CTA's stage
+    static constexpr int STAGE_BYTES = BM * BK * 2 + W_ROWS * BK * 2;
+    static constexpr int STAGES = PAIR ? 6 : BN > 128 ? 4 : (BN >= 96 ? 5 : 6);
     // two accumulators of BN columns; an allocation is a power of two of at least 32 columns
     static constexpr int TMEM_COLS = 2 * BN <= 32 ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));
     // Results on their way out: buffers of 128 rows x 128 bytes, STAGING_BUFS for each of the two epilogue teams,
@@ -163,14 +203,22 @@ template <int BN> struct Config {
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
 };
 
-template <int BN, typename TOut, bool TMA_OUT>
+// PAIR: clusters of two CTAs (2, 1, 1) that work on one tile of 256 rows x BN columns together (tcgen05 cta_group::2): a CTA
+// fetches its 128 rows of A and half of the tile's rows of W and keeps the accumulators of its rows; the first CTA issues
+// the MMAs, its barriers count the copies of both, and its commits arrive in both.  Per output a third fewer bytes enter
+// shared memory than with 128 x 256 tiles, which are bound by that memory's bandwidth (48 KB in and as much read per k-block
+// of 512 clocks): 5,824 x 4,800 x 1,600 69.7 -> 63.8 us (1.40 PFLOP/s), 4,099 x 8,192 x 2,048 109 -> 101.
+template <int BN, typename TOut, bool TMA_OUT, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_out, const float* __restrict__ bias, TOut* __restrict__ out,
                int ldo, int M, int N, int K, int act, int accumulate, int* __restrict__ status, KvScatter kv,
                TileExperts ex, ColumnGroups cg) {
-    using Cfg = Config<BN>;
+    using Cfg = Config<BN, PAIR>;
     constexpr int STAGES = Cfg::STAGES;
+    constexpr int TILE_M = PAIR ? 2 * BM : BM;
+    const int rank = PAIR ? (int)blockIdx.x & 1 : 0;               // which CTA of the pair
+    const int first_tile = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, tile_step = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* staging = tiles + (size_t)STAGES * Cfg::STAGE_BYTES;              // [2][128 rows][128 bytes]
@@ -185,24 +233,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // Set-up (barriers, tensor memory) and the first weight tiles do not depend on the kernel before this one:
     // they happen before the wait and overlap its end.
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_n = (N + BN - 1) / BN, tiles_m = (M + BM - 1) / BM;
-    const int per_m = (cg.groups > 0 ? cg.groups : 1) * tiles_n;        // tiles of one block of 128 rows
+    const int tiles_n = (N + BN - 1) / BN, tiles_m = (M + TILE_M - 1) / TILE_M;
+    const int per_m = (cg.groups > 0 ? cg.groups : 1) * tiles_n;        // tiles of one block of rows
     const int num_tiles = tiles_m * per_m;
     const int num_kb = (K + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 256); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], PAIR ? 512 : 256); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();                        // the other CTA's barriers are there too
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -211,20 +266,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (lane == 0) {
             // the weight tiles of the first stages (of this CTA's first tile) go out before the wait
             // (not where tiles choose their weights by a table that a kernel of this step has just written)
-            const uint32_t early = ((int)blockIdx.x < num_tiles && !ex.tile_expert && !cg.groups)
+            const uint32_t early = (first_tile < num_tiles && !ex.tile_expert && !cg.groups)
                                        ? (uint32_t)min(STAGES, num_kb) : 0u;
+            // (a pair's copies all count at the first CTA's barrier, which expects the bytes of both)
+            auto expect = [&](int s) {
+                if (!PAIR) mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
+                else if (rank == 0) mbar_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
+            };
+            auto load = [&](void* dst, const CUtensorMap* map, int x, int y, int s) {
+                if constexpr (PAIR) tma_load_2d_pair(dst, map, x, y, in_first_cta(&full[s]));
+                else tma_load_2d(dst, map, x, y, &full[s]);
+            };
             for (uint32_t kb = 0; kb < early; ++kb) {
-                const int n0 = ((int)blockIdx.x % tiles_n) * BN;
-                mbar_expect_tx(&full[kb], Cfg::STAGE_BYTES);
-                tma_load_2d(tiles + (size_t)kb * Cfg::STAGE_BYTES + BM * BK * 2, &map_w, (int)kb * BK, n0, &full[kb]);
+                const int n0 = (first_tile % tiles_n) * BN + rank * Cfg::W_ROWS;
+                expect(kb);
+                load(tiles + (size_t)kb * Cfg::STAGE_BYTES + BM * BK * 2, &map_w, (int)kb * BK, n0, kb);
             }
             pdl_prologue();
             const int* tile_expert = pdl_fresh(ex.tile_expert);
             uint32_t it = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const int m0 = (tile / per_m) * BM;
-                int n0 = (tile % tiles_n) * BN, k0 = 0, a_k0 = 0;
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
+                const int m0 = (tile / per_m) * TILE_M + rank * BM;
+                int n0 = (tile % tiles_n) * BN + rank * Cfg::W_ROWS, k0 = 0, a_k0 = 0;
                 if (cg.groups) {                                 // this tile's group: its columns of A, its rows of W
                     const int group = (tile % per_m) / tiles_n;
                     a_k0 = group * cg.a_cols;
@@ -241,11 +305,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     unsigned char* a_dst = tiles + (size_t)s * Cfg::STAGE_BYTES;
                     if (it >= early) {
                         if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; atomicExch(status, 11); break; }
-                        mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
-                        tma_load_2d(a_dst + BM * BK * 2, &map_w, k0 + kb * BK, n0, &full[s]);
+                        expect(s);
+                        load(a_dst + BM * BK * 2, &map_w, k0 + kb * BK, n0, s);
                     }
-                    tma_load_2d(a_dst, &map_a, a_k0 + kb * BK, m0, &full[s]);
+                    load(a_dst, &map_a, a_k0 + kb * BK, m0, s);
                 }
+            }
+            // a pair's CTA stays until the first CTA's last commits have arrived in its shared memory
+            if constexpr (PAIR) {
+                for (int n = 0; n < STAGES && ok; ++n, ++it)
+                    if (!mbar_wait(&empty[it % STAGES], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; atomicExch(status, 15); }
             }
         } else {
             pdl_prologue();
@@ -253,17 +322,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp == 1) {
         pdl_prologue();
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            // instruction descriptor: D = f32, A = B = bf16, both K-major, N = BN, M = 128
+        if (lane == 0 && rank == 0) {
+            // instruction descriptor: D = f32, A = B = bf16, both K-major, N = BN, M = 128 (256 for a pair)
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                                       ((uint32_t)(BM >> 4) << 24);
+                                       ((uint32_t)(TILE_M >> 4) << 24);
             uint32_t it = 0, local = 0;
             bool ok = true;
             const int* tile_expert = pdl_fresh(ex.tile_expert);
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local) {
                 if (tile_expert && tile_expert[tile / tiles_n] < 0) { --local; continue; }     // a tile of no expert
                 const int buf = local & 1;
-                if (!mbar_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag)) { ok = false; atomicExch(status, 12); break; }
+                if (!mbar_wait<PAIR>(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag)) { ok = false; atomicExch(status, 12); break; }
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
@@ -274,10 +343,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const uint64_t desc_a = umma_desc(a_addr), desc_b = umma_desc(a_addr + BM * BK * 2);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k)      // 16 bf16 = 32 bytes = 2 units of the address field
-                        umma_bf16(tmem_d, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) ? 1u : 0u);
-                    umma_commit(&empty[s]);                 // stage free once these MMAs have read it
+                        if constexpr (PAIR) umma_bf16_pair(tmem_d, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) ? 1u : 0u);
+                        else umma_bf16(tmem_d, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) ? 1u : 0u);
+                    if constexpr (PAIR) umma_commit_pair(&empty[s]);
+                    else umma_commit(&empty[s]);            // stage free once these MMAs have read it
                 }
-                if (ok) umma_commit(&acc_full[buf]);        // accumulator complete
+                if (ok) {                                   // accumulator complete
+                    if constexpr (PAIR) umma_commit_pair(&acc_full[buf]);
+                    else umma_commit(&acc_full[buf]);
+                }
             }
         }
     } else {
@@ -285,13 +359,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         pdl_prologue();
         const int quarter = warp & 3;                       // TMEM lanes 32*quarter .. +31
         const int team = (warp - 2) >> 2;                   // which column groups this warp takes
+        auto drained = [&](int buf) {                       // tell the MMA's issuer that this thread has read its part
+            if constexpr (PAIR) mbar_arrive_remote(in_first_cta(&acc_empty[buf]));
+            else mbar_arrive(&acc_empty[buf]);
+        };
         uint32_t local = 0;
         [[maybe_unused]] uint32_t chunk = 0;                // column groups this team has sent out so far
         bool ok = true;
         const int* tile_expert = pdl_fresh(ex.tile_expert);
-        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
+        for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local) {
             if (tile_expert && tile_expert[tile / tiles_n] < 0) { --local; continue; }         // a tile of no expert
-            const int m0 = (tile / per_m) * BM, n0 = (tile % tiles_n) * BN;
+            const int m0 = (tile / per_m) * TILE_M + rank * BM, n0 = (tile % tiles_n) * BN;
             const int out_col0 = cg.groups ? ((tile % per_m) / tiles_n) * cg.out_cols : 0;     // the group's columns
             const int buf = local & 1;
             // a q|k|v product whose key and value columns go straight into the pages: where this row's go
@@ -344,7 +422,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                         if (c + 2 * COLS >= BN && half == COLS / 32 - 1) {   // this team's last read of the accumulator
                             tc_fence_before();
-                            mbar_arrive(&acc_empty[buf]);
+                            drained(buf);
                             released = true;
                         }
                         const int n = n0 + c + 32 * half;
@@ -406,7 +484,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (leader) {
                         // (key and value columns of a scattering q|k|v product were written by the rows themselves;
                         // the query width is a multiple of the 64-column group, so a group is all one or the other)
-                        if (n0 + c < N && !(sizeof(TOut) == 2 && kv.k_pool && n0 + c >= kv.q_width)) {
+                        if (n0 + c < N && (!PAIR || m0 < M) && !(sizeof(TOut) == 2 && kv.k_pool && n0 + c >= kv.q_width)) {
                             if (accumulate & PS_ACCUMULATE) tma_reduce_add_2d(&map_out, stage_buf, n0 + c, m0);
                             else tma_store_2d(&map_out, stage_buf, n0 + c, m0);
                         }
@@ -415,7 +493,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 if (!released) {                                          // a team without a column group (BN < 2 groups)
                     tc_fence_before();
-                    mbar_arrive(&acc_empty[buf]);
+                    drained(buf);
                 }
                 continue;
             }
@@ -427,7 +505,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (c + 64 >= BN) {                          // this team's last read: hand TMEM back
                     tc_fence_before();
-                    mbar_arrive(&acc_empty[buf]);
+                    drained(buf);
                 }
                 const int n = n0 + c;
                 if (m < M && n < N) {
@@ -504,10 +582,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (TMA_OUT && (warp == 2 || warp == 6) && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();     // the other CTA is done with this one's shared memory, barriers and accumulators
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                     ::"r"(tmem_base), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
+        if constexpr (PAIR)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;"
+                         ::"r"(tmem_base), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                         ::"r"(tmem_base), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
     }
 }
 
@@ -567,20 +650,23 @@ static int sm_count() {
     return count;
 }
 
-template <int BN, typename TOut, bool TMA_OUT>
+template <int BN, typename TOut, bool TMA_OUT, bool PAIR>
 int launch_kernel(const CUtensorMap& map_a, const CUtensorMap& map_w, const CUtensorMap& map_out, const float* bias,
                   void* out, int ldo, int M, int N, int K, int act, int accumulate, int* status, const KvScatter& kv,
                   cudaStream_t stream, const TileExperts& ex, const ColumnGroups& cg) {
-    auto kernel = gemm_tc_kernel<BN, TOut, TMA_OUT>;
+    auto kernel = gemm_tc_kernel<BN, TOut, TMA_OUT, PAIR>;
+    using Cfg = Config<BN, PAIR>;
     static size_t raised[MAX_DEVICES] = {0};
-    if (!ensure_dynamic_smem((const void*)kernel, (size_t)Config<BN>::SMEM, raised)) return PS_ERR_LAUNCH;
-    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * (cg.groups > 0 ? cg.groups : 1);
-    const int grid = tiles < sm_count() ? tiles : sm_count();
-    return launch_pdl(kernel, dim3(grid), dim3(THREADS), Config<BN>::SMEM, stream, map_a, map_w, map_out, bias,
+    if (!ensure_dynamic_smem((const void*)kernel, (size_t)Cfg::SMEM, raised)) return PS_ERR_LAUNCH;
+    constexpr int TILE_M = PAIR ? 2 * BM : BM;
+    const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + BN - 1) / BN) * (cg.groups > 0 ? cg.groups : 1);
+    const int most = PAIR ? sm_count() / 2 : sm_count();
+    const int grid = tiles < most ? tiles : most;
+    return launch_pdl_clusters(kernel, dim3(PAIR ? 2 * grid : grid), dim3(THREADS), Cfg::SMEM, stream, dim3(PAIR ? 2 : 1), map_a, map_w, map_out, bias,
                       (TOut*)out, ldo, M, N, K, act, accumulate, status, kv, ex, cg);
 }
 
-template <int BN, typename TOut>
+template <int BN, typename TOut, bool PAIR = false>
 int launch(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo, int M, int N, int K,
            int act, int accumulate, int* status, const KvScatter& kv, cudaStream_t stream, const TileExperts& ex,
            const ColumnGroups& cg) {
@@ -588,10 +674,10 @@ int launch(const void* A, int lda, const void* W, int ldw, const float* bias, vo
     const int w_rows = cg.groups ? cg.groups * N : (ex.tile_expert ? (ex.experts - 1) * ex.rows_per_expert + N : N);
     const int w_cols = ex.tile_expert ? (ex.experts - 1) * ex.k_per_expert + K : K;
     const int a_cols = cg.groups ? (cg.groups - 1) * cg.a_cols + K : K;
-    if (!make_map(&map_a, A, M, a_cols, lda, BM) || !make_map(&map_w, W, w_rows, w_cols, ldw, BN)) return PS_ERR_LAUNCH;
+    if (!make_map(&map_a, A, M, a_cols, lda, BM) || !make_map(&map_w, W, w_rows, w_cols, ldw, Config<BN, PAIR>::W_ROWS)) return PS_ERR_LAUNCH;
     if (cg.groups) {            // every group writes its own block of columns: plain stores with bounds, no TMA boxes
         map_out = map_a;
-        return launch_kernel<BN, TOut, false>(map_a, map_w, map_out, bias, out, ldo, M, N, K, act, accumulate, status, kv,
+        return launch_kernel<BN, TOut, false, PAIR>(map_a, map_w, map_out, bias, out, ldo, M, N, K, act, accumulate, status, kv,
                                               stream, ex, cg);
     }
     // TMA can write the output when its rows start on 16-byte boundaries and end on one: a store is clipped at
@@ -601,10 +687,10 @@ int launch(const void* A, int lda, const void* W, int ldw, const float* bias, vo
                          (((size_t)N * sizeof(TOut)) % 16 == 0) &&
                          make_out_map(&map_out, out, M, N, ldo, (int)sizeof(TOut));
     if (tma_out)
-        return launch_kernel<BN, TOut, true>(map_a, map_w, map_out, bias, out, ldo, M, N, K, act, accumulate, status, kv, stream, ex, cg);
+        return launch_kernel<BN, TOut, true, PAIR>(map_a, map_w, map_out, bias, out, ldo, M, N, K, act, accumulate, status, kv, stream, ex, cg);
     if (kv.k_pool) return PS_ERR_UNSUPPORTED;      // the cache write lives in the TMA-store epilogue only
     map_out = map_a;    // unused
-    return launch_kernel<BN, TOut, false>(map_a, map_w, map_out, bias, out, ldo, M, N, K, act, accumulate, status, kv, stream, ex, cg);
+    return launch_kernel<BN, TOut, false, PAIR>(map_a, map_w, map_out, bias, out, ldo, M, N, K, act, accumulate, status, kv, stream, ex, cg);
 }
 
 template <typename TOut>
@@ -614,31 +700,48 @@ int pick(const void* A, int lda, const void* W, int ldw, const float* bias, void
     if (bn == 0 && cg.groups) bn = N <= 64 ? 64 : (N <= 128 ? 128 : 256);     // small matrices: one tile across
     if (bn == 0) {
         const int tiles_m = (M + BM - 1) / BM;
-        // widest tile that still gives the SMs enough tiles (measured on B200: 128 wide wins until the
-        // grid falls below half the SMs; 256 wide needs two full waves)
-        const int t128 = tiles_m * ((N + 127) / 128), t96 = tiles_m * ((N + 95) / 96);
-        const int t256 = tiles_m * ((N + 255) / 256);
-        if (t256 >= 2 * sm_count()) bn = 256;
-        // bfloat16 output whose 256-wide tiles are one wave while 128-wide ones would be two rounds per CTA: an
-        // MMA of 128 x N x 16 takes about 130 clocks whatever N is, so one wide tile costs half of two narrow
-        // ones (2,048 x 2,304 x 768: 12.4 -> 9.9 us inside a prefill step)
-        else if (sizeof(TOut) == 2 && t256 <= sm_count() && t128 > sm_count()) bn = 256;
-        // bfloat16 output of a deep product (K of 1,024 and more, where the main loop outweighs what a CTA does
-        // once): rounds of tiles per CTA times what a tile of each width costs beside one of 128 (measured alone:
-        // 1,024 x 4,800 x 1,600 takes 30.1 / 26.7 / 28.4 us at 128 / 192 / 256 columns, 2,048 x 3,072 x 1,024
-        // 23.0 / 21.4 / 23.0, 2,048 x 4,096 x 1,024 28.9 / 28.4 / 23.9)
-        else if (sizeof(TOut) == 2 && K >= 1024 && t128 > sm_count()) {
-            const int t192 = tiles_m * ((N + 191) / 192);
-            auto rounds = [&](int tiles) { return (tiles + sm_count() - 1) / sm_count(); };
-            const int c128 = rounds(t128) * 100, c192 = rounds(t192) * 130, c256 = rounds(t256) * 145;
-            bn = (c128 <= c192 && c128 <= c256) ? 128 : (c192 <= c256 ? 192 : 256);
+        const int t128 = tiles_m * ((N + 127) / 128), t96 = tiles_m * ((N + 95) / 96), t256 = tiles_m * ((N + 255) / 256);
+        if (K >= 1024 && t128 > sm_count()) {
+            // Deep products (where the main loop outweighs what a CTA does once) with more 128-wide tiles than SMs: the shape
+            // with the least modelled time, a fixed part plus the busiest CTA's (or pair's) tiles times what one costs:
+            // microseconds per k-block of 64 and per tile, fitted on B200 to products of 2,048 to 8,192 rows, 768 to 8,192
+            // columns and K of 768 to 6,400.  A k-block of a wider tile costs less per column (each operand byte that enters
+            // shared memory is used by more of the other operand; a pair of CTAs fetches half of the columns' operand each),
+            // float32 results cost more per tile than bfloat16 ones, and a last round that is nearly empty costs as much as a
+            // full one.  The choice was within 8 % of the best shape, 0.7 % on average; the rule before, which left float32
+            // results at 128 columns below two full rounds of 256-wide tiles, was 12 % behind on average (4,087 x 2,048 x
+            // 2,048 49.8 -> 30.5 us, 4,099 x 2,048 x 4,096 100.9 -> 53.9).
+            struct Shape { int bn, rows, columns, at_once; float fixed, block[2], tile[2]; };       // [bfloat16, float32 results]
+            const Shape shapes[4] = {{128, 128, 128, sm_count(), 2.5f, {.327f, .416f}, {1.f, .3f}},
+                                     {192, 128, 192, sm_count(), 2.8f, {.386f, .56f}, {.6f, .1f}},
+                                     {256, 128, 256, sm_count(), 4.f, {.464f, .585f}, {.4f, .3f}},
+                                     {PAIR_256, 256, 256, sm_count() / 2, 5.5f, {.425f, .51f}, {.4f, .3f}}};
+            const int wide = sizeof(TOut) == 4, blocks = (K + BK - 1) / BK;
+            float least = 0.f;
+            for (const Shape& shape : shapes) {
+                if (shape.bn == PAIR_256 && ex.tile_expert) continue;      // tiles of 128 rows have their own matrices
+                const int tiles = ((M + shape.rows - 1) / shape.rows) * ((N + shape.columns - 1) / shape.columns);
+                const float time = shape.fixed + (float)((tiles + shape.at_once - 1) / shape.at_once) * (blocks * shape.block[wide] + shape.tile[wide]);
+                if (least == 0.f || time < least) { least = time; bn = shape.bn; }
+            }
         }
+        // Shallow products: 256 wide with two full rounds of tiles, or for bfloat16 results where those are one round while
+        // 128-wide ones would be two: an MMA of 128 x N x 16 takes about 130 clocks whatever N is, so one wide tile costs half
+        // of two narrow ones (2,048 x 2,304 x 768: 12.4 -> 9.9 us inside a prefill step).  In between 128: inside a prefill
+        // step the CTAs that are done first make room for the next product's, which outweighs what wider tiles gain alone
+        // (2,048 x 3,072 x 768 with 192 columns 13.5 instead of 16.6 us alone, and 3 us more in a step of twelve layers each).
+        else if (t256 >= 2 * sm_count()) bn = 256;
+        else if (sizeof(TOut) == 2 && t256 <= sm_count() && t128 > sm_count()) bn = 256;
         // float32 output (the products that add into the residual stream, N = the model width): 96 wide when
         // that fills more of one wave (2,048 x 768: 128 CTAs instead of 96)
         else if (sizeof(TOut) == 4 && t128 < sm_count() && t96 <= sm_count() && t96 > t128 && 2 * t128 >= sm_count())
             bn = 96;
         else if (2 * t128 >= sm_count()) bn = 128;
         else bn = 64;
+    }
+    if (bn == PAIR_256) {
+        if (cg.groups || ex.tile_expert) return PS_ERR_UNSUPPORTED;
+        return launch<256, TOut, true>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, status, kv, stream, ex, cg);
     }
     if (bn == 256) return launch<256, TOut>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, status, kv, stream, ex, cg);
     if (bn == 192) return launch<192, TOut>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, status, kv, stream, ex, cg);
@@ -654,7 +757,7 @@ int pick(const void* A, int lda, const void* W, int ldw, const float* bias, void
 }  // namespace ps
 
 // status: device int32 that a bounded wait sets when it runs out (must not be null).
-// bn: 0 = choose, else 64, 96 (float32 output only), 128, 192 or 256 (the N extent of the MMA tile).
+// bn: 0 = choose, else 64, 96 (float32 output only), 128, 192 or 256 (the N extent of the MMA tile), or 512: 256 x 256 on pairs of CTAs.
 static int gemm_tc_entry(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo, int M,
                          int N, int K, int out_dtype, int act, int accumulate, int* status, int bn,
                          const ps::KvScatter& kv, void* stream,
