@@ -83,6 +83,12 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bflo
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * 16;
+    const int first = blockIdx.y * 8 * MT;                // this CTA's rows of A: up to 8 MT of them from here on
+    A += (size_t)first * lda;
+    out += (size_t)first * ldo;
+    M = min(M - first, 8 * MT);
+    kv.positions += first;
+    kv.token_row += first;
     int n_shift = 0;                                      // the group's first column of the stacked weight
     if (gr.cols) {
         const int group = n0 / gr.cols;
@@ -202,6 +208,18 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bflo
     }
 }
 
+// Token tiles of 8 rows in a CTA such that the CTAs of all blocks are resident at once, the fewest possible; 0: none of 1 to 3.
+// CTAs that are resident at once, by the instances of pick_warps: K up to 1,024, 3 per SM with one token tile (256 threads,
+// 80 registers) and 4 with two or three (128 threads); up to 2,048, 2 (256 threads); beyond, 1 (512 threads).
+inline int skinny_block(int M, int N, int K) {
+    const int steps = (K + 31) / 32, tiles = (M + 7) / 8;
+    for (int block = 1; block <= 3 && block <= tiles; ++block) {
+        const int resident = 148 * (steps <= 32 ? (block == 1 ? 3 : 4) : steps <= 64 ? 2 : 1);
+        if ((N + 15) / 16 * ((tiles + block - 1) / block) <= resident) return block;
+    }
+    return 0;
+}
+
 template <int MT, int WARPS, int UNROLL, typename TOut>
 int launch_skinny(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo,
                   int M, int N, int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s,
@@ -210,8 +228,9 @@ int launch_skinny(const void* A, int lda, const void* W, int ldw, const float* b
     auto kernel = gemm_skinny_kernel<MT, WARPS, UNROLL, TOut>;
     static size_t raised[MAX_DEVICES] = {0};
     if (!ensure_dynamic_smem((const void*)kernel, smem, raised)) return PS_ERR_LAUNCH;
-    return launch_pdl(kernel, dim3((N + 15) / 16), dim3(WARPS * 32), smem, s, (const __nv_bfloat16*)A, lda,
-                      (const __nv_bfloat16*)W, ldw, bias, (TOut*)out, ldo, M, N, K, act, accumulate, kv, gr);
+    return launch_pdl(kernel, dim3((N + 15) / 16, (M + 8 * MT - 1) / (8 * MT)), dim3(WARPS * 32), smem, s,
+                      (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)W, ldw, bias, (TOut*)out, ldo, M, N, K, act,
+                      accumulate, kv, gr);
 }
 
 template <int MT, typename TOut>
@@ -254,11 +273,16 @@ template <typename TOut>
 int pick_tiles(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo, int M,
                int N, int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s,
                const SkinnyGroups& gr = SkinnyGroups{}) {
-    // the MMAs of a CTA grow with the token tiles, and from 17 rows on they are what the kernel waits for:
-    // every count of tiles has its own instance
+    // The MMAs of a CTA grow with its token tiles, and beyond a few of them they are what the kernel waits for (an SM issues
+    // one in about 10 clocks): the rows are cut into blocks of as few token tiles as leave all CTAs resident at once
+    // (ps_gemm_skinny_block), each block reading the weights for itself from L2.  64 rows, us, all rows in one CTA / in
+    // blocks: 2,304 x 768 8.4 / 4.0, 768 x 768 7.5 / 2.4, 3,072 x 768 9.0 / 4.7, 768 x 3,072 12.1 / 4.5; 32 rows 4.6 / 3.1,
+    // 3.9 / 2.0, 5.2 / 3.4, 6.2 / 3.6.  With a second round of CTAs that is lost again (64 x 3,072 x 768 in blocks of 16
+    // rows, 768 CTAs: 6.9), so where no block fits a CTA keeps all rows: every count of tiles has its own instance.
 #define PS_TILES(MT_) \
     return pick_warps<MT_, TOut>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s, gr)
-    switch ((M + 7) / 8) {
+    const int block = skinny_block(M, N, K);
+    switch (block ? block : (M + 7) / 8) {
         case 1: PS_TILES(1);
         case 2: PS_TILES(2);
         case 3: PS_TILES(3);
@@ -300,6 +324,13 @@ gemm_skinny_fused_kernel(NormInput in, const __nv_bfloat16* __restrict__ W, int 
     // the cache address of each row [8*MT] (64-bit), then the normed rows [8*MT][K+8] bf16
     extern __shared__ __align__(16) float red[];
     constexpr int TOK = 8 * MT;
+    const int first = blockIdx.y * TOK;            // this CTA's rows: up to TOK of them from here on
+    if (in.rows) in.rows += first;
+    else in.x += (size_t)first * in.ldx;
+    out += (size_t)first * ldo;
+    M = min(M - first, TOK);
+    kv.positions += first;
+    kv.token_row += first;
     const int lda_s = K + 8;                       // padded: 16-byte reads of 8 rows hit 8 different bank groups
     float* gamma_s = red + (size_t)WARPS * 16 * TOK;
     float* beta_s = gamma_s + K;
@@ -532,8 +563,8 @@ int launch_skinny_fused(const NormInput& in, const void* W, int ldw, const float
     if (smem > 200 * 1024) return PS_ERR_UNSUPPORTED;
     static size_t raised[MAX_DEVICES] = {0};
     if (!ensure_dynamic_smem((const void*)kernel, smem, raised)) return PS_ERR_LAUNCH;
-    return launch_pdl(kernel, dim3((N + 15) / 16), dim3(WARPS * 32), smem, s, in, (const __nv_bfloat16*)W, ldw, bias,
-                      (TOut*)out, ldo, M, N, K, act, accumulate, kv);
+    return launch_pdl(kernel, dim3((N + 15) / 16, (M + 8 * MT - 1) / (8 * MT)), dim3(WARPS * 32), smem, s, in,
+                      (const __nv_bfloat16*)W, ldw, bias, (TOut*)out, ldo, M, N, K, act, accumulate, kv);
 }
 
 template <int MT, typename TOut>
@@ -551,7 +582,8 @@ template <typename TOut>
 int pick_tiles_fused(const NormInput& in, const void* W, int ldw, const float* bias, void* out, int ldo, int M, int N,
                      int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s) {
     if (M <= 8) return pick_warps_fused<1, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
-    if (M <= 16) return pick_warps_fused<2, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    // blocks of 16 rows where their CTAs are resident at once (2 per SM): a CTA norms only its own rows
+    if (M <= 16 || (N + 15) / 16 * ((M + 15) / 16) <= 2 * 148) return pick_warps_fused<2, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
     return pick_warps_fused<4, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
 }
 
@@ -560,6 +592,9 @@ int pick_tiles_fused(const NormInput& in, const void* W, int ldw, const float* b
 
 // An optional cache write of the key and value columns rides on the epilogue (kv_* arguments as for
 // ps_gemm_skinny_fused; k_pool null = none).
+// Rows (a multiple of 8) of a block in which a CTA of the kernel takes M rows while all CTAs are resident at once; 0: it takes all M.
+PS_EXPORT int ps_gemm_skinny_block(int M, int N, int K) { return 8 * ps::skinny_block(M, N, K); }
+
 PS_EXPORT int ps_gemm_skinny(const void* A, int lda, const void* W, int ldw, const float* bias, void* out,
                              int ldo, int M, int N, int K, int out_dtype, int act, int accumulate,
                              void* k_pool, void* v_pool, long long page_stride, const int* token_item,

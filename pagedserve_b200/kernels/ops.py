@@ -130,6 +130,7 @@ _SIGNATURES = {
         "ps_copy_h2d": [_P, _P, _L, _P],
     },
     "bf16": {
+        "ps_gemm_skinny_block": [_I, _I, _I],
         "ps_gemm_skinny": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I,
                            _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "ps_gemm_skinny_fused": [_P, _I, _P, _P, _P, _F, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I,
@@ -544,6 +545,10 @@ class Ops:
         K = a.shape[1]
         return (a.shape[0] <= 64 and K % 8 == 0 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
                 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+    def skinny_in_blocks(self, a, w):
+        """Whether the weight-streaming kernel takes these rows in blocks whose CTAs are all resident at once."""
+        return self.skinny_ok(a, w) and self.fast.ps_gemm_skinny_block(a.shape[0], w.shape[0], a.shape[1]) > 0
 
     FUSED_NORM_ROWS = 32          # most rows for which the norm is folded into the skinny product
     FUSED_NORM_COLUMNS = 16 * 2 * 148   # and most output columns
