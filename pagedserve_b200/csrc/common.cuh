@@ -73,6 +73,28 @@ __device__ __forceinline__ float apply_act(float x, int act) {
     return x;
 }
 
+// The inner activation of a gated feed-forward (csrc/moe.cu says what the kinds are).
+struct GateForm {
+    int kind;                 // 0: silu(g) u w; 2: gelu_tanh(g) u w; 1: clamped, weight on the input 
+    float limit;              // kind 1: the routed experts' limit
+    float shared_limit;       // kind 1: the shared expert's
+    float alpha;              // kind 1: the sigmoid's slope
+};
+
+// the tanh form of gelu, written 0.5 z (1 + tanh(a)) = z / (1 + exp(-2 a)): no difference of nearly equal numbers where z is
+// negative, and one exponential and one division on the special function units instead of tanhf
+__device__ __forceinline__ float gelu_tanh_sigmoid(float z) {
+    const float a = 0.7978845608028654f * (z + 0.044715f * z * z * z);
+    return __fdividef(z, 1.0f + __expf(-2.0f * a));
+}
+__device__ __forceinline__ float gated_inner(float g, float u, float w, int kind, float limit, float alpha) {
+    if (kind == 0) return silu(g) * u * w;
+    if (kind == 2) return gelu_tanh_sigmoid(g) * u * w;
+    g = fminf(g * w, limit);
+    u = fminf(fmaxf(u * w, -limit), limit);
+    return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);
+}
+
 // the same over a thread's block of values, with the choice made once outside the loop
 template <int N>
 __device__ __forceinline__ void apply_act_all(float (&v)[N], int act) {

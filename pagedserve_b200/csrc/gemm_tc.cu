@@ -186,6 +186,13 @@ struct ColumnGroups {
     int out_cols;
 };
 
+// A gated feed-forward's first product: output column n is form(gate row n . a, row n . a of the ups) times the row's weight, where
+// W holds N gate rows and, N rows further on, N up rows (of each expert, where tiles have experts).  row_weight null: 1.
+struct GatedResult {
+    GateForm form;
+    const float* row_weight;
+};
+
 template <int BN, bool PAIR> struct Config {
     static constexpr int W_ROWS = PAIR ? BN / 2 : BN;              // rows of W in a CTA's stage
     static constexpr int STAGE_BYTES = BM * BK * 2 + W_ROWS * BK * 2;
@@ -208,12 +215,15 @@ template <int BN, bool PAIR> struct Config {
 // the MMAs, its barriers count the copies of both, and its commits arrive in both.  Per output a third fewer bytes enter
 // shared memory than with 128 x 256 tiles, which are bound by that memory's bandwidth (48 KB in and as much read per k-block
 // of 512 clocks): 5,824 x 4,800 x 1,600 69.7 -> 63.8 us (1.40 PFLOP/s), 4,099 x 8,192 x 2,048 109 -> 101.
-template <int BN, typename TOut, bool TMA_OUT, bool PAIR>
+// GATED: the first half of a tile's rows of W are gates, the second the ups of the same output columns, and the epilogue forms
+// their activation from the two halves of the accumulator: the products' columns are never stored (the kernel that formed
+// the activation from them took 28 us for 8,198 rows of 2 x 2,048, beside 75 MB written and read again).
+template <int BN, typename TOut, bool TMA_OUT, bool PAIR, bool GATED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_out, const float* __restrict__ bias, TOut* __restrict__ out,
                int ldo, int M, int N, int K, int act, int accumulate, int* __restrict__ status, KvScatter kv,
-               TileExperts ex, ColumnGroups cg) {
+               TileExperts ex, ColumnGroups cg, GatedResult gated) {
     using Cfg = Config<BN, PAIR>;
     constexpr int STAGES = Cfg::STAGES;
     constexpr int TILE_M = PAIR ? 2 * BM : BM;
@@ -233,7 +243,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // Set-up (barriers, tensor memory) and the first weight tiles do not depend on the kernel before this one:
     // they happen before the wait and overlap its end.
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_n = (N + BN - 1) / BN, tiles_m = (M + TILE_M - 1) / TILE_M;
+    constexpr int OUT_N = GATED ? BN / 2 : BN;                     // output columns of a tile
+    const int tiles_n = (N + OUT_N - 1) / OUT_N, tiles_m = (M + TILE_M - 1) / TILE_M;
     const int per_m = (cg.groups > 0 ? cg.groups : 1) * tiles_n;        // tiles of one block of rows
     const int num_tiles = tiles_m * per_m;
     const int num_kb = (K + BK - 1) / BK;
@@ -277,10 +288,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if constexpr (PAIR) tma_load_2d_pair(dst, map, x, y, in_first_cta(&full[s]));
                 else tma_load_2d(dst, map, x, y, &full[s]);
             };
+            auto load_weights = [&](unsigned char* dst, int x, int n0, int s) {
+                if constexpr (!GATED) {
+                    load(dst, &map_w, x, n0 + rank * Cfg::W_ROWS, s);
+                } else if constexpr (PAIR) {                     // one CTA of the pair has the gates, the other the ups
+                    load(dst, &map_w, x, n0 + rank * N, s);
+                } else {
+                    load(dst, &map_w, x, n0, s);
+                    load(dst + OUT_N * BK * 2, &map_w, x, n0 + N, s);
+                }
+            };
             for (uint32_t kb = 0; kb < early; ++kb) {
-                const int n0 = (first_tile % tiles_n) * BN + rank * Cfg::W_ROWS;
                 expect(kb);
-                load(tiles + (size_t)kb * Cfg::STAGE_BYTES + BM * BK * 2, &map_w, (int)kb * BK, n0, kb);
+                load_weights(tiles + (size_t)kb * Cfg::STAGE_BYTES + BM * BK * 2, (int)kb * BK, (first_tile % tiles_n) * OUT_N, kb);
             }
             pdl_prologue();
             const int* tile_expert = pdl_fresh(ex.tile_expert);
@@ -288,7 +308,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             bool ok = true;
             for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
                 const int m0 = (tile / per_m) * TILE_M + rank * BM;
-                int n0 = (tile % tiles_n) * BN + rank * Cfg::W_ROWS, k0 = 0, a_k0 = 0;
+                int n0 = (tile % tiles_n) * OUT_N, k0 = 0, a_k0 = 0;
                 if (cg.groups) {                                 // this tile's group: its columns of A, its rows of W
                     const int group = (tile % per_m) / tiles_n;
                     a_k0 = group * cg.a_cols;
@@ -306,7 +326,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (it >= early) {
                         if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; atomicExch(status, 11); break; }
                         expect(s);
-                        load(a_dst + BM * BK * 2, &map_w, k0 + kb * BK, n0, s);
+                        load_weights(a_dst + BM * BK * 2, k0 + kb * BK, n0, s);
                     }
                     load(a_dst, &map_a, a_k0 + kb * BK, m0, s);
                 }
@@ -367,9 +387,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         [[maybe_unused]] uint32_t chunk = 0;                // column groups this team has sent out so far
         bool ok = true;
         const int* tile_expert = pdl_fresh(ex.tile_expert);
+        [[maybe_unused]] const float* gated_weight = pdl_fresh(gated.row_weight);
         for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local) {
             if (tile_expert && tile_expert[tile / tiles_n] < 0) { --local; continue; }         // a tile of no expert
-            const int m0 = (tile / per_m) * TILE_M + rank * BM, n0 = (tile % tiles_n) * BN;
+            const int m0 = (tile / per_m) * TILE_M + rank * BM, n0 = (tile % tiles_n) * OUT_N;
             const int out_col0 = cg.groups ? ((tile % per_m) / tiles_n) * cg.out_cols : 0;     // the group's columns
             const int buf = local & 1;
             // a q|k|v product whose key and value columns go straight into the pages: where this row's go
@@ -387,7 +408,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // holds the values of columns j, 32 + j, ... of each group and hands them out by shuffle below (a
             // first touch of these lines after the accumulator is complete costs about a microsecond per group).
             [[maybe_unused]] float bias_lane[TMA_OUT ? Cfg::GROUPS_PER_TEAM * Cfg::HALVES_MAX : 1];
-            if constexpr (TMA_OUT) {
+            if constexpr (TMA_OUT && !GATED) {
                 constexpr int COLS = 128 / (int)sizeof(TOut);
 #pragma unroll
                 for (int g = 0; g < Cfg::GROUPS_PER_TEAM * (COLS / 32); ++g) {
@@ -395,10 +416,62 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     bias_lane[g] = (bias && n < N && (team + 2 * (g / (COLS / 32))) * COLS < BN) ? bias[n] : 0.f;
                 }
             }
+            [[maybe_unused]] float weight = 1.f;                // GATED: this row's weight
+            if constexpr (GATED) {
+                const int row = m0 + quarter * 32 + lane;
+                if (gated.row_weight) weight = row < M ? gated_weight[row] : 0.f;
+            }
             if (!mbar_wait(&acc_full[buf], (local >> 1) & 1, abort_flag)) { ok = false; if (lane == 0) atomicExch(status, 14); break; }
             tc_fence_after();
             const int m = m0 + quarter * 32 + lane;
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
+            if constexpr (GATED) {
+                // team t forms the 64 output columns from 64 t on: gates in the first half of the accumulator, ups in the second
+                const int r = quarter * 32 + lane, c = 64 * team;
+                const bool leader = (quarter == 2 && lane == 0);
+                unsigned char* stage_buf = staging + (size_t)(team * Cfg::STAGING_BUFS) * (BM * 128);
+                if (leader) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                team_sync(team);
+#pragma unroll
+                for (int part = 0; part < 2; ++part) {
+                    uint32_t gate[32], up[32];
+                    tmem_ld32(taddr + c + 32 * part, gate);
+                    tmem_ld32(taddr + OUT_N + c + 32 * part, up);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (part == 1) {
+                        tc_fence_before();
+                        drained(buf);
+                    }
+                    float v[32];
+                    if (weight == 0.f) {                         // a row of no token: whatever the products are
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            v[j] = gated_inner(__uint_as_float(gate[j]), __uint_as_float(up[j]), weight, gated.form.kind,
+                                               gated.form.limit, gated.form.alpha);
+                    }
+#pragma unroll
+                    for (int piece = 0; piece < 4; ++piece) {
+                        uint4 pack;
+                        uint32_t* two = reinterpret_cast<uint32_t*>(&pack);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const __nv_bfloat162 p = __floats2bfloat162_rn(v[8 * piece + 2 * i], v[8 * piece + 2 * i + 1]);
+                            two[i] = *reinterpret_cast<const uint32_t*>(&p);
+                        }
+                        *reinterpret_cast<uint4*>(stage_buf + r * 128 + ((4 * part + piece) ^ (r & 7)) * 16) = pack;
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                team_sync(team);
+                if (leader) {
+                    if (n0 + c < N && m0 < M) tma_store_2d(&map_out, stage_buf, n0 + c, m0);
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+                continue;
+            }
             if constexpr (TMA_OUT) {
                 // columns per staged buffer: 128 bytes of output per row
                 constexpr int COLS = 128 / (int)sizeof(TOut);
@@ -650,20 +723,22 @@ static int sm_count() {
     return count;
 }
 
-template <int BN, typename TOut, bool TMA_OUT, bool PAIR>
+template <int BN, typename TOut, bool TMA_OUT, bool PAIR, bool GATED = false>
 int launch_kernel(const CUtensorMap& map_a, const CUtensorMap& map_w, const CUtensorMap& map_out, const float* bias,
                   void* out, int ldo, int M, int N, int K, int act, int accumulate, int* status, const KvScatter& kv,
-                  cudaStream_t stream, const TileExperts& ex, const ColumnGroups& cg) {
-    auto kernel = gemm_tc_kernel<BN, TOut, TMA_OUT, PAIR>;
+                  cudaStream_t stream, const TileExperts& ex, const ColumnGroups& cg,
+                  const GatedResult& gated = GatedResult{GateForm{0, 0.f, 0.f, 0.f}, nullptr}) {
+    auto kernel = gemm_tc_kernel<BN, TOut, TMA_OUT, PAIR, GATED>;
     using Cfg = Config<BN, PAIR>;
     static size_t raised[MAX_DEVICES] = {0};
     if (!ensure_dynamic_smem((const void*)kernel, (size_t)Cfg::SMEM, raised)) return PS_ERR_LAUNCH;
     constexpr int TILE_M = PAIR ? 2 * BM : BM;
-    const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + BN - 1) / BN) * (cg.groups > 0 ? cg.groups : 1);
+    constexpr int OUT_N = GATED ? BN / 2 : BN;
+    const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + OUT_N - 1) / OUT_N) * (cg.groups > 0 ? cg.groups : 1);
     const int most = PAIR ? sm_count() / 2 : sm_count();
     const int grid = tiles < most ? tiles : most;
     return launch_pdl_clusters(kernel, dim3(PAIR ? 2 * grid : grid), dim3(THREADS), Cfg::SMEM, stream, dim3(PAIR ? 2 : 1), map_a, map_w, map_out, bias,
-                      (TOut*)out, ldo, M, N, K, act, accumulate, status, kv, ex, cg);
+                      (TOut*)out, ldo, M, N, K, act, accumulate, status, kv, ex, cg, gated);
 }
 
 template <int BN, typename TOut, bool PAIR = false>
@@ -831,4 +906,36 @@ PS_EXPORT int ps_gemm_tc_qkv(const void* A, int lda, const void* W, int ldw, con
     ps::KvScatter kv{(__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, page_stride, token_item, positions, block_table,
                      bt_stride, q_width, kv_width, head_dim, page_size};
     return gemm_tc_entry(A, lda, W, ldw, bias, out, ldo, M, N, K, PS_BF16, PS_ACT_NONE, 0, status, 0, kv, stream);
+}
+
+// The first product of a gated feed-forward with its activation: out[m, n] (bfloat16, [M, F]) = form(A[m] . gate row n, A[m] . up row
+// n) with the row's weight (row_weight float32 [M], null: 1; a row of weight 0 gives zeros).  W [2 F, K]: F gate rows, then F up
+// rows; with tile_expert (as for ps_gemm_tc_experts) the experts' such matrices stacked by rows.
+PS_EXPORT int ps_gemm_tc_gated(const void* A, int lda, const void* W, int ldw, void* out, int ldo, int M, int F, int K, int kind,
+                               float limit, float alpha, const float* row_weight, const int* tile_expert, int experts,
+                               int* status, void* stream) {
+    if (M <= 0 || F <= 0) return PS_OK;
+    if (!status || kind < 0 || kind > 2 || (kind == 1 && !(limit > 0.f)) || (tile_expert && experts <= 0)) return PS_ERR_BAD_ARGUMENT;
+    if (K <= 0 || K % 8 || lda % 8 || ldw % 8 || ldo % 8 || F % 8 || lda < K || ldw < K || ldo < F) return PS_ERR_UNSUPPORTED;
+    if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)out) & 15) return PS_ERR_UNSUPPORTED;
+    using namespace ps::tc;
+    using bf = __nv_bfloat16;
+    CUtensorMap map_a, map_w, map_out;
+    if (!make_map(&map_a, A, M, K, lda, BM) || !make_map(&map_w, W, 2 * F * (tile_expert ? experts : 1), K, ldw, 128) ||
+        !make_out_map(&map_out, out, M, F, ldo, 2))
+        return PS_ERR_LAUNCH;
+    const GatedResult gated{ps::GateForm{kind, limit, limit, alpha}, row_weight};
+    const TileExperts ex{tile_expert, tile_expert ? 2 * F : 0, 0, experts};
+    const ps::KvScatter none = {};
+    const ColumnGroups no_groups{0, 0, 0};
+    // pairs of CTAs where they are modelled to be faster, as in pick()
+    const int across = (F + 127) / 128, blocks = (K + BK - 1) / BK, alone = (M + 127) / 128 * across, pairs = (M + 255) / 256 * across;
+    const float one = 4.f + (float)((alone + sm_count() - 1) / sm_count()) * (blocks * .464f + .4f);
+    const float two = 5.5f + (float)((pairs + sm_count() / 2 - 1) / (sm_count() / 2)) * (blocks * .425f + .4f);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (!tile_expert && two < one)
+        return launch_kernel<256, bf, true, true, true>(map_a, map_w, map_out, nullptr, out, ldo, M, F, K, PS_ACT_NONE, 0, status, none,
+                                                        s, ex, no_groups, gated);
+    return launch_kernel<256, bf, true, false, true>(map_a, map_w, map_out, nullptr, out, ldo, M, F, K, PS_ACT_NONE, 0, status, none, s,
+                                                     ex, no_groups, gated);
 }

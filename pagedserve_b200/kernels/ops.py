@@ -152,6 +152,7 @@ _SIGNATURES = {
                             _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "ps_gemm_tc_groups": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
         "ps_gemm_tc_experts": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P],
+        "ps_gemm_tc_gated": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _F, _P, _P, _I, _P, _P],
         "ps_gemm_tc_qkv": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "ps_prefill_attention_tc": [_P, _I, _I, _P, _I, _P, _L, _L, _L, _L, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I,
                                     _I, _I, _F, _I, _P, _F, _P, _I, _I, _P],
@@ -1836,6 +1837,41 @@ class Ops:
                                            K, dtype_code(out.dtype), _ACT_CODE[act], _ptr(tile_expert), experts,
                                            1 if along_k else 0, _ptr(status), _stream()), "gemm_tc_experts")
         return out
+
+    def gated_ok(self, a, w, inner):
+        """Whether the product of many rows with stacked gate and up matrices can form the activation itself
+        (:meth:`linear_gated`): bfloat16, more rows than the weight-streaming kernel takes, TMA's alignment."""
+        return (self.dtype == torch.bfloat16 and a.shape[0] > 64 and inner.shape[1] % 8 == 0 and inner.stride(0) % 8 == 0
+                and inner.stride(1) == 1 and a.stride(1) == 1 and w.stride(1) == 1 and inner.data_ptr() % 16 == 0
+                and self.tc_ok(a, w))
+
+    def linear_gated(self, a, w, inner, form=None, row_weight=None, tile_expert=None, experts=1):
+        """inner[m, n] = the gated activation ``form`` (:meth:`_gate_form`; of a clamped one the routed experts' limit where
+        ``tile_expert`` is given, else the shared expert's) of a[m] . w[n] and a[m] . w[F + n], times the row's weight
+        (float32 [M]; None: 1), in one tcgen05 product: ``w`` [2 F, K], or with ``tile_expert`` (as for
+        :meth:`linear_experts`) the experts' such matrices stacked by rows."""
+        M, K = a.shape
+        F = inner.shape[1]
+        if (w.shape != (2 * F * experts, K) or inner.shape[0] != M or not self.gated_ok(a, w, inner) or (tile_expert is None and experts != 1)
+                or (tile_expert is not None and tile_expert.numel() != -(-M // self.EXPERT_TILE))
+                or (row_weight is not None and (row_weight.numel() != M or not row_weight.is_contiguous()))):
+            raise KernelError("linear_gated: shapes do not match")
+        for name, tensor in (("a", a), ("w", w), ("inner", inner)):
+            _require(tensor, name, torch.bfloat16)
+        if row_weight is not None:
+            _require(row_weight, "row_weight", torch.float32)
+        if tile_expert is not None:
+            _require(tile_expert, "tile_expert", torch.int32)
+        kind, limit, shared_limit, alpha = self._gate_form(form)
+        if kind == 3:
+            raise KernelError("linear_gated: relu_squared has no gate")
+        if self._tc is None:
+            self._tc = _declare(_load_library("tc"), "tc")
+        self.launches += 1
+        _check(self._tc.ps_gemm_tc_gated(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(inner), inner.stride(0), M, F, K, kind,
+                                         limit if tile_expert is not None else shared_limit, alpha, _ptr(row_weight),
+                                         _ptr(tile_expert), experts, _ptr(self.status_flag(a.device)), _stream()), "gemm_tc_gated")
+        return inner
 
     # ------------------------------------------------------------------ sampling
     def sample(self, logits, temperature, seed, position, out, pos_offset=0):

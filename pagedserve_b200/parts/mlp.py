@@ -15,7 +15,8 @@ class DenseMLP(FeedForward):
     """residual += act(x W_up + b_up) W_down + b_down
     (reference: src/model/paged_decoder.py:178-179, 224-228, 273-280),
     or, with ``gate_name``, the gated form residual += (act(x W_gate) * (x W_up)) W_down (activation 'silu' or
-    'gelu_tanh', no biases): gate and up run as one product over the stacked matrices, one elementwise kernel forms the inner row.
+    'gelu_tanh', no biases): gate and up run as one product over the stacked matrices; many rows of it form the inner row in the product's epilogue, few
+    rows in an elementwise kernel.
     params: hidden_size, inner_size, activation ('gelu_tanh' | 'gelu_erf' | 'relu_squared' = max(z, 0)^2 | 'silu'),
     has_bias,
     stored_in_out, up_name, down_name, gate_name (None), init_std, out_init_std."""
@@ -68,7 +69,11 @@ class DenseMLP(FeedForward):
         p = self.params
         ops = self.env.ops
         inner = ops.empty((x.shape[0], p["inner_size"]), self.env.dtype, x.device)
-        if self.w_gate_up is not None:
+        if self.w_gate_up is not None and x.shape[0] > 64 and hasattr(x, "materialize"):
+            x = x.materialize()                  # (the norm is folded into products of few rows only)
+        if self.w_gate_up is not None and x.shape[0] > 64 and ops.gated_ok(x, self.w_gate_up, inner):
+            ops.linear_gated(x, self.w_gate_up, inner, form=p["activation"])
+        elif self.w_gate_up is not None:
             gate_up = ops.empty((x.shape[0], 2 * p["inner_size"]), self.env.dtype, x.device)
             ops.linear(x, self.w_gate_up, None, gate_up)
             ops.moe_gate_mul(gate_up, None, None, inner, 0, p["inner_size"], form=p["activation"])

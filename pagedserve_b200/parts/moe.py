@@ -37,7 +37,7 @@ class RoutedExperts(FeedForward):
     token passes through every expert's columns: the weights stream once, which is what bounds such a step.
     Many tokens in bfloat16: the (token, expert) pairs are sorted by expert into a buffer in which every expert's
     run starts on a tile of the tcgen05 product (``moe_plan``, ``moe_gather``); the two products read, per tile of
-    rows, the matrix of that tile's expert (``linear_experts``); ``moe_combine`` adds each token's rows into the
+    rows, the matrix of that tile's expert (``linear_gated`` with the activation, ``linear_experts``); ``moe_combine`` adds each token's rows into the
     residual in the order of its election.  The shared expert runs as two plain products beside them.
     Either way a token's result does not depend on the other tokens of the step, and both ways compute the same
     sums up to their order.
@@ -174,9 +174,8 @@ class RoutedExperts(FeedForward):
             ops.linear_experts(inner, self.w_down, down, tile_expert, E, along_k=True)
             ops.moe_combine(down, row_of, top, residual, weights=chosen_w, factor=self.result_factor)
             return
-        gate_up = ops.empty((rows_cap, 2 * F), dtype, device)
-        ops.linear_experts(rows, self.w_gate_up[:E * 2 * F], gate_up, tile_expert, E)
-        ops.moe_gate_mul_rows(gate_up, row_weight, inner, form=self.form)
+        ops.linear_gated(rows, self.w_gate_up[:E * 2 * F], inner, form=self.form, row_weight=row_weight, tile_expert=tile_expert,
+                         experts=E)
         ops.linear_experts(inner, self.w_down[:, :E * F], down, tile_expert, E, along_k=True)
         if self.result_factor is None:
             ops.moe_combine(down, row_of, top, residual)
@@ -184,10 +183,14 @@ class RoutedExperts(FeedForward):
             ops.moe_combine(down, row_of, top, residual, weights=self._ones(chosen_w), factor=self.result_factor)
         shared_ff = p.get("shared_ff") or 0
         if shared_ff:
-            gate_up_shared = ops.empty((tokens, 2 * shared_ff), dtype, device)
-            ops.linear(x, self.w_gate_up[E * 2 * F:], None, gate_up_shared)
             inner_shared = ops.empty((tokens, shared_ff), dtype, device)
-            ops.moe_gate_mul(gate_up_shared, dense, shared_gate, inner_shared, 0, shared_ff, form=self.form)
+            w_shared = self.w_gate_up[E * 2 * F:]
+            if ops.gated_ok(x, w_shared, inner_shared):
+                ops.linear_gated(x, w_shared, inner_shared, form=self.form, row_weight=shared_gate)
+            else:
+                gate_up_shared = ops.empty((tokens, 2 * shared_ff), dtype, device)
+                ops.linear(x, w_shared, None, gate_up_shared)
+                ops.moe_gate_mul(gate_up_shared, dense, shared_gate, inner_shared, 0, shared_ff, form=self.form)
             ops.linear(inner_shared, self.w_down[:, E * F:], None, residual, accumulate=True, factor=self.result_factor)
 
     def _ones(self, like):

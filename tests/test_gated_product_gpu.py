@@ -1,0 +1,67 @@
+"""The product that forms a gated activation in its epilogue, against 64 bits: every form, tails in rows and columns, rows of weight
+zero, experts by tile, one CTA and pairs of CTAs per tile."""
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+CLAMPED = ("clamped_swish", 1.5, 1.0, 1.702)
+
+
+def formed(g, u, w, form, limit):
+    if form == "silu":
+        return g * torch.sigmoid(g) * u * w
+    if form == "gelu_tanh":
+        return torch.nn.functional.gelu(g, approximate="tanh") * u * w
+    g, u = (g * w).clamp(max=limit), (u * w).clamp(-limit, limit)
+    return g * torch.sigmoid(1.702 * g) * (u + 1)
+
+
+@pytest.mark.parametrize("form", ["silu", "gelu_tanh", CLAMPED])
+@pytest.mark.parametrize("M,F,K", [(65, 8, 8), (128, 128, 64), (129, 136, 72), (300, 72, 200), (257, 264, 1024), (2600, 1160, 136)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_gated(form, M, F, K, weighted):
+    from pagedserve_b200.kernels.ops import Ops
+
+    ops, g = Ops(torch.bfloat16), torch.Generator().manual_seed(M + F + K)
+    a = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(2 * F, K, generator=g) * 2 / math.sqrt(K)).to(torch.bfloat16).to(DEV)
+    weight = torch.rand(M, generator=g).to(DEV) if weighted else None
+    if weighted:
+        weight[::7] = 0.0
+        a[::7] = float("inf")                                   # rows of no token give zeros whatever stands in them
+    inner = torch.full((M, F + 8), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.linear_gated(a, w, inner[:, :F], form=form, row_weight=weight)
+    y = a.double() @ w.double().T
+    want = formed(y[:, :F], y[:, F:], 1.0 if weight is None else weight[:, None].double(), form, 1.0)
+    if weighted:
+        want[::7] = 0.0
+    # bfloat16 results round at 2^-9; the sums and the exponentials are float32's
+    assert float((inner[:, :F].double() - want).abs().max()) < 6e-3 * float(want.abs().max())
+    assert bool(torch.isnan(inner[:, F:]).all()) and int(ops.status_flag(DEV).item()) == 0
+
+
+@pytest.mark.parametrize("F,K", [(72, 64), (256, 136)])
+def test_experts(F, K):
+    from pagedserve_b200.kernels.ops import Ops
+
+    ops, g, E = Ops(torch.bfloat16), torch.Generator().manual_seed(F), 3
+    tile_expert = torch.tensor([2, 0, -1, 1, 0], dtype=torch.int32, device=DEV)
+    M = 5 * 128
+    a = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(E * 2 * F, K, generator=g) * 2 / math.sqrt(K)).to(torch.bfloat16).to(DEV)
+    weight = torch.rand(M, generator=g).to(DEV)
+    inner = torch.zeros(M, F, dtype=torch.bfloat16, device=DEV)
+    ops.linear_gated(a, w, inner, form=CLAMPED, row_weight=weight, tile_expert=tile_expert, experts=E)
+    for tile, expert in enumerate(tile_expert.tolist()):
+        rows = slice(128 * tile, 128 * tile + 128)
+        if expert < 0:
+            assert bool((inner[rows] == 0).all())
+            continue
+        y = a[rows].double() @ w[2 * F * expert:2 * F * (expert + 1)].double().T
+        want = formed(y[:, :F], y[:, F:], weight[rows, None].double(), CLAMPED, 1.5)
+        assert float((inner[rows].double() - want).abs().max()) < 6e-3 * float(want.abs().max()), tile
