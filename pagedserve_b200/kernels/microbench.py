@@ -667,7 +667,6 @@ def time_experts(tokens, width, experts, top, ff, iters=10, score="softmax", nor
     row_weight = torch.empty(rows_cap, device=dev)
     tile_expert = torch.empty(rows_cap // ops.EXPERT_TILE, dtype=torch.int32, device=dev)
     rows = torch.empty(rows_cap, width, dtype=torch.bfloat16, device=dev)
-    gate_up = torch.empty(rows_cap, (2 if gated else 1) * ff, dtype=torch.bfloat16, device=dev)
     inner = torch.empty(rows_cap, ff, dtype=torch.bfloat16, device=dev)
     down = torch.empty(rows_cap, width, device=dev)
     y = torch.zeros(tokens, width, device=dev)
@@ -680,8 +679,7 @@ def time_experts(tokens, width, experts, top, ff, iters=10, score="softmax", nor
         ops.moe_plan(chosen, chosen_w, experts, row_of, row_token, row_weight, tile_expert)
         ops.moe_gather(x, row_token, rows)
         if gated:
-            ops.linear_experts(rows, w_gu, gate_up, tile_expert, experts)
-            ops.moe_gate_mul_rows(gate_up, row_weight, inner, form=form)
+            ops.linear_gated(rows, w_gu, inner, form=form, row_weight=row_weight, tile_expert=tile_expert, experts=experts)
         else:
             ops.linear_experts(rows, w_gu, inner, tile_expert, experts, act="relu_squared")
         ops.linear_experts(inner, w_down, down, tile_expert, experts, along_k=True)
@@ -693,10 +691,12 @@ def time_experts(tokens, width, experts, top, ff, iters=10, score="softmax", nor
     parts["plan_us"] = _time(lambda i: ops.moe_plan(chosen, chosen_w, experts, row_of, row_token, row_weight, tile_expert),
                              iters, graph=True) * 1e6
     parts["gather_us"] = _time(lambda i: ops.moe_gather(x, row_token, rows), iters, graph=True) * 1e6
-    parts["gate_up_us"] = _time(lambda i: ops.linear_experts(rows, w_gu, gate_up, tile_expert, experts), iters,
-                                graph=True) * 1e6
-    if gated:
-        parts["gate_mul_us"] = _time(lambda i: ops.moe_gate_mul_rows(gate_up, row_weight, inner, form=form), iters, graph=True) * 1e6
+    if gated:                                 # gates, ups and the activation in one product
+        parts["gate_up_us"] = _time(lambda i: ops.linear_gated(rows, w_gu, inner, form=form, row_weight=row_weight, tile_expert=tile_expert,
+                                                               experts=experts), iters, graph=True) * 1e6
+    else:
+        parts["gate_up_us"] = _time(lambda i: ops.linear_experts(rows, w_gu, inner, tile_expert, experts, act="relu_squared"), iters,
+                                    graph=True) * 1e6
     parts["down_us"] = _time(lambda i: ops.linear_experts(inner, w_down, down, tile_expert, experts, along_k=True), iters,
                              graph=True) * 1e6
     parts["combine_us"] = _time(lambda i: ops.moe_combine(down, row_of, top, y), iters, graph=True) * 1e6

@@ -119,7 +119,6 @@ _SIGNATURES = {
         "ps_head_mix": [_P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _P],
         "ps_moe_plan": [_P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
         "ps_moe_gather": [_P, _I, _P, _P, _I, _I, _I, _I, _P],
-        "ps_moe_gate_mul_rows": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P],
         "ps_moe_combine": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P],
         "ps_step_shape": [_I, _P, _P, _P, _I, _I, _I, _I, _P],
         "ps_step_fill": [_I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _L, _P, _I, _I, _I, _I, _P],
@@ -1777,22 +1776,6 @@ class Ops:
         _check(self.core.ps_moe_gather(_ptr(x), x.stride(0), _ptr(row_token), _ptr(rows), rows.stride(0),
                                        rows.shape[0], x.shape[1], self.code, _stream()), "moe_gather")
         return rows
-
-    def moe_gate_mul_rows(self, gate_up, row_weight, inner, form=None):
-        """inner[r, j] = silu(gate_up[r, j]) * gate_up[r, F + j] * row_weight[r], or the other ``form`` of
-        :meth:`_gate_form` (with the routed experts' limit)."""
-        R, F = inner.shape
-        _require(gate_up, "gate_up", self.dtype)
-        _require(inner, "inner", self.dtype)
-        _require(row_weight, "row_weight", torch.float32)
-        if gate_up.shape != (R, 2 * F) or row_weight.numel() != R or gate_up.stride(1) != 1 or inner.stride(1) != 1:
-            raise KernelError("moe_gate_mul_rows: shapes do not match")
-        self.launches += 1
-        kind, limit, _, alpha = self._gate_form(form)
-        _check(self.core.ps_moe_gate_mul_rows(_ptr(gate_up), gate_up.stride(0), _ptr(row_weight), _ptr(inner),
-                                              inner.stride(0), R, F, self.code, kind, limit, alpha, _stream()),
-               "moe_gate_mul_rows")
-        return inner
 
     def moe_combine(self, down, row_of, top, y, weights=None, factor=None):
         """y[t] += sum_k down[row_of[t * top + k]] (float32; k in rising order, rows < 0 skipped); with ``weights`` float32
