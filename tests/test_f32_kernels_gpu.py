@@ -177,3 +177,23 @@ def test_attention_keeps_a_later_infinity_out():
     layer.k_pool[page, :, place] = float("nan")
     ops.attention_f32(q, out, step.ctx, layer, 2, 2, 64, 0, 0.125)
     assert torch.equal(out[:70], clean[:70]) and bool(torch.isnan(out[70:]).all())
+
+
+@pytest.mark.parametrize("M", [1, 4, 5, 8, 16])
+@pytest.mark.parametrize("N,K", [(9473, 4), (9501, 768), (9490, 772), (9477, 1024)])
+def test_few_rows_of_a_vocabulary(M, N, K):
+    """CTAs that walk over several groups of columns: every epilogue, and the sums of the form without walking."""
+    ops, g = ops_for(), torch.Generator().manual_seed(M + N + K)
+    a, w, bias, base = (torch.randn(shape, generator=g) for shape in ((M, K), (N, K), (N,), (M, N)))
+    w /= K ** 0.5
+    a, w, bias, base = (t.to(DEV) for t in (a, w, bias, base))
+    for accumulate in (0, 1, 3):
+        out = base.clone()
+        ops.linear_f32_rows(a, w, bias, out, accumulate=accumulate)
+        want = product(a, w, None if accumulate == 3 else bias, None, bias if accumulate == 3 else None, base if accumulate else None)
+        assert float((out.double() - want).abs().max()) < sum_bound(K) * 8 * float(want.abs().max()), accumulate
+    part = torch.empty(M, 4000, device=DEV)
+    whole = torch.empty(M, N, device=DEV)
+    ops.linear_f32_rows(a, w[:4000], None, part)
+    ops.linear_f32_rows(a, w, None, whole)
+    assert torch.equal(whole[:, :4000], part)
