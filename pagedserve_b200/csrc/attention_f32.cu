@@ -10,10 +10,10 @@
 namespace ps {
 namespace af32 {
 
-// position -> offset of its row (of head g) in the pool, or -1 where the request has no page there
-__device__ __forceinline__ long long row_offset(const int* bt, int key, int page_size, long long page_stride, int g, int head_dim) {
-    const int page = bt[key / page_size];
-    return page < 0 ? -1 : (long long)page * page_stride + ((long long)g * page_size + (key % page_size)) * head_dim;
+// position -> offset of its row (of head g) in the pool, or -1 where the request has no page there; pages are 1 << shift long
+__device__ __forceinline__ long long row_offset(const int* bt, int key, int shift, long long page_stride, int g, int head_dim) {
+    const int page = bt[key >> shift];
+    return page < 0 ? -1 : (long long)page * page_stride + (long long)(((g << shift) + (key & ((1 << shift) - 1))) * head_dim);
 }
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool ok) {        // not ok: zeros
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
@@ -100,17 +100,18 @@ prompt_attention_f32_kernel(const float* __restrict__ q, int q_stride, float* __
     const int lo = first_visible_key(pos0, window);
     const int* bt = block_table + (size_t)(item_row ? item_row[item] : item) * bt_stride;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ty = lane >> 3, tx = lane & 7;
+    const int shift = 31 - __clz(page_size);
 
     for (int c = tid; c < BQ * PIECES; c += PROMPT_THREADS) {
         const int r = c / PIECES, d = (c % PIECES) * 4;
         const bool ok = r < rows && d < head_dim;
         copy16(q_s + r * ROW + d, q + (ok ? (size_t)(tok0 + r) * q_stride + h * head_dim + d : 0), ok);
     }
-    auto load = [&](int tile, const float* pool, long long shift, float* to) {
+    auto load = [&](int tile, const float* pool, long long beyond, float* to) {
         for (int c = tid; c < BKEY * PIECES; c += PROMPT_THREADS) {
             const int r = c / PIECES, d = (c % PIECES) * 4, key = tile * BKEY + r;
-            const long long at = key >= lo && key <= hi && d < head_dim ? row_offset(bt, key, page_size, page_stride, g, head_dim) : -1;
-            copy16(to + r * ROW + d, pool + (at >= 0 ? at + shift + d : 0), at >= 0);
+            const long long at = key >= lo && key <= hi && d < head_dim ? row_offset(bt, key, shift, page_stride, g, head_dim) : -1;
+            copy16(to + r * ROW + d, pool + (at >= 0 ? at + beyond + d : 0), at >= 0);
         }
     };
     const int first = lo / BKEY, last = hi / BKEY;
@@ -252,6 +253,7 @@ token_attention_f32_kernel(const float* __restrict__ q, int q_stride, float* __r
     const int p = positions[t], lo = first_visible_key(p, window);
     const int* bt = block_table + (size_t)token_row[t] * bt_stride;
     const bool inside = d < head_dim;
+    const int shift = 31 - __clz(page_size);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 query = inside ? *reinterpret_cast<const float4*>(q + (size_t)t * q_stride + h * head_dim + d) : zero;
     float m = -INFINITY, l = 0.f;
@@ -263,7 +265,7 @@ token_attention_f32_kernel(const float* __restrict__ q, int q_stride, float* __r
         for (int u = 0; u < UNROLL; ++u) {
             const int key = round + (u * TOKEN_WARPS + warp) * GROUPS + group;
             seen[u] = key >= lo && key <= p;
-            const long long at = seen[u] ? row_offset(bt, key, page_size, page_stride, g, head_dim) : -1;
+            const long long at = seen[u] ? row_offset(bt, key, shift, page_stride, g, head_dim) : -1;
             k[u] = at >= 0 && inside ? *reinterpret_cast<const float4*>(k_pool + at + d) : zero;
             v[u] = at >= 0 && inside ? *reinterpret_cast<const float4*>(v_pool + at + to_value + d) : zero;
         }
