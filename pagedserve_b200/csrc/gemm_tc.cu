@@ -213,8 +213,9 @@ template <int BN, bool PAIR> struct Config {
 // PAIR: clusters of two CTAs (2, 1, 1) that work on one tile of 256 rows x BN columns together (tcgen05 cta_group::2): a CTA
 // fetches its 128 rows of A and half of the tile's rows of W and keeps the accumulators of its rows; the first CTA issues
 // the MMAs, its barriers count the copies of both, and its commits arrive in both.  Per output a third fewer bytes enter
-// shared memory than with 128 x 256 tiles, which are bound by that memory's bandwidth (48 KB in and as much read per k-block
-// of 512 clocks): 5,824 x 4,800 x 1,600 69.7 -> 63.8 us (1.40 PFLOP/s), 4,099 x 8,192 x 2,048 109 -> 101.
+// shared memory than with 128 x 256 tiles (4,099 x 8,192 x 2,048: 1.51 -> 1.17 GB through L2, shared memory 64 -> 51 % busy) and
+// the tensor pipe is active 82 instead of 74 % of the time: 109 -> 101 us; 5,824 x 4,800 x 1,600 69.7 -> 63.8 us (1.40
+// PFLOP/s, where the card's power limit is near).
 // GATED: the first half of a tile's rows of W are gates, the second the ups of the same output columns, and the epilogue forms
 // their activation from the two halves of the accumulator: the products' columns are never stored (the kernel that formed
 // the activation from them took 28 us for 8,198 rows of 2 x 2,048, beside 75 MB written and read again).
