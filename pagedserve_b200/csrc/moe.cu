@@ -28,7 +28,8 @@
 // from E * F on to the shared expert.  Products in float32, rounded once.
 //
 // With many tokens the rows are sorted by expert instead (moe_plan, moe_gather, the products over tiles that
-// choose their expert's matrix, the first with the activation in its epilogue, moe_combine): every token passes only through its own experts.
+// choose their expert's matrix, the first with the activation in its epilogue or, where that has few tiles, with moe_gate_mul_rows
+// behind it, moe_combine): every token passes only through its own experts.
 #include "common.cuh"
 
 namespace ps {
@@ -421,6 +422,47 @@ moe_gather_kernel(const T* __restrict__ x, int x_stride, const int* __restrict__
     for (int c = threadIdx.x; c < W; c += blockDim.x) dst[c] = t < 0 ? from_float<T>(0.f) : src[c];
 }
 
+// inner[r, j] = silu(gate_up[r, j]) * gate_up[r, F + j] * row_weight[r], or the other form of GateForm
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_gate_mul_rows_kernel(const T* __restrict__ gate_up, int gu_stride, const float* __restrict__ row_weight,
+                         T* __restrict__ inner, int inner_stride, int rows, int F, int by8, GateForm form) {
+    pdl_prologue();
+    gate_up = pdl_fresh(gate_up);
+    row_weight = pdl_fresh(row_weight);
+    const long long total = (long long)rows * F;
+    if (by8) {
+        const int groups = F >> 3;
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)rows * groups;
+             i += (long long)gridDim.x * blockDim.x) {
+            const int r = (int)(i / groups), j = (int)(i - (long long)r * groups) << 3;
+            const float w = row_weight[r];
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (w != 0.f) {
+                const T* row = gate_up + (size_t)r * gu_stride;
+                float g[8], u[8];
+                load8(row + j, g);
+                load8(row + F + j, u);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = gated_inner(g[k], u[k], w, form.kind, form.limit, form.alpha);
+            }
+            store8(inner + (size_t)r * inner_stride + j, v);
+        }
+        return;
+    }
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int r = (int)(i / F), j = (int)(i - (long long)r * F);
+        const float w = row_weight[r];
+        float v = 0.f;
+        if (w != 0.f) {
+            const T* row = gate_up + (size_t)r * gu_stride;
+            v = gated_inner(to_float(row[j]), to_float(row[F + j]), w, form.kind, form.limit, form.alpha);
+        }
+        inner[(size_t)r * inner_stride + j] = from_float<T>(v);
+    }
+}
+
 // y[t] += sum over k (in rising order) of down[row_of[t * top + k]]; with weights, factor * sum of weight[t * top + k] *
 // down[...] (factor: one number per column, null: 1)
 __global__ void __launch_bounds__(256)
@@ -578,6 +620,29 @@ PS_EXPORT int ps_moe_gather(const void* x, int x_stride, const int* row_token, v
     if (dtype == PS_BF16)
         return ps::launch_pdl(ps::moe_gather_kernel<__nv_bfloat16>, dim3(R), dim3(128), 0, s, (const __nv_bfloat16*)x,
                               x_stride, row_token, (__nv_bfloat16*)rows, rows_stride, W, by16);
+    return PS_ERR_UNSUPPORTED;
+}
+
+// gate_up [R, 2 F] (gate columns, then up columns); row_weight float32 [R]; inner [R, F]
+PS_EXPORT int ps_moe_gate_mul_rows(const void* gate_up, int gu_stride, const float* row_weight, void* inner,
+                                   int inner_stride, int R, int F, int dtype, int kind, float limit, float alpha,
+                                   void* stream) {
+    if (R <= 0 || F <= 0) return PS_OK;
+    if (!gate_up || !row_weight || !inner) return PS_ERR_BAD_ARGUMENT;
+    if (kind < 0 || kind > 2 || (kind == 1 && !(limit > 0.f))) return PS_ERR_BAD_ARGUMENT;
+    const ps::GateForm form{kind, limit, limit, alpha};
+    cudaStream_t s = (cudaStream_t)stream;
+    const int by8 = F % 8 == 0 && gu_stride % 8 == 0 && inner_stride % 8 == 0 && !((uintptr_t)gate_up & 31) &&
+                    !((uintptr_t)inner & 31);
+    const long long blocks = ((long long)R * (by8 ? F / 8 : F) + 255) / 256;
+    const dim3 grid((unsigned)(blocks < 4736 ? blocks : 4736));
+    if (dtype == PS_F32)
+        return ps::launch_pdl(ps::moe_gate_mul_rows_kernel<float>, grid, dim3(256), 0, s, (const float*)gate_up,
+                              gu_stride, row_weight, (float*)inner, inner_stride, R, F, by8, form);
+    if (dtype == PS_BF16)
+        return ps::launch_pdl(ps::moe_gate_mul_rows_kernel<__nv_bfloat16>, grid, dim3(256), 0, s,
+                              (const __nv_bfloat16*)gate_up, gu_stride, row_weight, (__nv_bfloat16*)inner, inner_stride,
+                              R, F, by8, form);
     return PS_ERR_UNSUPPORTED;
 }
 

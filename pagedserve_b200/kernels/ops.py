@@ -119,6 +119,7 @@ _SIGNATURES = {
         "ps_head_mix": [_P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _P],
         "ps_moe_plan": [_P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
         "ps_moe_gather": [_P, _I, _P, _P, _I, _I, _I, _I, _P],
+        "ps_moe_gate_mul_rows": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P],
         "ps_moe_combine": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P],
         "ps_step_shape": [_I, _P, _P, _P, _I, _I, _I, _I, _P],
         "ps_step_fill": [_I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _L, _P, _I, _I, _I, _I, _P],
@@ -1777,6 +1778,22 @@ class Ops:
                                        rows.shape[0], x.shape[1], self.code, _stream()), "moe_gather")
         return rows
 
+    def moe_gate_mul_rows(self, gate_up, row_weight, inner, form=None):
+        """inner[r, j] = silu(gate_up[r, j]) * gate_up[r, F + j] * row_weight[r], or the other ``form`` of
+        :meth:`_gate_form` (with the routed experts' limit)."""
+        R, F = inner.shape
+        _require(gate_up, "gate_up", self.dtype)
+        _require(inner, "inner", self.dtype)
+        _require(row_weight, "row_weight", torch.float32)
+        if gate_up.shape != (R, 2 * F) or row_weight.numel() != R or gate_up.stride(1) != 1 or inner.stride(1) != 1:
+            raise KernelError("moe_gate_mul_rows: shapes do not match")
+        self.launches += 1
+        kind, limit, _, alpha = self._gate_form(form)
+        _check(self.core.ps_moe_gate_mul_rows(_ptr(gate_up), gate_up.stride(0), _ptr(row_weight), _ptr(inner),
+                                              inner.stride(0), R, F, self.code, kind, limit, alpha, _stream()),
+               "moe_gate_mul_rows")
+        return inner
+
     def moe_combine(self, down, row_of, top, y, weights=None, factor=None):
         """y[t] += sum_k down[row_of[t * top + k]] (float32; k in rising order, rows < 0 skipped); with ``weights`` float32
         [T, top], y[t] += factor * sum_k weights[t, k] * down[...] (``factor`` float32, one number per column, or None)."""
@@ -1827,6 +1844,17 @@ class Ops:
         return (self.dtype == torch.bfloat16 and a.shape[0] > 64 and inner.shape[1] % 8 == 0 and inner.stride(0) % 8 == 0
                 and inner.stride(1) == 1 and a.stride(1) == 1 and w.stride(1) == 1 and inner.data_ptr() % 16 == 0
                 and self.tc_ok(a, w))
+
+    GATED_TILE = 128              # rows, and columns of results, of a tile of the gated product
+
+    def gated_pays(self, rows, columns):
+        """Whether :meth:`linear_gated` is the faster way to ``rows`` x ``columns`` inner numbers: where its tiles are more than a
+        third of the SMs.  They are 256 wide (gates and ups), so with fewer of them SMs are idle that the narrower tiles of the
+        plain product would use, and a CTA forms a whole tile's activation alone.  Us, product and gate kernel / one product:
+        256 x 1,024 x 1,024 (16 tiles) 10.2 / 12.5, 512 x 512 x 512 (16) 7.6 / 9.4, 256 x 2,048 x 2,048 (32) 17.5 / 18.2, 384 x
+        2,048 x 2,048 (48) 18.2 / 17.9, 900 x 1,024 x 1,024 (64) 12.8 / 12.5, 1,024 x 2,048 x 1,024 (128) 16.3 / 13.1; four
+        experts of 1,024 x 1,024, rows of their runs: 768 (48) 12.6 / 13.3, 1,280 (80) 15.8 / 13.6."""
+        return 3 * -(-rows // self.GATED_TILE) * -(-columns // self.GATED_TILE) > 148
 
     def linear_gated(self, a, w, inner, form=None, row_weight=None, tile_expert=None, experts=1):
         """inner[m, n] = the gated activation ``form`` (:meth:`_gate_form`; of a clamped one the routed experts' limit where

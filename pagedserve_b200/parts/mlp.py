@@ -15,8 +15,8 @@ class DenseMLP(FeedForward):
     """residual += act(x W_up + b_up) W_down + b_down
     (reference: src/model/paged_decoder.py:178-179, 224-228, 273-280),
     or, with ``gate_name``, the gated form residual += (act(x W_gate) * (x W_up)) W_down (activation 'silu' or
-    'gelu_tanh', no biases): gate and up run as one product over the stacked matrices; many rows of it form the inner row in the product's epilogue, few
-    rows in an elementwise kernel.
+    'gelu_tanh', no biases): gate and up run as one product over the stacked matrices, with many rows with the inner row formed in
+    the product's epilogue, with few in an elementwise kernel.
     params: hidden_size, inner_size, activation ('gelu_tanh' | 'gelu_erf' | 'relu_squared' = max(z, 0)^2 | 'silu'),
     has_bias,
     stored_in_out, up_name, down_name, gate_name (None), init_std, out_init_std."""
@@ -71,7 +71,7 @@ class DenseMLP(FeedForward):
         inner = ops.empty((x.shape[0], p["inner_size"]), self.env.dtype, x.device)
         if self.w_gate_up is not None and x.shape[0] > 64 and hasattr(x, "materialize"):
             x = x.materialize()                  # (the norm is folded into products of few rows only)
-        if self.w_gate_up is not None and x.shape[0] > 64 and ops.gated_ok(x, self.w_gate_up, inner):
+        if self.w_gate_up is not None and ops.gated_pays(*inner.shape) and ops.gated_ok(x, self.w_gate_up, inner):
             ops.linear_gated(x, self.w_gate_up, inner, form=p["activation"])
         elif self.w_gate_up is not None:
             gate_up = ops.empty((x.shape[0], 2 * p["inner_size"]), self.env.dtype, x.device)

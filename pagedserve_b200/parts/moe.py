@@ -37,10 +37,12 @@ class RoutedExperts(FeedForward):
     token passes through every expert's columns: the weights stream once, which is what bounds such a step.
     Many tokens in bfloat16: the (token, expert) pairs are sorted by expert into a buffer in which every expert's
     run starts on a tile of the tcgen05 product (``moe_plan``, ``moe_gather``); the two products read, per tile of
-    rows, the matrix of that tile's expert (``linear_gated`` with the activation, ``linear_experts``); ``moe_combine`` adds each token's rows into the
+    rows, the matrix of that tile's expert: ``linear_gated`` with the activation (or ``linear_experts`` and
+    ``moe_gate_mul_rows`` where that has too few tiles), then ``linear_experts``; ``moe_combine`` adds each token's rows into the
     residual in the order of its election.  The shared expert runs as two plain products beside them.
-    Either way a token's result does not depend on the other tokens of the step, and both ways compute the same
-    sums up to their order.
+    Which way a step takes depends on its shape alone, and a token's result does not depend on the election of the others.  The
+    ways compute the same sums up to their order and to where gates and ups are rounded: to bfloat16 between a product and
+    the gate kernel, not at all in ``linear_gated``, whose result is the nearer one.
 
     params: hidden_size, n_experts, expert_ff, top, groups, group_keep, shared_ff (None: no shared expert),
     score ("softmax"), normalize (True), group_mark ("largest"), weight_scale (1), expert_form (None: silu), shared_limit, shared_gate (True),
@@ -174,8 +176,13 @@ class RoutedExperts(FeedForward):
             ops.linear_experts(inner, self.w_down, down, tile_expert, E, along_k=True)
             ops.moe_combine(down, row_of, top, residual, weights=chosen_w, factor=self.result_factor)
             return
-        ops.linear_gated(rows, self.w_gate_up[:E * 2 * F], inner, form=self.form, row_weight=row_weight, tile_expert=tile_expert,
-                         experts=E)
+        if ops.gated_pays(tokens * top + E * (ops.EXPERT_TILE // 2), F):          # (a run's last tile is half full on average)
+            ops.linear_gated(rows, self.w_gate_up[:E * 2 * F], inner, form=self.form, row_weight=row_weight, tile_expert=tile_expert,
+                             experts=E)
+        else:
+            gate_up = ops.empty((rows_cap, 2 * F), dtype, device)
+            ops.linear_experts(rows, self.w_gate_up[:E * 2 * F], gate_up, tile_expert, E)
+            ops.moe_gate_mul_rows(gate_up, row_weight, inner, form=self.form)
         ops.linear_experts(inner, self.w_down[:, :E * F], down, tile_expert, E, along_k=True)
         if self.result_factor is None:
             ops.moe_combine(down, row_of, top, residual)
@@ -185,7 +192,7 @@ class RoutedExperts(FeedForward):
         if shared_ff:
             inner_shared = ops.empty((tokens, shared_ff), dtype, device)
             w_shared = self.w_gate_up[E * 2 * F:]
-            if ops.gated_ok(x, w_shared, inner_shared):
+            if ops.gated_pays(tokens, shared_ff) and ops.gated_ok(x, w_shared, inner_shared):
                 ops.linear_gated(x, w_shared, inner_shared, form=self.form, row_weight=shared_gate)
             else:
                 gate_up_shared = ops.empty((tokens, 2 * shared_ff), dtype, device)
