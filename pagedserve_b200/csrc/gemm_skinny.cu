@@ -71,24 +71,26 @@ struct SkinnyGroups {
     int act_from = 0;
 };
 
-// MT: token tiles of 8. WARPS: warps per CTA. UNROLL: k steps whose loads a warp issues together (a round);
+// Most CTAs of an instance on an SM at once where rows are cut into blocks: the registers are bounded so that they are.
+constexpr int skinny_resident(int warps, int unroll) { return warps == 4 ? 4 : warps == 8 ? (unroll == 4 ? 3 : 2) : 1; }
+constexpr int SKINNY_BLOCK = 3;                            // most token tiles of a block
+
+// MT: token tiles of 8.  RESIDENT > 0: rows are cut into blocks of MT tiles (blockIdx.y), RESIDENT CTAs on an SM; 0: all rows. WARPS: warps per CTA. UNROLL: k steps whose loads a warp issues together (a round);
 // WARPS * UNROLL * 32 >= K makes it one round, so that the latency of the weights is paid once.
-template <int MT, int WARPS, int UNROLL, typename TOut>
-__global__ void __launch_bounds__(WARPS * 32)
+template <int MT, int WARPS, int UNROLL, typename TOut, int RESIDENT>
+__global__ void __launch_bounds__(WARPS * 32, RESIDENT)
 gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int ldw,
                    const float* __restrict__ bias, TOut* __restrict__ out, int ldo, int M, int N, int K,
                    int act, int accumulate, KvScatter kv, SkinnyGroups gr) {
     // cross-warp sums [WARPS][16][8*MT] floats, then the cache address of each row [8*MT] (64-bit)
     extern __shared__ __align__(16) float red[];
+    constexpr bool BLOCKS = RESIDENT > 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * 16;
-    const int first = blockIdx.y * 8 * MT;                // this CTA's rows of A: up to 8 MT of them from here on
-    A += (size_t)first * lda;
-    out += (size_t)first * ldo;
-    M = min(M - first, 8 * MT);
-    kv.positions += first;
-    kv.token_row += first;
+    // This CTA's rows: up to 8 MT from here on.  (Counted from the first of all, so that pointers stay where they came in: shifted
+    // ones took 6 to 10 registers more, and with those an SM held 3 CTAs of 128 threads instead of 4, or 1 of 256 instead of 2.)
+    const int first = BLOCKS ? (int)blockIdx.y * 8 * MT : 0;
     int n_shift = 0;                                      // the group's first column of the stacked weight
     if (gr.cols) {
         const int group = n0 / gr.cols;
@@ -104,7 +106,7 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bflo
     bool aok[MT];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
-        int m = 8 * mt + g;
+        int m = first + 8 * mt + g;
         aok[mt] = m < M;
         arow[mt] = A + (size_t)(aok[mt] ? m : 0) * lda + 8 * t;
     }
@@ -123,10 +125,10 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bflo
         pdl_prologue();
         if (kv.k_pool) {
             // where a row's keys and values go: offset of (page, head 0, position in page, 0), or -1
-            for (int m = threadIdx.x; m < M; m += WARPS * 32) {
+            for (int m = threadIdx.x; m < (BLOCKS ? min(M - first, TOK) : M); m += WARPS * 32) {
                 int index, within;
-                split_position(kv.positions[m], kv.page_size, &index, &within);
-                const int page = kv.block_table[(size_t)kv.token_row[m] * kv.bt_stride + index];
+                split_position(kv.positions[first + m], kv.page_size, &index, &within);
+                const int page = kv.block_table[(size_t)kv.token_row[first + m] * kv.bt_stride + index];
                 dst_s[m] = page >= 0 ? (long long)page * kv.page_stride + (long long)within * kv.head_dim : -1;
             }
         }
@@ -136,7 +138,7 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bflo
         for (int j = 0; j < EPT; ++j) {
             const int e = threadIdx.x + j * WARPS * 32;
             const int n = n0 + (e & 15), m = e >> 4;
-            prev[j] = ((accumulate & PS_ACCUMULATE) && e < 16 * TOK && m < M && n < N) ? to_float(out[(size_t)m * ldo + n - n_shift]) : 0.f;
+            prev[j] = ((accumulate & PS_ACCUMULATE) && e < 16 * TOK && first + m < M && n < N) ? to_float(out[(size_t)(first + m) * ldo + n - n_shift]) : 0.f;
         }
     };
     // the bias of this thread's output column (the same in every epilogue round: the CTA's thread count is a
@@ -191,7 +193,7 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bflo
         if (e >= 16 * TOK) break;
         int r = e & 15, m = e >> 4;           // weight row fastest: consecutive threads store consecutive n
         int n = n0 + r;
-        if (m >= M || n >= N) continue;
+        if (first + m >= M || n >= N) continue;
         float v = 0.f;
 #pragma unroll
         for (int w = 0; w < WARPS; ++w) v += red[(size_t)w * 16 * TOK + r * TOK + m];
@@ -204,33 +206,49 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bflo
             continue;
         }
         v += prev[j];
-        out[(size_t)m * ldo + n - n_shift] = from_float<TOut>(v);
+        out[(size_t)(first + m) * ldo + n - n_shift] = from_float<TOut>(v);
     }
 }
 
 // Token tiles of 8 rows in a CTA such that the CTAs of all blocks are resident at once, the fewest possible; 0: none of 1 to 3.
-// CTAs that are resident at once, by the instances of pick_warps: K up to 1,024, 3 per SM with one token tile (256 threads,
-// 80 registers) and 4 with two or three (128 threads); up to 2,048, 2 (256 threads); beyond, 1 (512 threads).
+// (skinny_resident, for the instances that pick_warps takes: K up to 1,024, 3 per SM with one token tile and 4 with two or three; up
+// to 2,048, 2; beyond, 1).
 inline int skinny_block(int M, int N, int K) {
     const int steps = (K + 31) / 32, tiles = (M + 7) / 8;
-    for (int block = 1; block <= 3 && block <= tiles; ++block) {
+    for (int block = 1; block <= SKINNY_BLOCK && block <= tiles; ++block) {
         const int resident = 148 * (steps <= 32 ? (block == 1 ? 3 : 4) : steps <= 64 ? 2 : 1);
         if ((N + 15) / 16 * ((tiles + block - 1) / block) <= resident) return block;
     }
     return 0;
 }
 
-template <int MT, int WARPS, int UNROLL, typename TOut>
-int launch_skinny(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo,
+template <int MT, int WARPS, int UNROLL, typename TOut, int RESIDENT>
+int launch_skinny_rows(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo,
                   int M, int N, int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s,
-                  const SkinnyGroups& gr = SkinnyGroups{}) {
+                  const SkinnyGroups& gr) {
     size_t smem = (size_t)WARPS * 16 * 8 * MT * sizeof(float) + (size_t)8 * MT * sizeof(long long);
-    auto kernel = gemm_skinny_kernel<MT, WARPS, UNROLL, TOut>;
+    auto kernel = gemm_skinny_kernel<MT, WARPS, UNROLL, TOut, RESIDENT>;
     static size_t raised[MAX_DEVICES] = {0};
     if (!ensure_dynamic_smem((const void*)kernel, smem, raised)) return PS_ERR_LAUNCH;
     return launch_pdl(kernel, dim3((N + 15) / 16, (M + 8 * MT - 1) / (8 * MT)), dim3(WARPS * 32), smem, s,
                       (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)W, ldw, bias, (TOut*)out, ldo, M, N, K, act,
                       accumulate, kv, gr);
+}
+
+template <int MT, int WARPS, int UNROLL, typename TOut>
+int launch_skinny(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo,
+                  int M, int N, int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s,
+                  const SkinnyGroups& gr = SkinnyGroups{}) {
+    if constexpr (MT <= SKINNY_BLOCK) {
+        constexpr int MOST = skinny_resident(WARPS, UNROLL);
+        if constexpr (MT > 1 && WARPS == 4) {              // with fewer CTAs each has more registers: 32 x 3,072 x 768 3.3 -> 3.1 us
+            if (M > 8 * MT && (N + 15) / 16 * ((M + 8 * MT - 1) / (8 * MT)) <= 148 * (MOST - 1))
+                return launch_skinny_rows<MT, WARPS, UNROLL, TOut, MOST - 1>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s, gr);
+        }
+        if (M > 8 * MT)
+            return launch_skinny_rows<MT, WARPS, UNROLL, TOut, MOST>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s, gr);
+    }
+    return launch_skinny_rows<MT, WARPS, UNROLL, TOut, 0>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s, gr);
 }
 
 template <int MT, typename TOut>
@@ -275,10 +293,11 @@ int pick_tiles(const void* A, int lda, const void* W, int ldw, const float* bias
                const SkinnyGroups& gr = SkinnyGroups{}) {
     // The MMAs of a CTA grow with its token tiles, and beyond a few of them they are what the kernel waits for (an SM issues
     // one in about 10 clocks): the rows are cut into blocks of as few token tiles as leave all CTAs resident at once
-    // (ps_gemm_skinny_block), each block reading the weights for itself from L2.  64 rows, us, all rows in one CTA / in
-    // blocks: 2,304 x 768 8.4 / 4.0, 768 x 768 7.5 / 2.4, 3,072 x 768 9.0 / 4.7, 768 x 3,072 12.1 / 4.5; 32 rows 4.6 / 3.1,
-    // 3.9 / 2.0, 5.2 / 3.4, 6.2 / 3.6.  With a second round of CTAs that is lost again (64 x 3,072 x 768 in blocks of 16
-    // rows, 768 CTAs: 6.9), so where no block fits a CTA keeps all rows: every count of tiles has its own instance.
+    // (ps_gemm_skinny_block), each block reading the weights for itself, from L2 behind the first.  Weights from memory, us, all rows in
+    // one CTA / in blocks: 64 rows 2,304 x 768 6.4 / 3.7, 768 x 768 5.5 / 2.4, 3,072 x 768 6.8 / 4.3, 768 x 3,072 12.1 / 4.6; 48 rows
+    // 3,072 x 1,024 6.6 / 5.2, 4,096 x 1,024 6.9 / 6.2; 32 rows 4.5 / 2.7, 3.8 / 1.9, 5.1 / 3.0, 6.1 / 3.6.  With a second round of
+    // CTAs that is lost again (64 x 3,072 x 768 in blocks of 16 rows, 768 CTAs: 6.8), so where no block fits a CTA keeps all
+    // rows: every count of tiles has its own instance.
 #define PS_TILES(MT_) \
     return pick_warps<MT_, TOut>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s, gr)
     const int block = skinny_block(M, N, K);
@@ -315,7 +334,7 @@ struct NormInput {
     int has_mean;
 };
 
-template <int MT, int WARPS, int UNROLL, typename TOut>
+template <int MT, int WARPS, int UNROLL, typename TOut, bool BLOCKS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS <= 8 ? 2 : 1)
 gemm_skinny_fused_kernel(NormInput in, const __nv_bfloat16* __restrict__ W, int ldw,
                          const float* __restrict__ bias, TOut* __restrict__ out, int ldo, int M, int N, int K,
@@ -324,13 +343,13 @@ gemm_skinny_fused_kernel(NormInput in, const __nv_bfloat16* __restrict__ W, int 
     // the cache address of each row [8*MT] (64-bit), then the normed rows [8*MT][K+8] bf16
     extern __shared__ __align__(16) float red[];
     constexpr int TOK = 8 * MT;
-    const int first = blockIdx.y * TOK;            // this CTA's rows: up to TOK of them from here on
-    if (in.rows) in.rows += first;
-    else in.x += (size_t)first * in.ldx;
-    out += (size_t)first * ldo;
-    M = min(M - first, TOK);
-    kv.positions += first;
-    kv.token_row += first;
+    const int first = BLOCKS ? (int)blockIdx.y * TOK : 0;  // this CTA's rows: up to TOK from here on
+    if constexpr (BLOCKS) {
+        if (in.rows) in.rows += first;
+        else in.x += (size_t)first * in.ldx;
+        out += (size_t)first * ldo;
+    }
+    if constexpr (BLOCKS) M = min(M - first, TOK);
     const int lda_s = K + 8;                       // padded: 16-byte reads of 8 rows hit 8 different bank groups
     float* gamma_s = red + (size_t)WARPS * 16 * TOK;
     float* beta_s = gamma_s + K;
@@ -376,8 +395,8 @@ gemm_skinny_fused_kernel(NormInput in, const __nv_bfloat16* __restrict__ W, int 
     const bool kv_row = kv.k_pool && threadIdx.x < M;
     int kv_p = 0, kv_table_row = 0;
     if (kv_row) {
-        kv_p = kv.positions[threadIdx.x];
-        kv_table_row = kv.token_row[threadIdx.x];
+        kv_p = kv.positions[first + threadIdx.x];
+        kv_table_row = kv.token_row[first + threadIdx.x];
     }
     pdl_prologue();            // the rows come from the kernel before this one
     int kv_page = -1, kv_index = 0, kv_within = 0;
@@ -555,11 +574,11 @@ inline size_t skinny_fused_smem(int MT, int WARPS, int K) {
            (size_t)8 * MT * (K + 8) * 2;
 }
 
-template <int MT, int WARPS, int UNROLL, typename TOut>
+template <int MT, int WARPS, int UNROLL, typename TOut, bool BLOCKS = false>
 int launch_skinny_fused(const NormInput& in, const void* W, int ldw, const float* bias, void* out, int ldo, int M,
                         int N, int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s) {
     size_t smem = skinny_fused_smem(MT, WARPS, K);
-    auto kernel = gemm_skinny_fused_kernel<MT, WARPS, UNROLL, TOut>;
+    auto kernel = gemm_skinny_fused_kernel<MT, WARPS, UNROLL, TOut, BLOCKS>;
     if (smem > 200 * 1024) return PS_ERR_UNSUPPORTED;
     static size_t raised[MAX_DEVICES] = {0};
     if (!ensure_dynamic_smem((const void*)kernel, smem, raised)) return PS_ERR_LAUNCH;
@@ -567,24 +586,28 @@ int launch_skinny_fused(const NormInput& in, const void* W, int ldw, const float
                       (const __nv_bfloat16*)W, ldw, bias, (TOut*)out, ldo, M, N, K, act, accumulate, kv);
 }
 
-template <int MT, typename TOut>
+template <int MT, typename TOut, bool BLOCKS = false>
 int pick_warps_fused(const NormInput& in, const void* W, int ldw, const float* bias, void* out, int ldo, int M, int N,
                      int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s) {
     // at least 8 warps: they also share the rows of the norm between them
     // UNROLL: the k steps of a warp whose weights are fetched before anything else
     int steps = (K + 31) / 32;
-    if (steps <= 24) return launch_skinny_fused<MT, 8, 3, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
-    if (steps <= 64) return launch_skinny_fused<MT, 8, 6, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
-    return launch_skinny_fused<MT, 16, 6, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    if (steps <= 24) return launch_skinny_fused<MT, 8, 3, TOut, BLOCKS>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    if (steps <= 64) return launch_skinny_fused<MT, 8, 6, TOut, BLOCKS>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    return launch_skinny_fused<MT, 16, 6, TOut, BLOCKS>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
 }
 
 template <typename TOut>
 int pick_tiles_fused(const NormInput& in, const void* W, int ldw, const float* bias, void* out, int ldo, int M, int N,
                      int K, int act, int accumulate, const KvScatter& kv, cudaStream_t s) {
-    if (M <= 8) return pick_warps_fused<1, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
-    // blocks of 16 rows where their CTAs are resident at once (2 per SM): a CTA norms only its own rows
-    if (M <= 16 || (N + 15) / 16 * ((M + 15) / 16) <= 2 * 148) return pick_warps_fused<2, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
-    return pick_warps_fused<4, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    // (One block too runs on the form for blocks, whose compiler knows that M is at most its rows: 8 x 2,304 x 768 3.2 -> 3.1 us, 32 x
+    // 3,072 x 1,024 16.9 -> 15.6; but for two token tiles, where it costs: 16 x 1,024 x 1,024 4.8 -> 5.4.)
+    if (M <= 8) return pick_warps_fused<1, TOut, true>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    if (M <= 16) return pick_warps_fused<2, TOut>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    // blocks of 16 rows where their CTAs are resident at once (2 per SM, beyond K of 2,048 1): a CTA norms only its own rows
+    if ((N + 15) / 16 * ((M + 15) / 16) <= (K <= 2048 ? 2 : 1) * 148)
+        return pick_warps_fused<2, TOut, true>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
+    return pick_warps_fused<4, TOut, true>(in, W, ldw, bias, out, ldo, M, N, K, act, accumulate, kv, s);
 }
 
 

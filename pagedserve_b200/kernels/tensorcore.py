@@ -23,8 +23,9 @@ def prefers_rows(ops, a, w) -> bool:
     64 x 4,800 x 1,600: 25.1 / 12.0 / 12.1;  64 x 1,600 x 6,400: 23.0 / 12.1 / 33.1;  33 x 4,800 x 1,600: 13.0 /
     10.7 / 12.2;  64 x 50,257 x 768: 73.9 / 35.6 / 45.5;  33 x 50,257 x 768: 35.6 / 31.5 / 30.6.
     Those are the weight-streaming kernel's times with all rows in one CTA; where it takes them in blocks whose CTAs are all
-    resident at once it wins (64 rows, us, blocks / few-rows tcgen05: 2,304 x 768 4.0 / 7.1, 768 x 768 2.4 / 6.6, 3,072 x 768
-    4.7 / 6.7, 768 x 3,072 4.5 / 8.1; 48 x 4,096 x 1,024 6.4 / 7.4, 48 x 1,024 x 4,096 6.2 / 9.0).
+    resident at once it wins (weights from memory, us, blocks / few-rows tcgen05: 64 rows 2,304 x 768 3.7 / 7.2, 768 x 768
+    2.4 / 6.0, 3,072 x 768 4.3 / 6.7, 768 x 3,072 4.6 / 7.5, 3,072 x 1,024 6.1 / 7.3; 48 rows 4,096 x 1,024 6.2 / 7.5, 1,024 x 4,096
+    6.6 / 8.7; 40 rows 1,600 x 1,600 5.3 / 7.2).
     The rule depends on the shapes alone, so that the same step always runs the same kernels."""
     rows, columns, depth = a.shape[0], w.shape[0], a.shape[1]
     if not (32 < rows <= 64) or not ops.tc_ok(a, w) or ops.skinny_in_blocks(a, w):
@@ -39,7 +40,7 @@ def prefers_tc(ops, a, w) -> bool:
     every CTA (16 output columns): from 17 rows on and 4,096 columns up (a vocabulary, the wide projections of
     large models) that traffic costs more than the half-empty 128-row tiles of the tcgen05 kernel (64 rows x
     50,257 x 768: 46 vs 85 us; 64 x 4,800 x 1,600: 12 vs 37 us; 16 rows: the streaming kernel wins at every
-    shape), unless it takes them in blocks (32 x 4,096 x 1,024: 5.3 us, 8.0 here)."""
+    shape), unless it takes them in blocks (32 x 4,096 x 1,024: 5.1 us, 8.1 here)."""
     if not ops.tc_ok(a, w) or prefers_rows(ops, a, w):
         return False
     return (a.shape[0] > 16 and w.shape[0] >= 4096 and not ops.skinny_in_blocks(a, w)) or not ops.skinny_ok(a, w)

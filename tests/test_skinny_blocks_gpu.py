@@ -68,3 +68,53 @@ def test_fused_norm_in_blocks(M, scatter):
         # rounded bfloat16 results of float32 sums in two orders: half a step of the largest at most, and then one
         assert float((out.float() - want.float()).abs().max()) <= 2.0 ** -7 * float(want.float().abs().max())
     engine.cache.check_invariants()
+
+
+@pytest.mark.parametrize("M", [8, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(768, 1024), (2400, 1024), (768, 2048), (768, 2080), (2384, 2080)])
+def test_fused_norm_at_depths(M, N, K):
+    """Depths on both sides of where an SM holds two CTAs and one, widths on both sides of where blocks of 16 rows are resident."""
+    ops, g = ops_for(), torch.Generator().manual_seed(M + N + K)
+    x, gamma, beta = torch.randn(M, K, generator=g) * 2 + 0.5, torch.randn(K, generator=g) * 0.2 + 1, torch.randn(K, generator=g) * 0.2
+    w = (torch.randn(N, K, generator=g) / K ** 0.5).to(torch.bfloat16)
+    x, gamma, beta, w = (t.to(DEV) for t in (x, gamma, beta, w))
+    prologue = SimpleNamespace(weight=gamma, bias=beta, eps=1e-5, has_mean=True)
+    rows = SimpleNamespace(x=x, rows=None, shape=x.shape, norm=SimpleNamespace(fused_prologue=lambda: prologue))
+    out = torch.empty(M, N, device=DEV)
+    ops.linear_skinny_fused(rows, w, None, out)
+    normed = torch.nn.functional.layer_norm(x.double(), (K,), gamma.double(), beta.double(), 1e-5).to(torch.bfloat16)
+    want = normed.double() @ w.double().T
+    # a normed number that lies between two bfloat16 values may round either way: one step of 2^-8 of it, in one of K terms
+    assert float((out.double() - want).abs().max()) < 2.0 ** -8 * 4 / K ** 0.5 * 4 + 2e-5 * float(want.abs().max())
+
+
+def milliseconds(calls):
+    for call in calls:
+        call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for call in calls:
+            call()
+    times = []
+    for _ in range(8):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        graph.replay()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(start.elapsed_time(end))
+    return min(times[2:])
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 3072, 768), (48, 3072, 1024), (64, 3072, 1024), (48, 4096, 1024), (40, 1600, 1600)])
+def test_blocks_are_taken_where_they_win(M, N, K):
+    """Weights that come from memory: the product takes blocks only where they beat the few-rows tcgen05 kernel and one CTA for all
+    rows.  With registers for fewer CTAs on an SM than the rule counts on, they lost by 8 to 28 % at these sizes."""
+    ops = ops_for()
+    a = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    weights = [(torch.randn(N, K, device=DEV) / K ** 0.5).to(torch.bfloat16) for _ in range(1 + int(260e6) // (2 * N * K))]
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    chosen = milliseconds([lambda w=w: ops.linear(a, w, None, out) for w in weights])
+    few = milliseconds([lambda w=w: ops.linear_rows_tc(a, w, None, out) for w in weights])
+    assert chosen < 1.03 * few
