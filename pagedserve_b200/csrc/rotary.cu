@@ -38,7 +38,8 @@ __device__ __forceinline__ P turned_pair(const float2& ab, float cs, float sn) {
     return pair_from_float<P>(fmaf(ab.x, cs, -(ab.y * sn)), fmaf(ab.y, cs, ab.x * sn));
 }
 
-template <typename T>
+// PIECES: a thread takes whole pieces of 16 bytes (rotary_by_pieces says when), else pairs or single numbers.
+template <typename T, bool PIECES>
 __global__ void __launch_bounds__(256)
 rotary_cache_write_kernel(T* __restrict__ q, int q_stride, const T* __restrict__ k, int k_stride,
                           const T* __restrict__ v, int v_stride, const float* __restrict__ inv_freq, int rot_dims,
@@ -59,13 +60,9 @@ rotary_cache_write_kernel(T* __restrict__ q, int q_stride, const T* __restrict__
         const int page = block_table[(size_t)token_row[t] * bt_stride + p / page_size];
         if (page >= 0) page_base = (long long)page * page_stride + (long long)(p % page_size) * head_dim;
     }
-    // Neighbouring pairs, sizes, strides and addresses in whole pieces of 16 bytes: a thread takes a piece of a head at a time (the
-    // pieces of a query head that turn, all pieces of a key head), the first one fetched beside the sines and cosines.
-    // Bound by the bytes: 4,087 tokens of 16 + 16 heads of 128, half of each turning, 8 us less than pair by pair (29.8).
+    // By pieces: those of a query head that turn, all pieces of a key head, the first one fetched beside the sines and cosines.
+    // Bound by the bytes: 4,087 tokens of 16 + 16 heads of 128, half of each turning, 27.9 us pair by pair, 15.2 by pieces.
     constexpr int VEC = 16 / (int)sizeof(T);
-    const bool by_pieces = interleaved && head_dim % VEC == 0 && rot_dims % VEC == 0 && q_stride % VEC == 0 && k_stride % VEC == 0 &&
-                           v_stride % VEC == 0 && page_stride % VEC == 0 &&
-                           !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15);
     const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
     const int q_pieces = rot_dims / VEC, all_pieces = head_dim / VEC, total_q = n_heads * q_pieces;
     const int total_pieces = total_q + (page_base >= 0 ? n_kv_heads * all_pieces : 0);
@@ -81,7 +78,7 @@ rotary_cache_write_kernel(T* __restrict__ q, int q_stride, const T* __restrict__
         const T* from = (idx < total_q ? q + (size_t)t * q_stride : k + (size_t)t * k_stride) + head * head_dim + d;
         piece = *reinterpret_cast<const uint4*>(from);
     };
-    if (by_pieces && first < total_pieces) fetch(first);
+    if (PIECES && first < total_pieces) fetch(first);
     // a token's sines and cosines are the same for every head: once into shared memory
     __shared__ float2 turn[ROTARY_MAX_PAIRS];
     const float pos = (float)p;
@@ -91,7 +88,7 @@ rotary_cache_write_kernel(T* __restrict__ q, int q_stride, const T* __restrict__
         turn[unit] = make_float2(cs, sn);
     }
     __syncthreads();
-    if (by_pieces) {
+    if constexpr (PIECES) {
         using P = typename PairOf<T>::type;
         for (int idx = first; idx < total_pieces; idx += step) {
             if (idx != first) fetch(idx);
@@ -195,6 +192,19 @@ rotary_cache_write_kernel(T* __restrict__ q, int q_stride, const T* __restrict__
     }
 }
 
+// Whether a launch goes by pieces: neighbouring pairs, sizes, strides and addresses in whole pieces of 16 bytes, and at least half a
+// megabyte of numbers to turn or to copy.  Below that a thread has one or two pairs anyway and the pieces' longer chain shows: 32 tokens of
+// 16 + 16 heads of 128 2.4 us pair by pair, 2.6 by pieces, 64 tokens (0.65 MB) 3.2 / 2.9; 16 + 4 heads of 64, 64 tokens (0.13 MB) 2.5 / 2.7,
+// 256 (0.52 MB) 3.4 / 3.0; 8 + 1 heads of 64, 256 tokens (0.33 MB) 2.5 / 2.7, 1,024 (1.3 MB) 3.8 / 3.6.
+inline bool rotary_by_pieces(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, int rot_dims,
+                             int interleaved, const void* k_pool, const void* v_pool, long long page_stride, int T, int n_heads,
+                             int n_kv_heads, int head_dim, int size) {
+    const int vec = 16 / size;
+    const long long numbers = (long long)T * ((long long)n_heads * rot_dims + (k_pool ? 2ll * n_kv_heads * head_dim : 0));
+    return numbers * size >= 512 * 1024 && interleaved && head_dim % vec == 0 && rot_dims % vec == 0 && q_stride % vec == 0 &&
+           k_stride % vec == 0 && v_stride % vec == 0 && page_stride % vec == 0 &&
+           !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15);
+}
 
 // ---- the same step for heads that are normed before they turn ----
 // Per head, over its first `dim` numbers (a head occupies `head_dim` >= dim numbers of its row; what lies behind
@@ -558,13 +568,16 @@ PS_EXPORT int ps_rotary_cache_write(void* q, int q_stride, const void* k, int k_
     const int threads = work >= 256 ? 256 : (work >= 128 ? 128 : 64);
     // a step of few tokens is bound by the chain of loads of one thread: spread a token over several CTAs
     const int split = T >= 512 ? 1 : (work + threads - 1) / threads;
+    const bool pieces = ps::rotary_by_pieces(q, q_stride, k, k_stride, v, v_stride, rot_dims, interleaved, k_pool, v_pool, page_stride, T,
+                                             n_heads, n_kv_heads, head_dim, dtype == PS_F32 ? 4 : 2);
     if (dtype == PS_F32)
-        return ps::launch_pdl(ps::rotary_cache_write_kernel<float>, dim3(T, split), dim3(threads), 0, s, (float*)q, q_stride,
+        return ps::launch_pdl(pieces ? ps::rotary_cache_write_kernel<float, true> : ps::rotary_cache_write_kernel<float, false>, dim3(T, split), dim3(threads), 0, s, (float*)q, q_stride,
                               (const float*)k, k_stride, (const float*)v, v_stride, inv_freq, rot_dims, interleaved,
                               token_row, positions, block_table, bt_stride, (float*)k_pool, (float*)v_pool,
                               page_stride, n_heads, n_kv_heads, head_dim, page_size);
     if (dtype == PS_BF16)
-        return ps::launch_pdl(ps::rotary_cache_write_kernel<__nv_bfloat16>, dim3(T, split), dim3(threads), 0, s,
+        return ps::launch_pdl(pieces ? ps::rotary_cache_write_kernel<__nv_bfloat16, true> : ps::rotary_cache_write_kernel<__nv_bfloat16, false>,
+                              dim3(T, split), dim3(threads), 0, s,
                               (__nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k, k_stride,
                               (const __nv_bfloat16*)v, v_stride, inv_freq, rot_dims, interleaved, token_row, positions,
                               block_table, bt_stride, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, page_stride,
