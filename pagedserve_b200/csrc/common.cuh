@@ -31,6 +31,7 @@
 // what its vector of one number per column (`bias`) is, a factor on the column instead of a summand
 #define PS_ACCUMULATE 1
 #define PS_COLUMN_FACTOR 2
+#define PS_WEIGHTS_READY 4           // the weights were complete before the kernel in front began: they may be read before the wait
 
 #define PS_EXPORT extern "C" __attribute__((visibility("default")))
 

@@ -143,15 +143,21 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
             copy_async<VEC>(to + (kb % STAGES) * STAGE + r * ROW, ok ? a_from + (size_t)r * lda + kb * BK : A, ok);
         }
     };
-    // the weights of the first stages do not depend on the kernel before this one
+    // weights that do not depend on the kernel before this one: those of the first stages go ahead of the wait
+    const bool ready = accumulate & PS_WEIGHTS_READY;
+    if (ready) {
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s)
-        if (s < blocks) load_weights(s);
+        for (int s = 0; s < STAGES - 1; ++s)
+            if (s < blocks) load_weights(s);
+    }
     pdl_prologue();
     a_from = pdl_fresh(a_from);
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < blocks) load_rows(s);
+        if (s < blocks) {
+            if (!ready) load_weights(s);
+            load_rows(s);
+        }
         copy_commit();
     }
     float acc[TM][TN];
@@ -261,10 +267,11 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
             w_s[my_k][r] = w_in[c].x; w_s[my_k + 1][r] = w_in[c].y; w_s[my_k + 2][r] = w_in[c].z; w_s[my_k + 3][r] = w_in[c].w;
         }
     };
-    fetch_weights(0);                                            // (they do not depend on the kernel before this one)
     pdl_prologue();
     a_from = pdl_fresh(a_from);
+    w_from = pdl_fresh(w_from);                                  // (the kernel in front may have made W too)
     fetch_rows(0);
+    fetch_weights(0);
     put(0);
     __syncthreads();
     unsigned long long acc[8][8];                                // row i, columns 2 j and 2 j + 1
@@ -333,9 +340,9 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
 template <int VEC>
 int run_tile(int tile, const float* A, int lda, const float* W, int ldw, const float* bias, float* out, int ldo, int M, int N, int K,
              int act, int accumulate, cudaStream_t s) {
-    if (tile == 1) return launch_tile<64, 64, 4, 8, 4, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
-    if (tile == 2) return launch_tile<32, 64, 4, 4, 5, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
-    if (tile == 3) return launch_tile<32, 32, 2, 4, 6, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
+    if (tile == 2) return launch_tile<64, 64, 4, 8, 4, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
+    if (tile == 3) return launch_tile<32, 64, 4, 4, 5, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
+    if (tile == 4) return launch_tile<32, 32, 2, 4, 6, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
     return launch_tile<32, 16, 2, 2, 8, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
 }
 
@@ -344,18 +351,21 @@ int run_tile(int tile, const float* A, int lda, const float* W, int ldw, const f
 // leave fewer SMs idle.  384 x 2,304 x 768: 54 us with 64 x 64 tiles, 41 with 32 x 64, 72 with 32 x 32; 128 x 768 x 768:
 // 36 / 24 / 15 / 15; 2,048 x 768 x 768: 73 / 81 / 108 / 130 (95 with 128 x 128).
 int pick_tile(const float* A, int lda, const float* W, int ldw, const float* bias, float* out, int ldo, int M, int N, int K,
-              int act, int accumulate, cudaStream_t s) {
+              int act, int accumulate, int tile, cudaStream_t s) {
     const bool aligned = (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && lda % 4 == 0 && ldw % 4 == 0 && K % 4 == 0;
     constexpr int rows[5] = {128, 64, 32, 32, 32}, columns[5] = {128, 64, 64, 32, 16};
     constexpr float fixed[5] = {24.f, 15.f, 10.f, 3.f, 4.f}, each[5] = {64.f, 21.5f, 13.3f, 11.4f, 6.3f};
-    int tile = 1;
-    float least = 0.f;
-    for (int t = aligned && M >= WIDE && N >= WIDE && K % WIDE_K == 0 ? 0 : 1; t < 5; ++t) {
-        const long long ctas = (long long)((M + rows[t] - 1) / rows[t]) * ((N + columns[t] - 1) / columns[t]);
-        const float cost = fixed[t] + each[t] * (float)((ctas + 147) / 148);
-        if (least == 0.f || cost < least) { least = cost; tile = t; }
+    const bool wide = aligned && M >= WIDE && N >= WIDE && K % WIDE_K == 0;
+    if (tile < 0 || tile > 5 || (tile == 1 && !wide)) return PS_ERR_UNSUPPORTED;
+    if (tile == 0) {
+        float least = 0.f;
+        for (int t = wide ? 0 : 1; t < 5; ++t) {
+            const long long ctas = (long long)((M + rows[t] - 1) / rows[t]) * ((N + columns[t] - 1) / columns[t]);
+            const float cost = fixed[t] + each[t] * (float)((ctas + 147) / 148);
+            if (least == 0.f || cost < least) { least = cost; tile = t + 1; }
+        }
     }
-    if (tile == 0)
+    if (tile == 1)
         return launch_pdl(gemm_f32_wide_kernel, dim3((N + WIDE - 1) / WIDE, (M + WIDE - 1) / WIDE), dim3(WIDE_THREADS), 0, s, A, lda,
                           W, ldw, bias, out, ldo, M, N, K, act, accumulate);
     if (aligned) return run_tile<4>(tile, A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
@@ -572,17 +582,20 @@ int launch_rows(const float* A, int lda, const float* W, int ldw, const float* b
 }  // namespace ps
 
 // in_dtype: dtype of A and W. out_dtype: dtype of out. accumulate: PS_ACCUMULATE: out += result (out must be f32);
-// PS_COLUMN_FACTOR: the numbers of `bias` multiply the columns.
+// PS_COLUMN_FACTOR: the numbers of `bias` multiply the columns; PS_WEIGHTS_READY: float32 weights may be read before the kernel in
+// front has ended.  tile: 0 = choose; float32: 1 to 5 = tiles of 128 x 128 (M and N at least 128, K a multiple of 16, 16-byte rows),
+// 64 x 64, 32 x 64, 32 x 32, 32 x 16.
 PS_EXPORT int ps_gemm_simt(const void* A, int lda, const void* W, int ldw, const float* bias, void* out,
                            int ldo, int M, int N, int K, int in_dtype, int out_dtype, int act,
-                           int accumulate, void* stream) {
+                           int accumulate, int tile, void* stream) {
     if (M <= 0 || N <= 0) return PS_OK;
     if (K <= 0 || lda < K || ldw < K || ldo < N) return PS_ERR_BAD_ARGUMENT;
     if ((accumulate & PS_ACCUMULATE) && out_dtype != PS_F32) return PS_ERR_BAD_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
     using bf = __nv_bfloat16;
     if (in_dtype == PS_F32 && out_dtype == PS_F32)
-        return ps::f32::pick_tile((const float*)A, lda, (const float*)W, ldw, bias, (float*)out, ldo, M, N, K, act, accumulate, s);
+        return ps::f32::pick_tile((const float*)A, lda, (const float*)W, ldw, bias, (float*)out, ldo, M, N, K, act, accumulate, tile, s);
+    if (tile) return PS_ERR_UNSUPPORTED;
     if (in_dtype == PS_BF16 && out_dtype == PS_F32)
         return ps::launch_gemm_simt<bf, float>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
     if (in_dtype == PS_BF16 && out_dtype == PS_BF16)
@@ -590,7 +603,8 @@ PS_EXPORT int ps_gemm_simt(const void* A, int lda, const void* W, int ldw, const
     return PS_ERR_UNSUPPORTED;
 }
 
-// float32 products of at most 16 rows: K and both leading dimensions multiples of 4, A and W on 16-byte boundaries.
+// float32 products of at most 16 rows: K and both leading dimensions multiples of 4, A and W on 16-byte boundaries.  W is read
+// before the kernel in front has ended, whatever PS_WEIGHTS_READY says.
 PS_EXPORT int ps_gemm_f32_rows(const float* A, int lda, const float* W, int ldw, const float* bias, float* out, int ldo, int M,
                                int N, int K, int act, int accumulate, void* stream) {
     if (M <= 0 || N <= 0) return PS_OK;

@@ -18,6 +18,7 @@ from pagedserve_b200.kernels.build import load as _load_library
 
 PS_F32, PS_BF16 = 0, 1
 _DTYPE_CODE = {torch.float32: PS_F32, torch.bfloat16: PS_BF16}
+WEIGHTS_READY = 4             # in linear_simt's ``accumulate``: the weights were complete before the kernel in front began
 COLUMN_FACTOR = 2             # in a product's ``accumulate``: its vector multiplies the columns instead of being added
 _ACT_CODE = {None: 0, "none": 0, "gelu_tanh": 1, "gelu_erf": 2, "relu_squared": 3, "silu": 4, "tanh": 5}
 _STATUS = {1: "bad argument", 2: "unsupported size or dtype", 3: "kernel launch failed"}
@@ -76,7 +77,7 @@ _SIGNATURES = {
         "ps_embed_sinusoid": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P],
         "ps_rms_norm_pair": [_P, _I, _I, _P, _P, _F, _P, _P, _I, _P],
         "ps_layernorm": [_P, _P, _I, _I, _P, _P, _F, _I, _P, _I, _P],
-        "ps_gemm_simt": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "ps_gemm_simt": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "ps_gemm_f32_rows": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "ps_kv_append": [_P, _P, _I, _P, _P, _P, _I, _P, _P, _L, _I, _I, _I, _I, _I, _P],
         "ps_paged_attention_simt": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P,
@@ -353,8 +354,10 @@ class Ops:
         return out
 
     # ------------------------------------------------------------------ matrix product
-    def linear_simt(self, a, w, bias, out, act=None, accumulate=False):
-        """out = act(a @ w.T + bias) on CUDA cores (float32 accumulation, fixed K order)."""
+    def linear_simt(self, a, w, bias, out, act=None, accumulate=False, tile=0):
+        """out = act(a @ w.T + bias) on CUDA cores (float32 accumulation, fixed K order).  ``w`` may have been made by the kernel in
+        front, unless ``accumulate`` holds WEIGHTS_READY.  ``tile`` (float32): 0, or the shape of the tiles (csrc/gemm_simt.cu:
+        ps_gemm_simt)."""
         M, K = a.shape
         N = w.shape[0]
         if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
@@ -374,14 +377,15 @@ class Ops:
         _check(self.core.ps_gemm_simt(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(bias),
                                       _ptr(out), out.stride(0), M, N, K,
                                       dtype_code(a.dtype), dtype_code(out.dtype),
-                                      _ACT_CODE[act], int(accumulate), _stream()),
+                                      _ACT_CODE[act], int(accumulate), tile, _stream()),
                "gemm_simt")
         return out
 
     F32_FEW_ROWS = 16             # most rows of a float32 product that run on the kernel that streams the weights once
 
     def linear_f32_rows(self, a, w, bias, out, act=None, accumulate=False):
-        """The float32 product of at most F32_FEW_ROWS rows (csrc/gemm_simt.cu: gemm_f32_rows_kernel)."""
+        """The float32 product of at most F32_FEW_ROWS rows (csrc/gemm_simt.cu: gemm_f32_rows_kernel).  ``w`` must have been
+        complete before the kernel in front began: it is read before that one has ended."""
         M, K = a.shape
         N = w.shape[0]
         if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
@@ -664,7 +668,8 @@ class Ops:
         return out
 
     def linear(self, a, w, bias, out, act=None, accumulate=False, factor=None):
-        """The matrix product of the model: float32 runs on FFMA, bfloat16 on tensor cores.
+        """The matrix product of the model: float32 runs on FFMA, bfloat16 on tensor cores.  ``w`` holds weights, which no kernel
+        of a step writes: the kernels read it before the one in front has ended.
         ``a`` may be a DeferredNorm: it is folded into the product where a kernel can, else evaluated.
         ``factor`` (float32, one number per column, instead of a bias) multiplies the product before it is stored or
         added: the product kernels take it as their vector of one number per column."""
@@ -679,7 +684,7 @@ class Ops:
         if self.dtype == torch.float32:
             if self._f32_rows_ok(a, w, out):
                 return self.linear_f32_rows(a, w, bias, out, act, accumulate)
-            return self.linear_simt(a, w, bias, out, act, accumulate)
+            return self.linear_simt(a, w, bias, out, act, int(accumulate) | WEIGHTS_READY)
         from pagedserve_b200.kernels import tensorcore
 
         return tensorcore.linear(self, a, w, bias, out, act, accumulate)

@@ -197,3 +197,20 @@ def test_few_rows_of_a_vocabulary(M, N, K):
     ops.linear_f32_rows(a, w[:4000], None, part)
     ops.linear_f32_rows(a, w, None, whole)
     assert torch.equal(whole[:, :4000], part)
+
+
+@pytest.mark.parametrize("tile", [0, 1, 2, 3, 4, 5])
+def test_weights_made_by_the_kernel_in_front(tile):
+    """linear_simt reads its second operand only when the kernel in front has ended, which may have made it: a product whose result is
+    the weight of the next, on every kind of tile, several times in a row with other numbers."""
+    M, N, K = 700, 512, 512
+    ops, g = ops_for(), torch.Generator().manual_seed(tile)
+    made, outs = torch.empty(N, K, device=DEV), torch.empty(6, M, N, device=DEV)
+    a = torch.randn(M, K, generator=g).to(DEV)
+    left, right = torch.randn(6, N, 256, generator=g).to(DEV), (torch.randn(6, K, 256, generator=g) / 16).to(DEV)
+    for i in range(6):
+        ops.linear_simt(left[i], right[i], None, made)
+        ops.linear_simt(a, made, None, outs[i], tile=tile)
+    for i in range(6):
+        want = a.double() @ (left[i].double() @ right[i].double().T).T
+        assert float((outs[i].double() - want).abs().max()) < 1e-5 * float(want.abs().max()), i
