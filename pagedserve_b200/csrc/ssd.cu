@@ -577,13 +577,13 @@ ssd_prompt_kernel(const __nv_bfloat16* __restrict__ conv, const __nv_bfloat16* _
     constexpr int CH = L::CH, TROW = L::TROW, PROW = L::PROW;
     extern __shared__ __align__(16) __nv_bfloat16 ssd_tiles[];
     __shared__ float s_dt[CH], s_log[CH], s_from[CH], s_to[CH];
-    const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int order = blockIdx.x / in.heads, h = blockIdx.x - order * in.heads, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // The longest entries go first, all heads of one before the next: a CTA takes as long as its entry has chunks, and where
     // there are more CTAs than SMs a long one that starts last is worked on alone (entries of 744, 1,443 and 1,500 tokens in
     // this order, 64 heads of 64 x 128: the layer 472.8 -> 463.8 us).
     __shared__ int s_entry;
-    const int entries = gridDim.y;
-    int entry = blockIdx.y;
+    const int entries = gridDim.x / in.heads;
+    int entry = order;
     if (entries > 1 && entries <= SSD_THREADS) {
         if (tid < entries) {
             const int own = q_start[first_item + tid + 1] - q_start[first_item + tid];
@@ -592,7 +592,7 @@ ssd_prompt_kernel(const __nv_bfloat16* __restrict__ conv, const __nv_bfloat16* _
                 const int other = q_start[first_item + i + 1] - q_start[first_item + i];
                 place += other > own || (other == own && i < tid);
             }
-            if (place == (int)blockIdx.y) s_entry = tid;
+            if (place == order) s_entry = tid;
         }
         __syncthreads();
         entry = s_entry;
@@ -916,8 +916,9 @@ int launch_ssd_prompt(const __nv_bfloat16* conv, const __nv_bfloat16* raw, const
     static size_t raised[MAX_DEVICES] = {0};
     if (!ensure_dynamic_smem((const void*)kernel, L::BYTES, raised)) return PS_ERR_LAUNCH;
     const int tiles = (in.P + PT - 1) / PT;
-    if ((long long)tiles * depth > 65535 || n_items - first_item > 65535) return PS_ERR_UNSUPPORTED;
-    return launch_pdl(kernel, dim3(in.heads, n_items - first_item, tiles * depth), dim3(SSD_THREADS), L::BYTES, s, conv, raw, in,
+    const long long pairs = (long long)in.heads * (n_items - first_item);        // (all on x: a step may bring more entries than y counts)
+    if ((long long)tiles * depth > 65535 || pairs > 0x7fffffffll) return PS_ERR_UNSUPPORTED;
+    return launch_pdl(kernel, dim3((unsigned)pairs, 1, tiles * depth), dim3(SSD_THREADS), L::BYTES, s, conv, raw, in,
                       state, state_stride, q_start, item_slot, first_item, segments, run_state, run_decay, out, out_stride);
 }
 
