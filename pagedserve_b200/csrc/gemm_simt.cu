@@ -350,21 +350,27 @@ int run_tile(int tile, const float* A, int lda, const float* W, int ldw, const f
 // 768 (us; the shapes' order among one another holds at other K): large tiles need fewer reads per multiply-add, small ones
 // leave fewer SMs idle.  384 x 2,304 x 768: 54 us with 64 x 64 tiles, 41 with 32 x 64, 72 with 32 x 32; 128 x 768 x 768:
 // 36 / 24 / 15 / 15; 2,048 x 768 x 768: 73 / 81 / 108 / 130 (95 with 128 x 128).
+// (wide: whether the 128 x 128 tiles take the shape.)
+inline int choose_tile(int M, int N, bool wide) {
+    constexpr int rows[5] = {128, 64, 32, 32, 32}, columns[5] = {128, 64, 64, 32, 16};
+    constexpr float fixed[5] = {24.f, 15.f, 10.f, 3.f, 4.f}, each[5] = {64.f, 21.5f, 13.3f, 11.4f, 6.3f};
+    int tile = 0;
+    float least = 0.f;
+    for (int t = wide ? 0 : 1; t < 5; ++t) {
+        const long long ctas = (long long)((M + rows[t] - 1) / rows[t]) * ((N + columns[t] - 1) / columns[t]);
+        const float cost = fixed[t] + each[t] * (float)((ctas + 147) / 148);
+        if (least == 0.f || cost < least) { least = cost; tile = t + 1; }
+    }
+    return tile;
+}
+inline bool takes_wide(int M, int N, int K, bool aligned) { return aligned && M >= WIDE && N >= WIDE && K % WIDE_K == 0; }
+
 int pick_tile(const float* A, int lda, const float* W, int ldw, const float* bias, float* out, int ldo, int M, int N, int K,
               int act, int accumulate, int tile, cudaStream_t s) {
     const bool aligned = (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && lda % 4 == 0 && ldw % 4 == 0 && K % 4 == 0;
-    constexpr int rows[5] = {128, 64, 32, 32, 32}, columns[5] = {128, 64, 64, 32, 16};
-    constexpr float fixed[5] = {24.f, 15.f, 10.f, 3.f, 4.f}, each[5] = {64.f, 21.5f, 13.3f, 11.4f, 6.3f};
-    const bool wide = aligned && M >= WIDE && N >= WIDE && K % WIDE_K == 0;
+    const bool wide = takes_wide(M, N, K, aligned);
     if (tile < 0 || tile > 5 || (tile == 1 && !wide)) return PS_ERR_UNSUPPORTED;
-    if (tile == 0) {
-        float least = 0.f;
-        for (int t = wide ? 0 : 1; t < 5; ++t) {
-            const long long ctas = (long long)((M + rows[t] - 1) / rows[t]) * ((N + columns[t] - 1) / columns[t]);
-            const float cost = fixed[t] + each[t] * (float)((ctas + 147) / 148);
-            if (least == 0.f || cost < least) { least = cost; tile = t + 1; }
-        }
-    }
+    if (tile == 0) tile = choose_tile(M, N, wide);
     if (tile == 1)
         return launch_pdl(gemm_f32_wide_kernel, dim3((N + WIDE - 1) / WIDE, (M + WIDE - 1) / WIDE), dim3(WIDE_THREADS), 0, s, A, lda,
                           W, ldw, bias, out, ldo, M, N, K, act, accumulate);
@@ -601,6 +607,11 @@ PS_EXPORT int ps_gemm_simt(const void* A, int lda, const void* W, int ldw, const
     if (in_dtype == PS_BF16 && out_dtype == PS_BF16)
         return ps::launch_gemm_simt<bf, bf>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
     return PS_ERR_UNSUPPORTED;
+}
+
+// The tile that ps_gemm_simt chooses for a float32 product; aligned: K and leading dimensions multiples of 4, 16-byte addresses.
+PS_EXPORT int ps_gemm_f32_tile(int M, int N, int K, int aligned) {
+    return ps::f32::choose_tile(M, N, ps::f32::takes_wide(M, N, K, aligned && K % 4 == 0));
 }
 
 // float32 products of at most 16 rows: K and both leading dimensions multiples of 4, A and W on 16-byte boundaries.  W is read

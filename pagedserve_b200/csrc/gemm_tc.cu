@@ -1,10 +1,11 @@
 // Tensor-core GEMM for sm_100a: out[M,N] = epilogue(A[M,K] W[N,K]^T + bias), bfloat16 in, float32 accumulate.
 //
 //   TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast)  ->  shared memory ring of STAGES k-blocks
-//   tcgen05.mma.cta_group::1.kind::f16 (M=128, N=BN, K=16), issued by one thread, accumulating in TMEM
+//   tcgen05.mma.kind::f16 (K=16) of one CTA (cta_group::1, M=128, N=BN) or of a pair (cta_group::2, M=256, N=256; gemm_tc_kernel),
+//   issued by one thread, accumulating in TMEM
 //   tcgen05.ld 32x32b -> registers -> bias / GELU / residual-accumulate epilogue -> global memory
 //
-// The kernel is persistent: one CTA per SM walks the output tiles (n fastest, so neighbouring CTAs share
+// The kernel is persistent: one CTA per SM (or a pair on two) walks the output tiles (n fastest, so neighbouring CTAs share
 // the same rows of A in L2). TMEM holds two accumulators of BN columns; while the four epilogue warps
 // drain one, the MMA warp fills the other.
 //   warp 0: TMA producer (one lane)          warp 1: TMEM allocation + MMA issue (one lane)
@@ -898,31 +899,33 @@ PS_EXPORT int ps_gemm_tc_groups(const void* A, int lda, const void* W, int ldw, 
 
 // The packed q|k|v projection of a step with prompt portions: columns [0, q_width) go to `out` (bfloat16), the
 // key and value columns (kv_width each) go straight into the pages of each row's request. q_width must be a
-// multiple of 64 and head_dim of 8; `out` rows must start on 16-byte boundaries.
+// multiple of 64 and head_dim of 8; `out` rows must start on 16-byte boundaries.  bn as for ps_gemm_tc.
 PS_EXPORT int ps_gemm_tc_qkv(const void* A, int lda, const void* W, int ldw, const float* bias, void* out, int ldo,
                              int M, int N, int K, int* status, void* k_pool, void* v_pool, long long page_stride,
                              const int* token_item, const int* positions, const int* block_table, int bt_stride,
-                             int q_width, int kv_width, int head_dim, int page_size, void* stream) {
+                             int q_width, int kv_width, int head_dim, int page_size, int bn, void* stream) {
     if (!k_pool || !v_pool || !token_item || !positions || !block_table) return PS_ERR_BAD_ARGUMENT;
     if (q_width + 2 * kv_width != N || q_width % 64 != 0 || head_dim <= 0 || head_dim % 8 != 0 ||
         kv_width % head_dim != 0 || page_size <= 0)
         return PS_ERR_UNSUPPORTED;
     ps::KvScatter kv{(__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, page_stride, token_item, positions, block_table,
                      bt_stride, q_width, kv_width, head_dim, page_size};
-    return gemm_tc_entry(A, lda, W, ldw, bias, out, ldo, M, N, K, PS_BF16, PS_ACT_NONE, 0, status, 0, kv, stream);
+    return gemm_tc_entry(A, lda, W, ldw, bias, out, ldo, M, N, K, PS_BF16, PS_ACT_NONE, 0, status, bn, kv, stream);
 }
 
 // The first product of a gated feed-forward with its activation: out[m, n] (bfloat16, [M, F]) = form(A[m] . gate row n, A[m] . up row
 // n) with the row's weight (row_weight float32 [M], null: 1; a row of weight 0 gives zeros).  W [2 F, K]: F gate rows, then F up
-// rows; with tile_expert (as for ps_gemm_tc_experts) the experts' such matrices stacked by rows.
+// rows; with tile_expert (as for ps_gemm_tc_experts) the experts' such matrices stacked by rows.  bn: 0 = choose, 256 = one CTA a tile,
+// 512 = pairs of CTAs (not with tile_expert).
 PS_EXPORT int ps_gemm_tc_gated(const void* A, int lda, const void* W, int ldw, void* out, int ldo, int M, int F, int K, int kind,
                                float limit, float alpha, const float* row_weight, const int* tile_expert, int experts,
-                               int* status, void* stream) {
+                               int* status, int bn, void* stream) {
     if (M <= 0 || F <= 0) return PS_OK;
     if (!status || kind < 0 || kind > 2 || (kind == 1 && !(limit > 0.f)) || (tile_expert && experts <= 0)) return PS_ERR_BAD_ARGUMENT;
     if (K <= 0 || K % 8 || lda % 8 || ldw % 8 || ldo % 8 || F % 8 || lda < K || ldw < K || ldo < F) return PS_ERR_UNSUPPORTED;
     if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)out) & 15) return PS_ERR_UNSUPPORTED;
     using namespace ps::tc;
+    if ((bn != 0 && bn != 256 && bn != PAIR_256) || (bn == PAIR_256 && tile_expert)) return PS_ERR_UNSUPPORTED;
     using bf = __nv_bfloat16;
     CUtensorMap map_a, map_w, map_out;
     if (!make_map(&map_a, A, M, K, lda, BM) || !make_map(&map_w, W, 2 * F * (tile_expert ? experts : 1), K, ldw, 128) ||
@@ -937,7 +940,7 @@ PS_EXPORT int ps_gemm_tc_gated(const void* A, int lda, const void* W, int ldw, v
     const float one = 4.f + (float)((alone + sm_count() - 1) / sm_count()) * (blocks * .464f + .4f);
     const float two = 5.5f + (float)((pairs + sm_count() / 2 - 1) / (sm_count() / 2)) * (blocks * .425f + .4f);
     cudaStream_t s = (cudaStream_t)stream;
-    if (!tile_expert && two < one)
+    if (bn == PAIR_256 || (bn == 0 && !tile_expert && two < one))
         return launch_kernel<256, bf, true, true, true>(map_a, map_w, map_out, nullptr, out, ldo, M, F, K, PS_ACT_NONE, 0, status, none,
                                                         s, ex, no_groups, gated);
     return launch_kernel<256, bf, true, false, true>(map_a, map_w, map_out, nullptr, out, ldo, M, F, K, PS_ACT_NONE, 0, status, none, s,

@@ -78,6 +78,7 @@ _SIGNATURES = {
         "ps_rms_norm_pair": [_P, _I, _I, _P, _P, _F, _P, _P, _I, _P],
         "ps_layernorm": [_P, _P, _I, _I, _P, _P, _F, _I, _P, _I, _P],
         "ps_gemm_simt": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "ps_gemm_f32_tile": [_I, _I, _I, _I],
         "ps_gemm_f32_rows": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "ps_kv_append": [_P, _P, _I, _P, _P, _P, _I, _P, _P, _L, _I, _I, _I, _I, _I, _P],
         "ps_paged_attention_simt": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P,
@@ -153,8 +154,8 @@ _SIGNATURES = {
                             _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "ps_gemm_tc_groups": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
         "ps_gemm_tc_experts": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P],
-        "ps_gemm_tc_gated": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _F, _P, _P, _I, _P, _P],
-        "ps_gemm_tc_qkv": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+        "ps_gemm_tc_gated": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _F, _P, _P, _I, _P, _I, _P],
+        "ps_gemm_tc_qkv": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "ps_prefill_attention_tc": [_P, _I, _I, _P, _I, _P, _L, _L, _L, _L, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I,
                                     _I, _I, _F, _I, _P, _F, _P, _I, _I, _P],
     },
@@ -648,8 +649,8 @@ class Ops:
         self.linear(a, w, bias, out)
         return False
 
-    def linear_tc_qkv(self, a, w, bias, out, ctx, layer, q_width, kv_width, head_dim):
-        """tcgen05 q|k|v projection: query columns to ``out``, key and value columns into the pages."""
+    def linear_tc_qkv(self, a, w, bias, out, ctx, layer, q_width, kv_width, head_dim, bn=0):
+        """tcgen05 q|k|v projection: query columns to ``out``, key and value columns into the pages (``bn`` as in :meth:`linear_tc`)."""
         M, K = a.shape
         N = w.shape[0]
         if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
@@ -664,7 +665,7 @@ class Ops:
             _ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(bias), _ptr(out), out.stride(0), M, N, K,
             _ptr(self.status_flag(a.device)), _ptr(layer.k_pool), _ptr(layer.v_pool), layer.page_stride,
             _ptr(ctx.token_slot), _ptr(ctx.positions), _ptr(layer.block_table), layer.block_table.stride(0),
-            q_width, kv_width, head_dim, layer.page_size, _stream()), "gemm_tc_qkv")
+            q_width, kv_width, head_dim, layer.page_size, bn, _stream()), "gemm_tc_qkv")
         return out
 
     def linear(self, a, w, bias, out, act=None, accumulate=False, factor=None):
@@ -1861,11 +1862,11 @@ class Ops:
         experts of 1,024 x 1,024, rows of their runs: 768 (48) 12.6 / 13.3, 1,280 (80) 15.8 / 13.6."""
         return 3 * -(-rows // self.GATED_TILE) * -(-columns // self.GATED_TILE) > 148
 
-    def linear_gated(self, a, w, inner, form=None, row_weight=None, tile_expert=None, experts=1):
+    def linear_gated(self, a, w, inner, form=None, row_weight=None, tile_expert=None, experts=1, bn=0):
         """inner[m, n] = the gated activation ``form`` (:meth:`_gate_form`; of a clamped one the routed experts' limit where
         ``tile_expert`` is given, else the shared expert's) of a[m] . w[n] and a[m] . w[F + n], times the row's weight
         (float32 [M]; None: 1), in one tcgen05 product: ``w`` [2 F, K], or with ``tile_expert`` (as for
-        :meth:`linear_experts`) the experts' such matrices stacked by rows."""
+        :meth:`linear_experts`) the experts' such matrices stacked by rows.  ``bn``: 0 (choose), 256 or 512 (pairs of CTAs)."""
         M, K = a.shape
         F = inner.shape[1]
         if (w.shape != (2 * F * experts, K) or inner.shape[0] != M or not self.gated_ok(a, w, inner) or (tile_expert is None and experts != 1)
@@ -1886,7 +1887,7 @@ class Ops:
         self.launches += 1
         _check(self._tc.ps_gemm_tc_gated(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(inner), inner.stride(0), M, F, K, kind,
                                          limit if tile_expert is not None else shared_limit, alpha, _ptr(row_weight),
-                                         _ptr(tile_expert), experts, _ptr(self.status_flag(a.device)), _stream()), "gemm_tc_gated")
+                                         _ptr(tile_expert), experts, _ptr(self.status_flag(a.device)), bn, _stream()), "gemm_tc_gated")
         return inner
 
     # ------------------------------------------------------------------ sampling

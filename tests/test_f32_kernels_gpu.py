@@ -28,10 +28,17 @@ def product(a, w, bias, act, factor, base):
     return y if base is None else y + base.double()
 
 
-# float32 sums of K products of numbers of order one over sqrt(K): each addition rounds by at most 2^-24 of a partial sum that
-# is of the size of the result; K + 40 of them in a row is the longest chain
-def sum_bound(K):
-    return (K + 40) * 2.0 ** -24
+# The error of a float32 sum of K products of normal numbers, relative to the largest of the results: every addition rounds by at
+# most 2^-24 of a partial sum of at most the size of the result, signs at random, so that sqrt(K) of them add up (a result is
+# about 0.4 sqrt(K) 2^-24 off at one standard deviation); and a few roundings of what comes behind the sum.  Operands rounded to 10
+# bits of mantissa are off by 2^-11 of a product, which is far beyond it (tests/test_f32_bound_cpu.py).
+def bound(K):
+    return 3 * (K ** 0.5 + 4) * 2.0 ** -24
+
+
+def size_of(want):
+    """The largest result, or one (a sum's standard deviation) where there are few and they happen to be small."""
+    return max(1.0, float(want.abs().max()))
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16])
@@ -46,7 +53,7 @@ def test_few_rows(M, N, K):
         ops.linear_f32_rows(a_d, w_d, bias_d, out, act=act, accumulate={"store": 0, "add": 1, "factor": 3}[how])
         want = product(a, w, None if how == "factor" else bias, act, bias if how == "factor" else None,
                        None if how == "store" else base)
-        assert float((out.cpu().double() - want).abs().max()) < sum_bound(K) * 8 * float(want.abs().max()), (act, how)
+        assert float((out.cpu().double() - want).abs().max()) < bound(K) * size_of(want), (act, how)
     # a row alone and a row among others, rows that lie apart
     wide = torch.randn(M, K + 8, generator=g).to(DEV)
     wide[:, :K] = a_d
@@ -60,7 +67,7 @@ def test_few_rows(M, N, K):
                                    (300, 2100, 40), (1500, 1030, 20), (128, 768, 3072),
                                    (128, 128, 16), (1030, 2051, 48), (2049, 1155, 160)])
 def test_tiles(M, N, K):
-    """Every tile shape of the many-rows kernel, tails in M, N and K, rows on and off 16-byte boundaries."""
+    """The tiles that the rule takes (test_every_tile has each of them), tails in M, N and K, rows on and off 16-byte boundaries."""
     ops, g = ops_for(), torch.Generator().manual_seed(M + N + K)
     a, w, bias, base = (torch.randn(shape, generator=g) for shape in ((M, K), (N, K), (N,), (M, N)))
     w /= K ** 0.5
@@ -71,7 +78,7 @@ def test_tiles(M, N, K):
         out = base.clone().to(DEV)
         ops.linear_simt(rows, w.to(DEV), bias.to(DEV), out, accumulate=True)
         want = product(a, w, bias, None, None, base)
-        assert float((out.cpu().double() - want).abs().max()) < sum_bound(K) * 8 * float(want.abs().max())
+        assert float((out.cpu().double() - want).abs().max()) < bound(K) * size_of(want)
         outs.append(out)
     assert torch.equal(outs[0], outs[1])                         # however the rows lie: the same sums in the same order
 
@@ -191,7 +198,7 @@ def test_few_rows_of_a_vocabulary(M, N, K):
         out = base.clone()
         ops.linear_f32_rows(a, w, bias, out, accumulate=accumulate)
         want = product(a, w, None if accumulate == 3 else bias, None, bias if accumulate == 3 else None, base if accumulate else None)
-        assert float((out.double() - want).abs().max()) < sum_bound(K) * 8 * float(want.abs().max()), accumulate
+        assert float((out.double() - want).abs().max()) < bound(K) * size_of(want), accumulate
     part = torch.empty(M, 4000, device=DEV)
     whole = torch.empty(M, N, device=DEV)
     ops.linear_f32_rows(a, w[:4000], None, part)
@@ -214,3 +221,78 @@ def test_weights_made_by_the_kernel_in_front(tile):
     for i in range(6):
         want = a.double() @ (left[i].double() @ right[i].double().T).T
         assert float((outs[i].double() - want).abs().max()) < 1e-5 * float(want.abs().max()), i
+
+
+@pytest.mark.parametrize("tile,M,N,K,aligned", [(1, 2048, 2304, 768, 1), (1, 1900, 2305, 48, 1), (2, 1030, 2051, 48, 1), (2, 2048, 2304, 768, 0),
+                                                (2, 2048, 2304, 772, 1), (3, 384, 2304, 768, 1), (4, 128, 768, 768, 1), (5, 33, 31, 36, 1)])
+def test_the_rule_takes_every_tile(tile, M, N, K, aligned):
+    assert ops_for().core.ps_gemm_f32_tile(M, N, K, aligned) == tile
+
+
+@pytest.mark.parametrize("tile", [1, 3, 4, 5])
+@pytest.mark.parametrize("M", [128, 129, 255, 257])
+@pytest.mark.parametrize("N,K", [(128, 16), (129, 48), (255, 784), (257, 48), (385, 16)])
+def test_every_tile(tile, M, N, K):
+    """Each shape of tiles has the bits of the 64 x 64 ones and the sums of 64 bits, with every epilogue: the last tiles of 128 x 128 are
+    moved back inside the matrix, store nothing twice and, with an odd first column, halves of pairs; what lies beside the result
+    stays."""
+    ops, g = ops_for(), torch.Generator().manual_seed(M + N + K)
+    a, w, vector, base = (torch.randn(shape, generator=g) for shape in ((M, K), (N, K), (N,), (M, N)))
+    w /= K ** 0.5
+    a_d, w_d, vector_d = a.to(DEV), w.to(DEV), vector.to(DEV)
+    for act, accumulate in ((None, 0), ("gelu_tanh", 0), (None, 1), (None, 2), (None, 3)):
+        outs = []
+        for which in (tile, 2):
+            room = torch.full((M + 1, N + 3), 7.0, device=DEV)
+            room[:M, :N] = base.to(DEV)
+            ops.linear_simt(a_d, w_d, vector_d, room[:M, :N], act=act, accumulate=accumulate, tile=which)
+            assert bool((room[M:] == 7.0).all()) and bool((room[:, N:] == 7.0).all())
+            outs.append(room[:M, :N])
+        assert torch.equal(outs[0], outs[1]), (act, accumulate)
+        want = product(a, w, None if accumulate & 2 else vector, act, vector if accumulate & 2 else None, base if accumulate & 1 else None)
+        assert float((outs[0].cpu().double() - want).abs().max()) < bound(K) * size_of(want), (act, accumulate)
+
+
+@pytest.mark.parametrize("N,K", [(768, 768), (300, 3072), (50, 1028)])
+def test_sums_by_rows(N, K):
+    """A row's sums are the same bits in every product of at most 16 rows, and in every product of more; between the two they differ as
+    float32 sums in two orders do."""
+    ops, g = ops_for(), torch.Generator().manual_seed(N + K)
+    a, w = torch.randn(300, K, generator=g).to(DEV), (torch.randn(N, K, generator=g) / K ** 0.5).to(DEV)
+    results = {}
+    for M in (1, 3, 16, 17, 64, 300):
+        results[M] = torch.empty(M, N, device=DEV)
+        ops.linear(a[:M], w, None, results[M])
+    for few, more in ((1, 16), (3, 16), (17, 300), (64, 300)):
+        assert torch.equal(results[few], results[more][:few]), (few, more)
+    assert float((results[16] - results[300][:16]).abs().max()) < bound(K) * size_of(results[16])
+
+
+@pytest.mark.parametrize("head_dim", [64, 100])
+@pytest.mark.parametrize("window", [0, 70])
+def test_attention_of_a_prompt_in_portions(head_dim, window):
+    """A prompt of 200 tokens whole and in portions: 16 tokens and more run on the prompt kernel, with the same bits as the whole; fewer, and
+    single ones, on the token kernel, whose bits too do not depend on the cut.  Between the two: float32 sums in two orders."""
+    heads, kv_heads, total = 4, 2, 200
+    step, ops = Step([(total, total)], heads, kv_heads, head_dim, page=16, seed=head_dim), ops_for()
+    q, row = step.q[0].reshape(total, -1).to(DEV), int(step.ctx.item_slot[0])
+    as_ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+
+    def run(portion):
+        out = torch.empty(total, heads * head_dim, device=DEV)
+        for begin in range(0, total, portion):
+            end = min(begin + portion, total)
+            short = portion < 16
+            ctx = SimpleNamespace(num_items=1, num_short_items=int(short), num_short_tokens=end - begin if short else 0,
+                                  num_long_blocks=-(-(end - begin) // 64), q_start=as_ints([0, end - begin]), kv_len=as_ints([end]),
+                                  item_slot=as_ints([row]), token_slot=as_ints([row] * (end - begin)), positions=as_ints(range(begin, end)))
+            ops.attention_f32(q[begin:end], out[begin:end], ctx, step.layer, heads, kv_heads, head_dim, window, head_dim ** -0.5)
+        return out
+
+    whole, single = run(total), run(1)
+    for portion in (16, 17, 63, 64, 130):
+        assert torch.equal(run(portion), whole), portion
+    for portion in (5, 15):
+        assert torch.equal(run(portion), single), portion
+    # weights that add up to one times values of a few, each from sums of up to 200 float32 terms
+    assert float((whole - single).abs().max()) < 2e-6

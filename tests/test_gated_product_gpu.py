@@ -45,6 +45,34 @@ def test_gated(form, M, F, K, weighted):
     assert bool(torch.isnan(inner[:, F:]).all()) and int(ops.status_flag(DEV).item()) == 0
 
 
+@pytest.mark.parametrize("form", ["silu", CLAMPED])
+@pytest.mark.parametrize("M", [65, 129, 257, 385, 512])
+@pytest.mark.parametrize("F,K", [(8, 64), (136, 200), (264, 1032)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_pairs_of_ctas(form, M, F, K, weighted):
+    """One CTA of the pair has the gates, the other the ups; the second one's rows may all lie past the last, its columns end inside a
+    tile.  The bits of one CTA per tile, and the sums of 64 bits."""
+    from pagedserve_b200.kernels.ops import Ops
+
+    ops, g = Ops(torch.bfloat16), torch.Generator().manual_seed(M + F + K)
+    a = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(2 * F, K, generator=g) * 2 / math.sqrt(K)).to(torch.bfloat16).to(DEV)
+    weight = torch.rand(M, generator=g).to(DEV) if weighted else None
+    if weighted:
+        weight[::7] = 0.0
+        a[::7] = float("inf")
+    room = torch.full((2, M + 1, F + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    for inner, bn in zip(room, (256, 512)):
+        ops.linear_gated(a, w, inner[:M, :F], form=form, row_weight=weight, bn=bn)
+    assert torch.equal(room[0], room[1]) and bool((room[:, M:] == 7.0).all()) and bool((room[:, :, F:] == 7.0).all())
+    y = a.double() @ w.double().T
+    want = formed(y[:, :F], y[:, F:], 1.0 if weight is None else weight[:, None].double(), form, 1.0)
+    if weighted:
+        want[::7] = 0.0
+    assert float((room[1, :M, :F].double() - want).abs().max()) < 6e-3 * float(want.abs().max())
+    assert int(ops.status_flag(DEV).item()) == 0
+
+
 @pytest.mark.parametrize("F,K", [(72, 64), (256, 136)])
 def test_experts(F, K):
     from pagedserve_b200.kernels.ops import Ops
