@@ -346,10 +346,13 @@ int run_tile(int tile, const float* A, int lda, const float* W, int ldw, const f
     return launch_tile<32, 16, 2, 2, 8, VEC>(A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate, s);
 }
 
-// The tile shape by the tiles that the busiest SM gets: a fixed cost and a cost per tile of each shape, measured on B200 at K =
-// 768 (us; the shapes' order among one another holds at other K): large tiles need fewer reads per multiply-add, small ones
-// leave fewer SMs idle.  384 x 2,304 x 768: 54 us with 64 x 64 tiles, 41 with 32 x 64, 72 with 32 x 32; 128 x 768 x 768:
-// 36 / 24 / 15 / 15; 2,048 x 768 x 768: 73 / 81 / 108 / 130 (95 with 128 x 128).
+// The tile shape by the tiles that the busiest SM gets: a fixed cost and a cost per tile of each shape, fitted on B200 at K = 768 (us):
+// large tiles need fewer reads per multiply-add, small ones leave fewer SMs idle.  The best shape hardly depends on K, which the rule
+// leaves out: over 17 to 2,048 rows, 768 to 6,400 columns and K of 768 to 6,400 it is 2.1 % behind the best shape on average, at most
+// 14 % but for 200 x 1,600 x 6,400 (22 %).  Us with 128 x 128 / 64 x 64 / 32 x 64 / 32 x 32 / 32 x 16 tiles: 384 x 2,304 x 768
+// 97 / 54 / 41 / 56 / 68, 128 x 768 x 768 92 / 36 / 24 / 14 / 15, 2,048 x 768 x 768 95 / 74 / 80 / 98 / 118, 128 x 768 x 3,072
+// 377 / 118 / 82 / 50 / 55, 2,048 x 768 x 3,072 357 / 258 / 296 / 377 / 457, 651 x 1,024 x 4,096 476 / 257 / 197 / 241 / 294, 2,048 x 1,024 x
+// 4,096 473 / 476 / 538 / 636 / 790.
 // (wide: whether the 128 x 128 tiles take the shape.)
 inline int choose_tile(int M, int N, bool wide) {
     constexpr int rows[5] = {128, 64, 32, 32, 32}, columns[5] = {128, 64, 64, 32, 16};
