@@ -3,8 +3,12 @@
 //
 // prompt_attention_f32_kernel: prompt portions, 64 queries of one head per CTA, key tiles of 64 aligned to absolute positions.
 // token_attention_f32_kernel:  single tokens (decode steps, short portions), one CTA per (token, head).
-// Scores, softmax and results are float32 throughout (expf, tanhf); the order of every sum depends only on a query's position
-// (reference: src/model/paged_attention.py:262-295), so it makes no difference how a prompt was cut into portions.
+// Scores, softmax and results are float32 throughout (expf, tanhf).  Within each kernel the order of every sum depends only on a
+// query's position (reference: src/model/paged_attention.py:262-295): its bits are the same whatever else is in the step and, of
+// portions that all run on one kernel, wherever a prompt was cut.  The two add in different orders (the prompt kernel key by key with a
+// running maximum, the token kernel in states per lane group that are merged), so a query of a short portion differs from the same query of
+// a long one by the rounding of float32 sums.  One order for both (states per tile of 64 keys, joined in order) was measured: 12 heads of 64,
+// one token, 100 keys 4.2 -> 7.2 us, 1,000 keys 18.2 -> 23.7.
 #include "common.cuh"
 
 namespace ps {

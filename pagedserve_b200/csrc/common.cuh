@@ -76,7 +76,7 @@ __device__ __forceinline__ float apply_act(float x, int act) {
 
 // The inner activation of a gated feed-forward (csrc/moe.cu says what the kinds are).
 struct GateForm {
-    int kind;                 // 0: silu(g) u w; 2: gelu_tanh(g) u w; 1: clamped, weight on the input 
+    int kind;                 // 0: silu(g) u w; 2: gelu_tanh(g) u w; 1: clamped, weight on the input
     float limit;              // kind 1: the routed experts' limit
     float shared_limit;       // kind 1: the shared expert's
     float alpha;              // kind 1: the sigmoid's slope
