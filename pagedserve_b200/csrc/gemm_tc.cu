@@ -938,7 +938,7 @@ PS_EXPORT int ps_gemm_tc_gated(const void* A, int lda, const void* W, int ldw, v
     // Pairs of CTAs where they are modelled to be faster, as in pick() but with what a pair's tile costs with this epilogue: it takes
     // about 5 us, which a main loop of 16 k-blocks hides behind one CTA's MMAs and not behind a pair's, whose accumulator waits for both
     // CTAs.  Us, one CTA / pairs: 8,192 x 2,048 x 1,024 56.9 / 64.2, 3,000 x 4,096 x 1,024 44.8 / 51.8, 2,048 x 4,096 x 2,048 58.6 / 53.9,
-    // 8,192 x 6,400 x 1,600 277 / 255, 2,048 x 1,600 x 6,400 82.6 / 71.3.  Over 512 to 8,192 rows, K of 512 to 6,400, on two boxes: 0.1 and 0.3 %
+    // 8,192 x 6,400 x 1,600 277 / 255, 2,048 x 1,600 x 6,400 82.6 / 71.3.  Over 512 to 8,192 rows, K of 512 to 6,400, in two runs: 0.1 and 0.3 %
     // behind the better one on average, 5 and 9 at most (with pick()'s numbers 1.7 and 18).
     const int across = (F + 127) / 128, blocks = (K + BK - 1) / BK, alone = (M + 127) / 128 * across, pairs = (M + 255) / 256 * across;
     const float one = 4.f + (float)((alone + sm_count() - 1) / sm_count()) * (blocks * .464f + .4f);
