@@ -149,6 +149,8 @@ _SIGNATURES = {
                                  _F, _P, _I, _I, _P],
     },
     "tc": {
+        "ps_gemm_f32_tc": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+        "ps_gemm_f32_tc_parts": [_I],
         "ps_gemm_tc": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P],
         "ps_gemm_rows_tc": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I,
                             _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
@@ -409,6 +411,38 @@ class Ops:
                 and a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1 and a.stride(0) % 4 == 0
                 and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
+    def linear_f32_tc(self, a, w, bias, out, act=None, accumulate=False, splits=0, status=None):
+        """The float32 product on the tensor cores, operands as exact sums of bfloat16 numbers (csrc/gemm_f32_tc.cu).  ``w`` as for
+        :meth:`linear_simt`; ``splits``: 0, or how many CTAs share K (1 or the parts of K; the results are the same)."""
+        M, K = a.shape
+        N = w.shape[0]
+        if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
+            raise KernelError("linear_f32_tc: shapes do not match")
+        for name, tensor in (("a", a), ("w", w), ("out", out)):
+            _require(tensor, name, torch.float32)
+            if tensor.stride(1) != 1:
+                raise KernelError("linear_f32_tc: innermost stride must be 1")
+        if bias is not None:
+            _require(bias, "bias", torch.float32)
+            if bias.numel() != N:
+                raise KernelError("linear_f32_tc: bias length")
+        self._tc_library()
+        if status is None:
+            status = self.status_flag(a.device)
+        self.launches += 1
+        _check(self._tc.ps_gemm_f32_tc(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(bias), _ptr(out), out.stride(0), M, N, K,
+                                       _ACT_CODE[act], int(accumulate), splits, _ptr(status), _stream()), "gemm_f32_tc")
+        return out
+
+    @staticmethod
+    def _f32_tc_ok(a, w, out):
+        """Whether a float32 product of more than F32_FEW_ROWS rows runs on the tensor cores.  By the shape of ``w`` and alignment, not by
+        the rows: a row's bits are then those of the row alone in any larger step.  From 17 rows on it is the faster one at K of 768
+        (17 x 768 x 768: 9.3 us, multiply-adds 10.4); the multiply-adds' time falls with K, here 7 us stay."""
+        return (a.shape[1] >= 640 and w.shape[0] >= 64 and a.shape[1] % 4 == 0 and a.dtype == w.dtype == out.dtype == torch.float32
+                and a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1 and a.stride(0) % 4 == 0
+                and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
     def linear_skinny(self, a, w, bias, out, act=None, accumulate=False, kv=None):
         """Weight-streaming product for at most 64 rows of ``a`` (bfloat16 operands).  ``kv`` =
         (ctx, layer, q_width, kv_width, head_dim) sends the key and value columns of a packed q|k|v
@@ -480,8 +514,7 @@ class Ops:
         launch of the tcgen05 kernel over (row tile, group) pairs (csrc/gemm_tc.cu: ColumnGroups)."""
         groups, M, K = a.shape
         cols = out.shape[2]
-        if self._tc is None:
-            self._tc = _declare(_load_library("tc"), "tc")
+        self._tc_library()
         if status is None:
             status = self.status_flag(a.device)
         self.launches += 1
@@ -503,8 +536,7 @@ class Ops:
             _require(bias, "bias", torch.float32)
         if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
             raise KernelError("linear_tc: innermost stride must be 1")
-        if self._tc is None:
-            self._tc = _declare(_load_library("tc"), "tc")
+        self._tc_library()
         if status is None:
             status = self.status_flag(a.device)
         self.launches += 1
@@ -529,8 +561,7 @@ class Ops:
             _require(bias, "bias", torch.float32)
         if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
             raise KernelError("linear_rows_tc: innermost stride must be 1")
-        if self._tc is None:
-            self._tc = _declare(_load_library("tc"), "tc")
+        self._tc_library()
         if status is None:
             status = self.status_flag(a.device)
         self.launches += 1
@@ -539,6 +570,11 @@ class Ops:
                                         int(accumulate), _ptr(status), splits,
                                         *self._kv_arguments(kv, N), _stream()), "gemm_rows_tc")
         return out
+
+    def _tc_library(self):
+        if self._tc is None:
+            self._tc = _declare(_load_library("tc"), "tc")
+        return self._tc
 
     @staticmethod
     def tc_ok(a, w):
@@ -658,8 +694,7 @@ class Ops:
         _require(a, "a", torch.bfloat16)
         _require(w, "w", torch.bfloat16)
         _require(out, "out", torch.bfloat16)
-        if self._tc is None:
-            self._tc = _declare(_load_library("tc"), "tc")
+        self._tc_library()
         self.launches += 1
         _check(self._tc.ps_gemm_tc_qkv(
             _ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(bias), _ptr(out), out.stride(0), M, N, K,
@@ -669,7 +704,7 @@ class Ops:
         return out
 
     def linear(self, a, w, bias, out, act=None, accumulate=False, factor=None):
-        """The matrix product of the model: float32 runs on FFMA, bfloat16 on tensor cores.  ``w`` holds weights, which no kernel
+        """The matrix product of the model, on tensor cores but for few rows and small matrices of float32.  ``w`` holds weights, which no kernel
         of a step writes: the kernels read it before the one in front has ended.
         ``a`` may be a DeferredNorm: it is folded into the product where a kernel can, else evaluated.
         ``factor`` (float32, one number per column, instead of a bias) multiplies the product before it is stored or
@@ -685,6 +720,8 @@ class Ops:
         if self.dtype == torch.float32:
             if self._f32_rows_ok(a, w, out):
                 return self.linear_f32_rows(a, w, bias, out, act, accumulate)
+            if self._f32_tc_ok(a, w, out):
+                return self.linear_f32_tc(a, w, bias, out, act, int(accumulate) | WEIGHTS_READY)
             return self.linear_simt(a, w, bias, out, act, int(accumulate) | WEIGHTS_READY)
         from pagedserve_b200.kernels import tensorcore
 
@@ -967,8 +1004,7 @@ class Ops:
         layer's index inside it; ``max_blocks`` >= the number of 128-query blocks of the items.
         ``row_threads``: 1 or 2 threads per query row (0: the kernel's launcher decides)."""
         _require(q, "q", torch.bfloat16)
-        if self._tc is None:
-            self._tc = _declare(_load_library("tc"), "tc")
+        self._tc_library()
         if status is None:
             status = self.status_flag(q.device)
         pages, layers, planes, kv_heads, ps, hd = pool.shape
@@ -1834,8 +1870,7 @@ class Ops:
         _require(tile_expert, "tile_expert", torch.int32)
         if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
             raise KernelError("linear_experts: innermost stride must be 1")
-        if self._tc is None:
-            self._tc = _declare(_load_library("tc"), "tc")
+        self._tc_library()
         if status is None:
             status = self.status_flag(a.device)
         self.launches += 1
@@ -1882,8 +1917,7 @@ class Ops:
         kind, limit, shared_limit, alpha = self._gate_form(form)
         if kind == 3:
             raise KernelError("linear_gated: relu_squared has no gate")
-        if self._tc is None:
-            self._tc = _declare(_load_library("tc"), "tc")
+        self._tc_library()
         self.launches += 1
         _check(self._tc.ps_gemm_tc_gated(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(inner), inner.stride(0), M, F, K, kind,
                                          limit if tile_expert is not None else shared_limit, alpha, _ptr(row_weight),

@@ -1,0 +1,126 @@
+"""Float32 products on the tensor cores (csrc/gemm_f32_tc.cu) against 64 bits and against the float32 multiply-adds they replace."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def ops_for():
+    from pagedserve_b200.kernels.ops import Ops
+
+    return Ops(torch.float32)
+
+
+# A float32 sum of K products of normal numbers, relative to the largest of the results: sqrt(K) roundings of at most 2^-24 of the result add
+# up (tests/test_f32_kernels_gpu.py derives the same bound; tests/test_f32_bound_cpu.py shows that operands of 10 bits are beyond it).
+def bound(K):
+    return 3 * (K ** 0.5 + 4) * 2.0 ** -24
+
+
+def size_of(want):
+    return max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("M", [1, 17, 127, 128, 129, 300])
+@pytest.mark.parametrize("N,K", [(64, 256), (127, 260), (129, 508), (385, 516), (257, 2044), (768, 3080)])
+def test_every_epilogue(M, N, K):
+    """Edges of the 128 x 128 tiles, blocks of 64 k's and parts that end inside one, rows on their own pitch, K in clusters or in one CTA."""
+    ops, g = ops_for(), torch.Generator().manual_seed(M + N + K)
+    a, w, vector, base = (torch.randn(shape, generator=g) for shape in ((M, K), (N, K), (N,), (M, N)))
+    w /= K ** 0.5
+    wide = torch.full((M, K + 4), float("nan"))
+    wide[:, :K] = a
+    a_d, w_d, vector_d = wide.to(DEV)[:, :K], w.to(DEV), vector.to(DEV)
+    parts = ops._tc_library().ps_gemm_f32_tc_parts(K)
+    exact = a.double() @ w.double().T
+    for act, accumulate in ((None, 0), ("gelu_tanh", 4), (None, 1), (None, 2), (None, 3 + 4)):
+        outs = []
+        for splits in (1, parts // 2, parts, 0):
+            room = torch.full((M + 1, N + 3), 7.0, device=DEV)
+            room[:M, :N] = base.to(DEV)
+            ops.linear_f32_tc(a_d, w_d, vector_d, room[:M, :N], act=act, accumulate=accumulate, splits=splits)
+            assert bool((room[M:] == 7.0).all()) and bool((room[:, N:] == 7.0).all())
+            outs.append(room[:M, :N].clone())
+        assert all(torch.equal(outs[0], other) for other in outs[1:]), (act, accumulate)
+        want = exact * vector.double() if accumulate & 2 else exact + vector.double()
+        if act == "gelu_tanh":
+            want = torch.nn.functional.gelu(want, approximate="tanh")
+        if accumulate & 1:
+            want = want + base.double()
+        assert float((outs[0].cpu().double() - want).abs().max()) < bound(K) * size_of(want), (act, accumulate)
+    assert int(ops.status.item()) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(384, 2304, 768), (2048, 768, 768), (651, 1024, 4096), (384, 768, 3072), (200, 1600, 6400), (64, 768, 256)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "wide"])
+def test_error_is_no_larger_than_that_of_multiply_adds(M, N, K, kind):
+    """Against 64 bits, beside the float32 kernel that adds one product after the other: signs at random, no signs (every cut of a sum
+    in the same direction), magnitudes over many powers of two."""
+    ops, g = ops_for(), torch.Generator(device=DEV).manual_seed(M + N + K)
+    a, w = (torch.randn(shape, generator=g, device=DEV) for shape in ((M, K), (N, K)))
+    if kind == "positive":
+        a, w = a.abs(), w.abs()
+    elif kind == "wide":
+        a = a * torch.exp2(torch.randint(-12, 12, (M, K), generator=g, device=DEV).float())
+    want = a.double() @ w.double().T
+    errors = []
+    for run in (ops.linear_f32_tc, ops.linear_simt):
+        out = torch.empty(M, N, device=DEV)
+        run(a, w, None, out)
+        errors.append(float((out.double() - want).norm() / want.norm()))
+    assert errors[0] <= errors[1], errors
+
+
+def test_infinities_and_nans():
+    ops, g = ops_for(), torch.Generator().manual_seed(1)
+    a, w = torch.randn(140, 512, generator=g), torch.randn(130, 512, generator=g)
+    a[3, 7], a[4, 9], a[5, 500], a[6, 0], a[6, 511] = float("inf"), float("-inf"), float("nan"), float("inf"), float("inf")
+    w[11, 7], w[12, 9], w[13, 100] = 0.0, -0.0, float("inf")
+    w[14] = 1.0                                                  # numbers without second pieces
+    a[20], w[20] = 3.4e38, 1e-3                                  # near the largest float: no piece is rounded up to an infinity
+    a[21] = 3.0e38                                               # sums beyond it
+    a[22] = torch.randn(512, generator=g) * 2.0 ** -100
+    want = (a.double() @ w.double().T).float()
+    for splits in (0, 1, 2):
+        out = torch.empty(140, 130, device=DEV)
+        ops.linear_f32_tc(a.to(DEV), w.to(DEV), None, out, splits=splits)
+        out = out.cpu()
+        plain = torch.empty(140, 130, device=DEV)
+        ops.linear_simt(a.to(DEV), w.to(DEV), None, plain)
+        plain = plain.cpu()
+        finite = torch.isfinite(plain)
+        assert torch.equal(torch.isnan(out), torch.isnan(plain)) and torch.equal(torch.isinf(out), torch.isinf(plain))
+        assert torch.equal(out[torch.isinf(plain)], plain[torch.isinf(plain)])
+        rows = [r for r in range(140) if r not in (20, 21)]
+        assert torch.allclose(out[rows][finite[rows]], want[rows][finite[rows]], rtol=1e-5, atol=1e-4)
+        assert torch.allclose(out[20][finite[20]], plain[20][finite[20]], rtol=1e-3)
+
+
+def test_products_in_a_row():
+    """Products launched one behind the other, each reading what the one before wrote: the weights among it where they may be."""
+    ops, g = ops_for(), torch.Generator().manual_seed(2)
+    made, outs = torch.empty(512, 512, device=DEV), torch.empty(6, 300, 512, device=DEV)
+    a = torch.randn(300, 512, generator=g).to(DEV)
+    left, right = torch.randn(6, 512, 256, generator=g).to(DEV), (torch.randn(6, 512, 256, generator=g) / 16).to(DEV)
+    for i in range(6):
+        ops.linear_f32_tc(left[i], right[i], None, made)
+        ops.linear_f32_tc(a, made, None, outs[i], splits=(1, 2, 4)[i % 3])
+    for i in range(6):
+        want = a.double() @ (left[i].double() @ right[i].double().T).T
+        assert float((outs[i].double() - want).abs().max()) < 1e-5 * float(want.abs().max()), i
+
+
+def test_refused():
+    from pagedserve_b200.kernels.ops import KernelError
+
+    ops = ops_for()
+    a, w, out = torch.zeros(32, 512, device=DEV), torch.zeros(64, 512, device=DEV), torch.zeros(32, 64, device=DEV)
+    with pytest.raises(KernelError):
+        ops.linear_f32_tc(a, w, None, out, splits=3)
+    with pytest.raises(KernelError):
+        ops.linear_f32_tc(a[:, 1:], w[:, 1:], None, out)
+    with pytest.raises(KernelError):
+        ops.linear_f32_tc(a[:, :128], w[:, :128], None, out)
