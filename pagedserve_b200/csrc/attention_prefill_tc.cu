@@ -15,7 +15,7 @@
 //               row's running maximum the row's thread first rescales its O row in TMEM (skipped by a whole
 //               warp when none of its 32 rows changed, which is the common case after the first tiles)
 // TMA brings the Q tile from the step's q|k|v buffer and, page by page, the K and V tiles from the pool
-// (one box of page_size x 64 per page; no multicast); two K/V stages.
+// (one box of page_size x 64 per page; no multicast); two K/V stages (one where two CTAs of head size 128 share an SM).
 //   warp 0: TMA producer      warp 1: TMEM allocation + MMA issue      warps 2..9: softmax rows / output
 // mma.sync on this GPU gives about 1/15 of the tcgen05 rate (measured: 112 TFLOP/s at best for the mma.sync
 // kernel in csrc/attention_prefill.cu), which is why prompt attention is here. Head sizes other than 64 and
@@ -28,7 +28,7 @@
 namespace ps {
 namespace pftc {
 
-constexpr int BQ = 128, BKEY = 128, KV_STAGES = 2;
+constexpr int BQ = 128, BKEY = 128;
 constexpr uint64_t WAIT_LIMIT_NS = 200ull * 1000 * 1000;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -167,26 +167,38 @@ __device__ __forceinline__ bool slot_get(const unsigned long long* slot, uint32_
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// SPLIT: threads per query row (1: two CTAs per SM at head size 64, best when there are many query blocks;
-// 2: one CTA per SM, each row's chain half as long, best when few blocks decide the duration).
-template <int HD, int SPLIT>
+// SPLIT: threads per query row; RESIDENT: CTAs per SM.  Two CTAs are best when there are many query blocks, one with two threads per
+// row, whose chain is half as long, when few blocks decide the duration.
+// Two CTAs at head size 128 (SHARED) have 256 columns of tensor memory and 102 KB each: P takes the place of S, so that the next
+// scores wait for the product with the values, and one stage of keys and values does.  A tile waits mostly for the chain of its row
+// threads (6,000 of 8,200 clocks), which the other CTA fills: 16 heads of 128, window 1,024, capped, 777 + 1,262 + 2,048 tokens, us: one
+// CTA, one thread a row 103, two threads 94; scores capped by multiply-adds 86; two CTAs and the cap's polynomial in raw scores 73.
+// 16 heads of 64, the same: 70 -> 55.  Without a cap, in instances of their own, 25 heads of 64, nine prompts of 335 to 1,023: 75 -> 69.
+// Tried and not kept: the base of the exponentials behind the maximum by up to a factor of 256 (hardly faster, and the largest weight of a
+// row is no longer exact in bfloat16), and blocks of all entries in order of their length (73.0 -> 72.3, two prompts of 1,024 18.0 -> 19.1).
+template <int HD, int SPLIT, int RESIDENT>
 struct Layout {
     static constexpr int ROW_THREADS = 128 * SPLIT, THREADS = 64 + ROW_THREADS;
     static constexpr int COLS = BKEY / SPLIT;                         // keys of a tile per row thread
+    static constexpr bool SHARED = HD == 128 && RESIDENT == 2;        // P lies where S was
+    static constexpr int KV_STAGES = SHARED ? 1 : 2;
     static constexpr int KCH = HD / 64;                               // 64-wide pieces of the head dim
     static constexpr int Q_BYTES = BQ * HD * 2;                       // [KCH][128 rows][128 bytes]
     static constexpr int KV_BYTES = BKEY * HD * 2;                    // one K or V tile, same arrangement
-    static constexpr int STAGE_BYTES = 2 * KV_BYTES;                  // K then V
+    static constexpr int STAGE_BYTES = 2 * KV_BYTES;                  // K then V, each with barriers of its own
     // after the tiles: barriers (256 bytes), then what row partners exchange: [2 tiles][SPLIT][128] slots
     static constexpr int EXCHANGE_BYTES = 2 * SPLIT * BQ * 8;
     static constexpr size_t SMEM = Q_BYTES + (size_t)KV_STAGES * STAGE_BYTES + 1024 + 256 + EXCHANGE_BYTES;
     // TMEM columns: S (128 fp32) | P (64 columns of packed bf16 pairs) | O_j (HD fp32)
-    static constexpr int S_COL = 0, P_COL = 128, O_COL = 192;
-    static constexpr int TMEM_COLS = HD == 64 ? 256 : 512;
+    static constexpr int S_COL = 0, P_COL = SHARED ? 0 : 128, O_COL = SHARED ? 128 : 192;
+    static constexpr int TMEM_COLS = HD == 64 || SHARED ? 256 : 512;
+    // first column of P of a row thread, which holds COLS keys: where P takes the place of S, in that thread's own columns of S
+    __host__ __device__ static constexpr int p_col(int half) { return P_COL + half * (SHARED ? COLS : COLS / 2); }
 };
 
-template <int HD, int SPLIT>
-__global__ void __launch_bounds__(64 + 128 * SPLIT, (HD == 64 && SPLIT == 1) ? 2 : 1)
+// CAPPED: scores go through the cap (instances of their own: the others would spill registers)
+template <int HD, int SPLIT, bool CAPPED, int RESIDENT>
+__global__ void __launch_bounds__(64 + 128 * SPLIT, RESIDENT)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                             __nv_bfloat16* __restrict__ out, int out_stride, const int* __restrict__ q_start,
                             const int* __restrict__ kv_len, const int* __restrict__ block_table, int bt_stride,
@@ -194,17 +206,19 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             int n_kv_heads, int page_size, int window,
                             float scale_log2, long long k_row_base, long long v_row_base, long long page_rows,
                             int* __restrict__ status, SoftmaxExtras extras, int all_values) {
-    using L = Layout<HD, SPLIT>;
-    constexpr int ROW_THREADS = L::ROW_THREADS, THREADS = L::THREADS, COLS = L::COLS;
+    using L = Layout<HD, SPLIT, RESIDENT>;
+    constexpr int ROW_THREADS = L::ROW_THREADS, THREADS = L::THREADS, COLS = L::COLS, KV_STAGES = L::KV_STAGES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* q_s = base;
     unsigned char* kv_s = base + L::Q_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(kv_s + (size_t)KV_STAGES * L::STAGE_BYTES);
     uint64_t* q_full = bars;                  // TMA -> MMA
-    uint64_t* kv_full = bars + 1;             // [KV_STAGES] TMA -> MMA
-    uint64_t* kv_empty = kv_full + KV_STAGES; // [KV_STAGES] MMA -> TMA
-    uint64_t* s_full = kv_empty + KV_STAGES;  // MMA -> softmax: S is complete
+    uint64_t* k_full = bars + 1;              // [KV_STAGES] TMA -> MMA
+    uint64_t* k_empty = k_full + KV_STAGES;   // [KV_STAGES] MMA -> TMA
+    uint64_t* v_full = k_empty + KV_STAGES;   // [KV_STAGES] TMA -> MMA, and the row threads that clear rows of V
+    uint64_t* v_empty = v_full + KV_STAGES;   // [KV_STAGES] MMA -> TMA
+    uint64_t* s_full = v_empty + KV_STAGES;   // MMA -> softmax: S is complete
     uint64_t* p_ready = s_full + 1;           // softmax (all row threads) -> MMA: P is in TMEM, S and O_j are consumed
     uint64_t* o_full = p_ready + 1;           // MMA -> softmax: O_j is complete
     uint64_t* s_free = o_full + 1;            // softmax (all row threads) -> MMA: S is in registers, the next S may land
@@ -238,7 +252,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         mbar_init(q_full, 1);
-        for (int s = 0; s < KV_STAGES; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
+        for (int s = 0; s < KV_STAGES; ++s) {
+            mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1);
+            mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+        }
         mbar_init(s_full, 1);
         mbar_init(p_ready, ROW_THREADS);
         mbar_init(o_full, 1);
@@ -275,19 +292,23 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // the page id is read before the wait: the table lookups of all pages run in parallel and overlap it
             long long page = 0;
             if (lane >= pg_lo && lane <= pg_hi) page = bt[key0 / page_size + lane];
-            if (!mbar_wait(&kv_empty[s], ((it / KV_STAGES) & 1) ^ 1, abort_flag)) { if (lane == 0) atomicExch(status, 31); break; }
             unsigned char* k_dst = kv_s + (size_t)s * L::STAGE_BYTES;
             unsigned char* v_dst = k_dst + L::KV_BYTES;
-            if (lane == 0) mbar_expect_tx(&kv_full[s], 2u * L::KCH * page_bytes * (uint32_t)(pg_hi - pg_lo + 1));
-            __syncwarp();
-            if (lane >= pg_lo && lane <= pg_hi) {
-                const long long row = page * page_rows + (long long)g * page_size;
+            const uint32_t bytes = (uint32_t)L::KCH * page_bytes * (uint32_t)(pg_hi - pg_lo + 1), free = ((it / KV_STAGES) & 1) ^ 1;
+            const bool mine = lane >= pg_lo && lane <= pg_hi;
+            const long long row = page * page_rows + (long long)g * page_size;
+            auto bring = [&](unsigned char* dst, int first_row, uint64_t* full, uint64_t* empty) -> bool {
+                if (!mbar_wait(empty, free, abort_flag)) { if (lane == 0) atomicExch(status, 31); return false; }
+                if (lane == 0) mbar_expect_tx(full, bytes);
+                __syncwarp();
+                if (mine) {
 #pragma unroll
-                for (int c = 0; c < L::KCH; ++c) {
-                    tma_load_2d(k_dst + c * (BKEY * 128) + lane * page_bytes, &map_kv, 64 * c, (int)(k_row_base + row), &kv_full[s]);
-                    tma_load_2d(v_dst + c * (BKEY * 128) + lane * page_bytes, &map_kv, 64 * c, (int)(v_row_base + row) + to_value, &kv_full[s]);
+                    for (int c = 0; c < L::KCH; ++c) tma_load_2d(dst + c * (BKEY * 128) + lane * page_bytes, &map_kv, 64 * c, first_row, full);
                 }
-            }
+                return true;
+            };
+            if (!bring(k_dst, (int)(k_row_base + row), &k_full[s], &k_empty[s])) break;
+            if (!bring(v_dst, (int)(v_row_base + row) + to_value, &v_full[s], &v_empty[s])) break;
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
@@ -301,7 +322,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // S = Q K^T of tile `t` (its K tile must have landed); completion is signalled on s_full
             auto issue_qk = [&](uint32_t t) -> bool {
                 const int st = t % KV_STAGES;
-                if (!mbar_wait(&kv_full[st], (t / KV_STAGES) & 1, abort_flag)) { atomicExch(status, 33); return false; }
+                if (!mbar_wait(&k_full[st], (t / KV_STAGES) & 1, abort_flag)) { atomicExch(status, 33); return false; }
                 tc_fence_after();
                 const uint32_t k_addr = smem_u32(kv_s + (size_t)st * L::STAGE_BYTES);
 #pragma unroll
@@ -310,6 +331,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     for (int k = 0; k < 4; ++k)
                         umma_ss(tmem_base + L::S_COL, desc_sw128(smem_u32(q_s) + c * (BQ * 128), 16) + 2 * k,
                                 desc_sw128(k_addr + c * (BKEY * 128), 16) + 2 * k, idesc_qk, (c | k) ? 1u : 0u);
+                umma_commit(&k_empty[st]);
                 umma_commit(s_full);
                 return true;
             };
@@ -319,20 +341,23 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const int s = it % KV_STAGES;
                 // the scores of the next tile are computed while the rows work on this one: S is free as
                 // soon as every row has it in registers
-                if (it + 1 < n_tiles) {
+                if (!L::SHARED && it + 1 < n_tiles) {
                     if (!mbar_wait(s_free, it & 1, abort_flag)) { atomicExch(status, 34); break; }
                     if (!issue_qk(it + 1)) break;
                 }
                 // P of this tile is in TMEM (and O rescaled): O += P V over the 128 keys, 16 keys = 2048 bytes of V
                 if (!mbar_wait(p_ready, it & 1, abort_flag)) { atomicExch(status, 35); break; }
+                if (!mbar_wait(&v_full[s], (it / KV_STAGES) & 1, abort_flag)) { atomicExch(status, 30); break; }
                 tc_fence_after();
                 const uint32_t v_addr = smem_u32(kv_s + (size_t)s * L::STAGE_BYTES) + L::KV_BYTES;
 #pragma unroll
                 for (int k = 0; k < BKEY / 16; ++k)
-                    umma_ts(tmem_base + L::O_COL, tmem_base + L::P_COL + 8 * k,
+                    umma_ts(tmem_base + L::O_COL, tmem_base + L::p_col(16 * k / COLS) + 8 * (k % (COLS / 16)),
                             desc_sw128(v_addr, BKEY * 128) + (uint64_t)((2048 * k) >> 4), idesc_pv, (it | k) ? 1u : 0u);
-                umma_commit(&kv_empty[s]);
+                umma_commit(&v_empty[s]);
                 umma_commit(o_full);
+                // (MMAs run in the order of their issue: the scores replace P when the product has read it)
+                if (L::SHARED && it + 1 < n_tiles && !issue_qk(it + 1)) break;
             }
         }
     } else {
@@ -353,7 +378,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             l_run = half == 0 ? 1.f : 0.f;
         }
         // capped scores are brought to their final units first and then take the place of the raw ones
-        const float unit_scale = extras.cap_log2 > 0.f ? 1.0f : scale_log2;
+        const float unit_scale = CAPPED ? 1.0f : scale_log2;
         bool ok = true;
         uint32_t it = 0;
         for (int kb = kb_first; kb <= kb_last && ok; ++kb, ++it) {
@@ -364,11 +389,30 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             uint32_t sr[COLS];
             tmem_ld_cols<COLS>(lane_base + L::S_COL + col0, sr);
             tc_fence_before();
-            mbar_arrive(s_free);                                  // the next tile's scores may overwrite S
-            if (extras.cap_log2 > 0.f) {
+            if constexpr (!L::SHARED) mbar_arrive(s_free);        // the next tile's scores may overwrite S
+            if constexpr (CAPPED) {
+                // Special functions are what capped scores wait for: three a score (16 a clock and SM), two of them tanh's.  Scores well
+                // within the cap, the ordinary case, get it from multiply-adds.  (32 at a time: the registers do for no more.)
 #pragma unroll
-                for (int j = 0; j < COLS; ++j)
-                    sr[j] = __float_as_uint(extras.cap_log2 * tanh_ex2(__uint_as_float(sr[j]) * extras.scale_over_cap));
+                for (int c = 0; c < COLS; c += 32) {
+                    float big = 0.f;
+#pragma unroll
+                    for (int j = c; j < c + 32; ++j) big = fmaxf(big, fabsf(__uint_as_float(sr[j])));
+                    if (extras.scale_over_cap >= TANH_LEAST_SCALE && __all_sync(0xffffffffu, big * extras.scale_over_cap <= TANH_RANGE)) {
+                        const CapPolynomial capped(extras);
+#pragma unroll
+                        for (int j = c; j < c + 32; j += 2) {
+                            float even, odd;
+                            pair_split(capped(pair_of(__uint_as_float(sr[j]), __uint_as_float(sr[j + 1]))), even, odd);
+                            sr[j] = __float_as_uint(even);
+                            sr[j + 1] = __float_as_uint(odd);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = c; j < c + 32; ++j)
+                            sr[j] = __float_as_uint(extras.cap_log2 * tanh_ex2(__uint_as_float(sr[j]) * extras.scale_over_cap));
+                    }
+                }
             }
             const bool need_mask = (key0 + COLS - 1 > pos0) || key0 < lo_all || rows < BQ;
             if (need_mask) {
@@ -423,7 +467,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     pr[j >> 1] = *reinterpret_cast<uint32_t*>(&lo2);
                     pr[(j >> 1) + 1] = *reinterpret_cast<uint32_t*>(&hi2);
                 }
-                tmem_st32(lane_base + L::P_COL + ((col0 + c) >> 1), pr);
+                tmem_st32(lane_base + L::p_col(half) + (c >> 1), pr);
             }
             const float sum = (sum0 + sum1) + (sum2 + sum3);
             l_run = l_run * corr + sum;
@@ -443,7 +487,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             // V rows of keys outside [lo, hi] hold stale shared memory or stale cache contents: 0 * garbage
             // must stay 0, so the row's threads clear them (half a row each) before the product reads the tile
-            {
+            if (kb * BKEY + BKEY - 1 > hi || kb * BKEY < lo) {
+                if (!mbar_wait(&v_full[it % KV_STAGES], (it / KV_STAGES) & 1, abort_flag)) { ok = false; if (lane == 0) atomicExch(status, 29); break; }
                 const int key = kb * BKEY + r;
                 if (key > hi || key < lo) {
                     unsigned char* v_tile = kv_s + (size_t)(it % KV_STAGES) * L::STAGE_BYTES + L::KV_BYTES;
@@ -542,7 +587,7 @@ static bool make_map(CUtensorMap* map, const void* base, long long rows, int col
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int HD, int SPLIT>
+template <int HD, int SPLIT, bool CAPPED, int RESIDENT>
 int launch(const void* q, int q_stride, int T, void* out, int out_stride, const void* pool, long long pool_rows,
            long long k_row_base, long long v_row_base, long long page_rows, const int* q_start, const int* kv_len,
            const int* block_table, int bt_stride, const int* item_row, int first_item, int n_items, int max_blocks,
@@ -551,8 +596,8 @@ int launch(const void* q, int q_stride, int T, void* out, int out_stride, const 
     CUtensorMap map_q, map_kv;
     if (!make_map(&map_q, q, T, n_heads * HD, q_stride, BQ)) return PS_ERR_LAUNCH;
     if (!make_map(&map_kv, pool, pool_rows, HD, HD, page_size)) return PS_ERR_LAUNCH;
-    using L = Layout<HD, SPLIT>;
-    auto kernel = prefill_attention_tc_kernel<HD, SPLIT>;
+    using L = Layout<HD, SPLIT, RESIDENT>;
+    auto kernel = prefill_attention_tc_kernel<HD, SPLIT, CAPPED, RESIDENT>;
     static size_t raised[MAX_DEVICES] = {0};
     if (!ensure_dynamic_smem((const void*)kernel, (size_t)L::SMEM, raised)) return PS_ERR_LAUNCH;
     // heads vary fastest: the heaviest query blocks of all heads are scheduled first
@@ -569,7 +614,7 @@ int launch(const void* q, int q_stride, int T, void* out, int out_stride, const 
 // seen as pool_rows rows of head_dim elements; a page's rows start at page * page_rows; within a page the K rows
 // of this cache layer start at k_row_base and the V rows at v_row_base, kv head g at + g * page_size.
 // max_blocks >= sum over the items of ceil(q_len / 128). Head sizes 64 and 128, pages of 8..64 tokens.
-// row_threads: threads per query row, 1 or 2 (0: chosen here).
+// row_threads: 2: one CTA per SM with two threads per query row; 1: two CTAs, with one thread a row where scores have no cap (0: chosen here).
 // item_row (may be null): the block-table row of each item, where the table is kept by request slot.
 // softcap > 0: scores become softcap * tanh(score / softcap); sink (may be null): one float per query head whose
 // exponential joins the softmax's denominator.  all_values: every query head meets the values of every key/value head;
@@ -597,16 +642,19 @@ PS_EXPORT int ps_prefill_attention_tc(const void* q, int q_stride, int T, void* 
     // Measured, 12 heads of 64: 2 x 1,024 tokens 17.6 (two) vs 23.5 us (one); 8 x 1,024: 66.9 vs 53.7 us.
     // row_threads 0 leaves the choice to a count of the blocks.
     const bool two = row_threads ? row_threads == 2 : (long long)max_blocks * n_heads <= 148;
-#define PS_PFTC_LAUNCH(HD, SPLIT)                                                                                     \
-    return ps::pftc::launch<HD, SPLIT>(q, q_stride, T, out, out_stride, pool, pool_rows, k_row_base, v_row_base,     \
-                                       page_rows, q_start, kv_len, block_table, bt_stride, item_row, first_item,      \
-                                       n_items, max_blocks, n_heads, n_kv_heads, page_size, window, scale, status,    \
-                                       softcap, sink, all_values, wide, s)
-    if (head_dim == 64) {
-        if (two) PS_PFTC_LAUNCH(64, 2);
-        PS_PFTC_LAUNCH(64, 1);
-    }
-    if (two) PS_PFTC_LAUNCH(128, 2);
-    PS_PFTC_LAUNCH(128, 1);
+#define PS_PFTC_LAUNCH(HD, SPLIT, CAPPED, RESIDENT)                                                                  \
+    return ps::pftc::launch<HD, SPLIT, CAPPED, RESIDENT>(q, q_stride, T, out, out_stride, pool, pool_rows,           \
+                                       k_row_base, v_row_base, page_rows, q_start, kv_len, block_table, bt_stride,   \
+                                       item_row, first_item, n_items, max_blocks, n_heads, n_kv_heads, page_size,    \
+                                       window, scale, status, softcap, sink, all_values, wide, s)
+    // two CTAs on an SM: one thread a row; with a cap, whose 128 scores a thread do not fit in its registers, two
+#define PS_PFTC_HEADS(HD)                                                                                            \
+    if (two && softcap > 0.f) PS_PFTC_LAUNCH(HD, 2, true, 1);                                                         \
+    if (two) PS_PFTC_LAUNCH(HD, 2, false, 1);                                                                         \
+    if (softcap > 0.f) PS_PFTC_LAUNCH(HD, 2, true, 2);                                                                \
+    PS_PFTC_LAUNCH(HD, 1, false, 2)
+    if (head_dim == 64) { PS_PFTC_HEADS(64); }
+    PS_PFTC_HEADS(128);
+#undef PS_PFTC_HEADS
 #undef PS_PFTC_LAUNCH
 }

@@ -211,6 +211,27 @@ __device__ __forceinline__ float tanh_ex2(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
     return fmaf(-2.0f, r, 1.0f);
 }
+// Capped scores on multiply-adds alone, for raw q.k products within TANH_RANGE of the cap (|raw * scale_over_cap|): cap * tanh(x) is raw
+// times a polynomial in raw^2, whose coefficients take up the scales.  Fitted to tanh(x) / x for the least relative error over the range (1.3e-8;
+// 1.1e-7 with the rounding of the steps).
+constexpr float TANH_RANGE = 0.5f, TANH_LEAST_SCALE = 1e-4f;                       // (below it the last coefficient could vanish)
+struct CapPolynomial {
+    unsigned long long c[5];
+    __device__ __forceinline__ explicit CapPolynomial(const SoftmaxExtras& x) {
+        const float square = x.scale_over_cap * x.scale_over_cap, fit[5] = {1.f, -0.3333306908607483f, 0.13324779272079468f,
+                                                                             -0.05298607423901558f, 0.017135001718997955f};
+        float factor = x.cap_log2 * x.scale_over_cap;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            c[i] = pair_of(fit[i] * factor, fit[i] * factor);
+            factor *= square;
+        }
+    }
+    __device__ __forceinline__ unsigned long long operator()(unsigned long long raw) const {
+        const unsigned long long u = pair_mul(raw, raw);
+        return pair_mul(raw, pair_fma(pair_fma(pair_fma(pair_fma(c[4], u, c[3]), u, c[2]), u, c[1]), u, c[0]));
+    }
+};
 // a raw q.k product in log2 units, capped or not
 __device__ __forceinline__ float score_log2(float raw, float scale_log2, const SoftmaxExtras& x) {
     return x.cap_log2 > 0.f ? x.cap_log2 * tanh_ex2(raw * x.scale_over_cap) : raw * scale_log2;

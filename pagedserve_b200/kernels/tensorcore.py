@@ -112,13 +112,14 @@ def attention(ops, q, out, ctx, layer, n_heads, n_kv_heads, head_dim, window, sc
                                    token_row=ctx.token_slot[:short_tokens], softcap=softcap, sink=sink, all_values=all_values)
     if long_items:
         if ops.prefill_tc_ok(head_dim, layer.page_size, q, every, getattr(layer, "pool", None)):
-            # blocks of 128 queries: never more than the count of 64-query blocks
             # Two threads per query row halve the chain of each 128-key tile but leave one CTA per SM: worth it
             # when all blocks are resident at once, or nearly so while some block runs over many tiles.
-            blocks = -(-ctx.num_long_blocks // 2) * columns          # an upper bound of the 128-query blocks
+            # (an entry of b blocks of 64 queries has at most (b + 1) / 2 of 128)
+            most_blocks = (ctx.num_long_blocks + long_items) // 2
+            blocks = -(-ctx.num_long_blocks // 2) * columns          # near enough the 128-query blocks of all heads
             two = blocks <= 148 or (blocks <= 296 and ctx.max_kv_len >= 768)
             ops.prefill_attention_tc(q, every, layer.pool, layer.pool_layer, ctx.q_start, ctx.kv_len, layer.block_table,
-                                     ctx.num_short_items, long_items, ctx.num_long_blocks, n_heads, n_kv_heads,
+                                     ctx.num_short_items, long_items, most_blocks, n_heads, n_kv_heads,
                                      head_dim, layer.page_size, window, scale, status=ctx.status,
                                      row_threads=2 if two else 1, item_row=ctx.item_slot, softcap=softcap, sink=sink,
                                      all_values=all_values)
