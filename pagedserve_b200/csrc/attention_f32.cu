@@ -1,7 +1,8 @@
 // Paged causal attention in float32 on CUDA cores, for head sizes that are multiples of 4 up to 128 (other sizes run on the
 // general kernel of attention_simt.cu, whose cache layout, masks, cap, sink and all_values these share).
 //
-// prompt_attention_f32_kernel: prompt portions, 64 queries of one head per CTA, key tiles of 64 aligned to absolute positions.
+// prompt_attention_f32_kernel: prompt portions, 64 queries of one head per CTA, key tiles of 64 aligned to absolute positions (head sizes of
+//                              36 to 64 run on tensor cores instead: attention_f32_tc.cu).
 // token_attention_f32_kernel:  single tokens (decode steps, short portions), one CTA per (token, head).
 // Scores, softmax and results are float32 throughout (expf, tanhf).  Within each kernel the order of every sum depends only on a
 // query's position (reference: src/model/paged_attention.py:262-295): its bits are the same whatever else is in the step and, of
@@ -74,7 +75,7 @@ __device__ __forceinline__ void add_values(float (&o)[4][HD / 8], const float* p
 // weights meet the values, the next values while the scores are formed.  Head sizes below HD are filled up with zeros.
 // Blocks late in their prompt see the most keys and go first.
 template <int HD>
-__global__ void __launch_bounds__(PROMPT_THREADS, HD <= 64 ? 3 : 1)
+__global__ void __launch_bounds__(PROMPT_THREADS, HD <= 32 ? 3 : 1)
 prompt_attention_f32_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, int out_stride,
                             const float* __restrict__ k_pool, const float* __restrict__ v_pool, long long page_stride,
                             const int* __restrict__ q_start, const int* __restrict__ kv_len, const int* __restrict__ block_table,
@@ -355,8 +356,7 @@ PS_EXPORT int ps_prompt_attention_f32(const float* q, int q_stride, float* out, 
                                    page_size, all_values);
     if (rc) return rc;
     if (max_blocks > 65535) return PS_ERR_UNSUPPORTED;
-    auto launch = head_dim <= 32 ? ps::af32::launch_prompt<32> : head_dim <= 64 ? ps::af32::launch_prompt<64>
-                                                                                : ps::af32::launch_prompt<128>;
+    auto launch = head_dim <= 32 ? ps::af32::launch_prompt<32> : ps::af32::launch_prompt<128>;
     return launch(q, q_stride, out, out_stride, k_pool, v_pool, page_stride, q_start, kv_len, block_table, bt_stride, item_row,
                   first_item, n_items, max_blocks, n_heads, n_kv_heads, head_dim, page_size, window, scale, softcap, sink,
                   all_values, (cudaStream_t)stream);

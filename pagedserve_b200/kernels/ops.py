@@ -151,6 +151,7 @@ _SIGNATURES = {
     "tc": {
         "ps_gemm_f32_tc": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
         "ps_gemm_f32_tc_parts": [_I],
+        "ps_prompt_attention_f32_tc": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _I, _P, _P],
         "ps_gemm_tc": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P],
         "ps_gemm_rows_tc": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I,
                             _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
@@ -776,6 +777,8 @@ class Ops:
             1 if out.dtype == torch.float32 and self.dtype != torch.float32 else 0, self.code, _stream()), "paged_attention_simt")
         return out
 
+    F32_TC_HEADS = (36, 64)                                 # head sizes of the float32 prompt attention on the tensor cores
+
     @staticmethod
     def attention_f32_ok(q, out, k_pool, v_pool, page_stride, head_dim):
         """Whether the float32 kernels of csrc/attention_f32.cu take these rows: 16-byte pieces, head sizes up to 128."""
@@ -798,18 +801,24 @@ class Ops:
         pools = (_ptr(layer.k_pool), _ptr(layer.v_pool), layer.page_stride)
         table = (_ptr(layer.block_table), layer.block_table.stride(0))
         rest = (n_heads, n_kv_heads, head_dim, layer.page_size, window or 0, scale, float(softcap or 0.0), _ptr(sink),
-                1 if all_values else 0, _stream())
+                1 if all_values else 0)
         if ctx.num_short_tokens:
             self.launches += 1
             _check(self.core.ps_token_attention_f32(_ptr(q), q.stride(0), _ptr(out), out.stride(0), *pools, _ptr(ctx.token_slot),
-                                                    _ptr(ctx.positions), *table, ctx.num_short_tokens, *rest),
+                                                    _ptr(ctx.positions), *table, ctx.num_short_tokens, *rest, _stream()),
                    "token_attention_f32")
         long_items = ctx.num_items - ctx.num_short_items
         if long_items:
             self.launches += 1
-            _check(self.core.ps_prompt_attention_f32(_ptr(q), q.stride(0), _ptr(out), out.stride(0), *pools, _ptr(ctx.q_start),
-                                                     _ptr(ctx.kv_len), *table, _ptr(ctx.item_slot), ctx.num_short_items,
-                                                     long_items, ctx.num_long_blocks, *rest), "prompt_attention_f32")
+            arguments = (_ptr(q), q.stride(0), _ptr(out), out.stride(0), *pools, _ptr(ctx.q_start), _ptr(ctx.kv_len), *table,
+                         _ptr(ctx.item_slot), ctx.num_short_items, long_items)
+            # (by the head size alone: a prompt's bits are the same however it is cut into portions)
+            if self.F32_TC_HEADS[0] <= head_dim <= self.F32_TC_HEADS[1]:
+                # an entry of b blocks of 64 queries has at most (b + 1) / 2 of 128
+                _check(self._tc_library().ps_prompt_attention_f32_tc(*arguments, (ctx.num_long_blocks + long_items) // 2, *rest,
+                                                                     _ptr(self.status_flag(q.device)), _stream()), "prompt_attention_f32_tc")
+            else:
+                _check(self.core.ps_prompt_attention_f32(*arguments, ctx.num_long_blocks, *rest, _stream()), "prompt_attention_f32")
         return out
 
     @staticmethod
@@ -1002,7 +1011,7 @@ class Ops:
         """tcgen05 causal attention of prompt portions (bfloat16, head size 64 or 128).  ``pool`` is the cache
         group's whole pool ``[pages, layers, planes, kv heads, page size, head dim]`` (one plane: the values are the keys); ``cache_layer_local`` the
         layer's index inside it; ``max_blocks`` >= the number of 128-query blocks of the items.
-        ``row_threads``: 1 or 2 threads per query row (0: the kernel's launcher decides)."""
+        ``row_threads``: 2: one CTA per SM, two threads per query row; 1: two CTAs (0: the kernel's launcher decides)."""
         _require(q, "q", torch.bfloat16)
         self._tc_library()
         if status is None:

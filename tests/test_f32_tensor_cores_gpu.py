@@ -1,4 +1,5 @@
-"""Float32 products on the tensor cores (csrc/gemm_f32_tc.cu) against 64 bits and against the float32 multiply-adds they replace."""
+"""Float32 products and prompt attention on the tensor cores (csrc/gemm_f32_tc.cu, csrc/attention_f32_tc.cu) against 64 bits and against the
+float32 multiply-adds they replace."""
 
 import pytest
 import torch
@@ -124,3 +125,49 @@ def test_refused():
         ops.linear_f32_tc(a[:, 1:], w[:, 1:], None, out)
     with pytest.raises(KernelError):
         ops.linear_f32_tc(a[:, :128], w[:, :128], None, out)
+
+
+@pytest.mark.parametrize("head_dim,all_values", [(64, False), (36, True), (60, False)])
+@pytest.mark.parametrize("window,softcap,with_sink", [(0, 0.0, False), (300, 5.0, True), (-200, 0.0, True)])
+def test_prompt_attention(head_dim, all_values, window, softcap, with_sink):
+    """Edges of the blocks of 128 queries and of the tiles of 128 keys, portions behind cached keys; no further from 64 bits than the kernel of
+    multiply-adds (half as much again where both are at a rounding's size)."""
+    from test_f32_kernels_gpu import Step, plain
+
+    entries = [(16, 16), (127, 127), (128, 128), (129, 129), (700, 257), (1100, 20), (512, 128)]
+    step, ops, scale = Step(entries, 4, 2, head_dim, page=16, seed=head_dim), ops_for(), head_dim ** -0.5
+    sink = torch.randn(4, generator=torch.Generator().manual_seed(3)) if with_sink else None
+    q = torch.cat([rows.reshape(len(rows), -1) for rows in step.q]).to(DEV)
+    want = plain(step, scale, window, softcap, sink, all_values)
+    errors = []
+    for heads in (ops.F32_TC_HEADS, (1, 0)):
+        ops.F32_TC_HEADS = heads
+        out = torch.full((len(q), want.shape[1]), float("nan"), device=DEV)
+        ops.attention_f32(q, out, step.ctx, step.layer, 4, 2, head_dim, window, scale, softcap, None if sink is None else sink.to(DEV), all_values)
+        errors.append(float((out.cpu().double() - want).norm() / want.norm()))
+    assert errors[0] <= 1.5 * errors[1] and errors[0] < 1e-6, errors
+    assert int(ops.status.item()) == 0
+
+
+def test_prompt_attention_of_infinities():
+    """Scores and values that are not finite reach the rows that see them, as they do term by term, and no others."""
+    from test_f32_kernels_gpu import Step
+
+    step, ops = Step([(200, 200)], 2, 2, 64, page=16, seed=7), ops_for()
+    layer, q = step.layer, step.q[0].reshape(200, -1).to(DEV)
+    place = lambda token: (int(layer.block_table[int(step.ctx.item_slot[0]), token // 16]), slice(None), token % 16)
+    layer.k_pool[place(60)][:, 5] = float("-inf")
+    layer.v_pool[place(70)][:, 3] = float("inf")
+    layer.v_pool[place(150)][:, 9] = float("nan")
+    layer.k_pool[place(180)][:] = 1e30
+    q[100, 64:] = float("inf")
+    outs = []
+    for heads in (ops.F32_TC_HEADS, (1, 0)):
+        ops.F32_TC_HEADS = heads
+        outs.append(torch.empty(200, 128, device=DEV))
+        ops.attention_f32(q, outs[-1], step.ctx, layer, 2, 2, 64, 0, 0.125)
+    new, old = outs
+    assert torch.equal(torch.isnan(new), torch.isnan(old)) and torch.equal(torch.isinf(new), torch.isinf(old))
+    assert bool(torch.isfinite(new[:60]).all()) and bool(torch.isinf(new[70:, 3]).any()) and bool(torch.isnan(new[160, 9]))
+    there = torch.isfinite(old)
+    assert torch.allclose(new[there], old[there], rtol=1e-5, atol=1e-5)
