@@ -35,11 +35,7 @@ class KernelError(RuntimeError):
 
 def _ptr(tensor):
     """Device address of a tensor (or of a :class:`MappedHostBuffer`); None stays a null pointer."""
-    if tensor is None:
-        return None
-    if isinstance(tensor, MappedHostBuffer):
-        return tensor.device_ptr
-    return tensor.data_ptr()
+    return None if tensor is None else tensor.data_ptr()
 
 
 class MappedHostBuffer:
@@ -54,6 +50,9 @@ class MappedHostBuffer:
         self.device_ptr = device.value
         self.count = count
         self.array = np.ctypeslib.as_array((ctypes.c_int32 * count).from_address(self.host_ptr))
+
+    def data_ptr(self):
+        return self.device_ptr
 
     def close(self):
         if self.host_ptr:
@@ -174,12 +173,13 @@ def _declare(lib, name: str):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_number = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)      # (the tensors at hand: CUDA has been initialised)
 
 
 def _stream():
     """The current CUDA stream's handle (the fast private lookup when torch has it)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_device_number())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -217,6 +217,7 @@ class StepArena:
 
     def __init__(self):
         self.chunks = []             # uint8 tensors, never freed
+        self._kept = []              # of each: its device, its first aligned place, its bytes, views of it by type
         self.chunk = 0
         self.offset = 0
 
@@ -233,29 +234,38 @@ class StepArena:
         self.chunk, self.offset = mark
 
     def empty(self, shape, dtype, device):
-        count = 1
-        for extent in shape:
-            count *= int(extent)
-        nbytes = count * torch.empty((), dtype=dtype).element_size()
+        # One tensor operation a call (each costs the host 1 to 2 us): a view of the chunk that has the type is kept per chunk.
+        shape = tuple(shape)
+        itemsize = dtype.itemsize
+        strides, count = [0] * len(shape), 1
+        for axis in range(len(shape) - 1, -1, -1):
+            strides[axis] = count
+            count *= int(shape[axis])
+        nbytes = count * itemsize
         if nbytes == 0:
-            return torch.empty(tuple(shape), dtype=dtype, device=device)
+            return torch.empty(shape, dtype=dtype, device=device)
         size = -(-nbytes // self.ALIGN) * self.ALIGN
         while True:
             if self.chunk < len(self.chunks):
-                chunk = self.chunks[self.chunk]
-                start = self.offset + (-(chunk.data_ptr() + self.offset)) % self.ALIGN     # an aligned address
-                if chunk.device == torch.device(device) and start + size <= chunk.numel():
-                    piece = chunk[start:start + nbytes]
-                    self.offset = start + size
-                    return piece.view(dtype).view(tuple(shape))
+                where, begin, room, typed = self._kept[self.chunk]
+                start = begin + self.offset                   # (sizes are multiples of ALIGN: an aligned address)
+                if where == torch.device(device) and start + size <= room:
+                    self.offset += size
+                    whole = typed.get(dtype)
+                    if whole is None:
+                        chunk = self.chunks[self.chunk]
+                        whole = typed[dtype] = chunk[:room // itemsize * itemsize].view(dtype)
+                    return whole.as_strided(shape, strides, start // itemsize)
                 self.chunk += 1
                 self.offset = 0
                 continue
             if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
                 # a capture runs the step that an eager run made room for just before; if it asks for more
                 # all the same, the graph's own pool serves it
-                return torch.empty(tuple(shape), dtype=dtype, device=device)
-            self.chunks.append(torch.empty(max(self.CHUNK_BYTES, size) + self.ALIGN, dtype=torch.uint8, device=device))
+                return torch.empty(shape, dtype=dtype, device=device)
+            chunk = torch.empty(max(self.CHUNK_BYTES, size) + self.ALIGN, dtype=torch.uint8, device=device)
+            self.chunks.append(chunk)
+            self._kept.append((chunk.device, -chunk.data_ptr() % self.ALIGN, chunk.numel(), {}))
 
 
 class Ops:

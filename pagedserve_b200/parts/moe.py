@@ -104,11 +104,16 @@ class RoutedExperts(FeedForward):
 
     def bind(self, tensors):
         t = lambda name: tensors[self._n(name)]
-        names = self._expert_names()
+        names, p = self._expert_names(), self.params
         self.router = t("router").contiguous()
         self.w_gate_up = torch.cat([t(name + which) for name in names for which in (("gate", "up") if self.gated else ("up",))],
                                    dim=0).contiguous()           # [2 * columns, W]: per expert its gates, then its ups
         self.w_down = torch.cat([t(name + "down") for name in names], dim=1).contiguous()      # [W, columns]
+        # the parts of the two that the sorted path's products take: routed experts, shared expert
+        wide = p["n_experts"] * (2 if self.gated else 1) * p["expert_ff"]
+        self.w_experts_up, self.w_shared_up = self.w_gate_up[:wide], self.w_gate_up[wide:]
+        narrow = p["n_experts"] * p["expert_ff"]
+        self.w_experts_down, self.w_shared_down = self.w_down[:, :narrow], self.w_down[:, narrow:]
         self.w_shared_gate = t("shared.sg").reshape(-1).contiguous() if self.has_shared_gate else None
         name = self.params.get("correction_name")
         self.correction = t(name).contiguous() if name else None
@@ -172,18 +177,18 @@ class RoutedExperts(FeedForward):
         down = ops.empty((rows_cap, width), torch.float32, device)
         if not self.gated:
             # the activation is the first product's epilogue, the weights join where the rows come together
-            ops.linear_experts(rows, self.w_gate_up, inner, tile_expert, E, act="relu_squared")
-            ops.linear_experts(inner, self.w_down, down, tile_expert, E, along_k=True)
+            ops.linear_experts(rows, self.w_experts_up, inner, tile_expert, E, act="relu_squared")
+            ops.linear_experts(inner, self.w_experts_down, down, tile_expert, E, along_k=True)
             ops.moe_combine(down, row_of, top, residual, weights=chosen_w, factor=self.result_factor)
             return
         if ops.gated_pays(tokens * top + E * (ops.EXPERT_TILE // 2), F):          # (a run's last tile is half full on average)
-            ops.linear_gated(rows, self.w_gate_up[:E * 2 * F], inner, form=self.form, row_weight=row_weight, tile_expert=tile_expert,
+            ops.linear_gated(rows, self.w_experts_up, inner, form=self.form, row_weight=row_weight, tile_expert=tile_expert,
                              experts=E)
         else:
             gate_up = ops.empty((rows_cap, 2 * F), dtype, device)
-            ops.linear_experts(rows, self.w_gate_up[:E * 2 * F], gate_up, tile_expert, E)
+            ops.linear_experts(rows, self.w_experts_up, gate_up, tile_expert, E)
             ops.moe_gate_mul_rows(gate_up, row_weight, inner, form=self.form)
-        ops.linear_experts(inner, self.w_down[:, :E * F], down, tile_expert, E, along_k=True)
+        ops.linear_experts(inner, self.w_experts_down, down, tile_expert, E, along_k=True)
         if self.result_factor is None:
             ops.moe_combine(down, row_of, top, residual)
         else:                                                   # (the weights are in the inner rows already)
@@ -191,14 +196,14 @@ class RoutedExperts(FeedForward):
         shared_ff = p.get("shared_ff") or 0
         if shared_ff:
             inner_shared = ops.empty((tokens, shared_ff), dtype, device)
-            w_shared = self.w_gate_up[E * 2 * F:]
+            w_shared = self.w_shared_up
             if ops.gated_pays(tokens, shared_ff) and ops.gated_ok(x, w_shared, inner_shared):
                 ops.linear_gated(x, w_shared, inner_shared, form=self.form, row_weight=shared_gate)
             else:
                 gate_up_shared = ops.empty((tokens, 2 * shared_ff), dtype, device)
                 ops.linear(x, w_shared, None, gate_up_shared)
                 ops.moe_gate_mul(gate_up_shared, dense, shared_gate, inner_shared, 0, shared_ff, form=self.form)
-            ops.linear(inner_shared, self.w_down[:, E * F:], None, residual, accumulate=True, factor=self.result_factor)
+            ops.linear(inner_shared, self.w_shared_down, None, residual, accumulate=True, factor=self.result_factor)
 
     def _ones(self, like):
         """Float32 ones of the shape of ``like``, kept for the life of the part."""
