@@ -1,6 +1,6 @@
 // Routed experts: the router and the gated inner activation.
 //
-// moe_route, one CTA per token, float32 throughout:
+// moe_route, one CTA per token or per four, float32 throughout:
 //     z = W_router h                    (E numbers; the operands may be bfloat16, sums are float32)
 //     s = softmax(z) over all E experts, or s = sigmoid(z) expert by expert (score_kind 1)
 //     with groups: the experts are `groups` runs of E / groups neighbours; a group's mark is its largest s, or
@@ -36,7 +36,9 @@ namespace ps {
 
 constexpr int MOE_MAX_EXPERTS = 256;
 constexpr int MOE_WARPS = 4;
-constexpr int MOE_BATCH = 16;                     // experts whose sums a lane keeps in registers at a time
+// tokens of a CTA of the router, and experts whose sums a lane keeps in registers at a time
+constexpr int MOE_TOKENS = 4;
+constexpr int moe_batch(int tokens) { return tokens == 1 ? 16 : 8; }
 
 // eight neighbouring elements as floats: one 16-byte access of bfloat16, two of float32
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
@@ -65,8 +67,11 @@ __device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
     *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(MOE_WARPS * 32, 8)
+// What bounds it with many tokens: every token reads all of the router's weights from L1 and L2 (4,099 tokens, 8 experts of 2,048: 134 MB).
+// A CTA takes TOKENS of them, reads the weights once for all, and its warps elect side by side; each sum is that of one token a CTA.
+// 4,099 tokens x 2,048, 8 experts: 29.7 -> 17.5 us; 256 x 1,024 (one token a CTA, fewer exchanges) 6.1 -> 5.7.
+template <typename T, int TOKENS>
+__global__ void __launch_bounds__(MOE_WARPS * 32, TOKENS == 1 ? 8 : 5)
 moe_route_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ router, int router_stride,
                  const T* __restrict__ shared_gate_w, float* __restrict__ dense, int* __restrict__ chosen,
                  float* __restrict__ chosen_w, float* __restrict__ shared_gate, int tokens, int W, int E, int top,
@@ -76,107 +81,145 @@ moe_route_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ ro
     pdl_prologue();
     x = pdl_fresh(x);
     raw = pdl_fresh(raw);
-    // One CTA per token.  The E logits (and the shared gate's, as one more row) are dot products over the row: the
+    // The E logits (and the shared gate's, as one more row) are dot products over the row: the
     // threads of the CTA share the row's columns, so that with eight numbers per thread a row of 1,024 is one round
-    // of loads, all in flight together; partial sums meet in shared memory; warp 0 then holds the election.
-    __shared__ float score[MOE_MAX_EXPERTS + 1];
-    __shared__ float partial[MOE_WARPS][MOE_BATCH];
+    // of loads, all in flight together; partial sums meet in shared memory; a warp then holds a token's election.
+    static_assert(TOKENS <= MOE_WARPS, "a warp elects for a token");
+    constexpr int BATCH = moe_batch(TOKENS);
+    __shared__ float scores[TOKENS][MOE_MAX_EXPERTS + 1];
+    __shared__ float partial[TOKENS][MOE_WARPS][BATCH];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x;
+    const int t0 = blockIdx.x * TOKENS, here = min(TOKENS, tokens - t0);
     if (raw) {
-        // The RMS norm in front, folded in: this CTA norms its token's float32 row (x / sqrt(mean(x^2) + eps) * gain),
-        // leaves the rounded row in x_out for the experts' products, and reads its own numbers back below (every
+        // The RMS norm in front, folded in: this CTA norms its tokens' float32 rows (x / sqrt(mean(x^2) + eps) * gain),
+        // leaves the rounded rows in x_out for the experts' products, and reads its own numbers back below (every
         // thread the columns it wrote itself).
         __shared__ float square[MOE_WARPS];
         __shared__ float inv_shared;
-        const float* source = raw + (size_t)t * raw_stride;
-        T* target = x_out + (size_t)t * x_stride;
-        float sq = 0.f;
-        if (by8) {
-            for (int j = 8 * threadIdx.x; j < W; j += 8 * MOE_WARPS * 32) {
-                float v[8];
-                load8(source + j, v);
+        for (int m = 0; m < here; ++m) {
+            const float* source = raw + (size_t)(t0 + m) * raw_stride;
+            T* target = x_out + (size_t)(t0 + m) * x_stride;
+            float sq = 0.f;
+            if (by8) {
+                for (int j = 8 * threadIdx.x; j < W; j += 8 * MOE_WARPS * 32) {
+                    float v[8];
+                    load8(source + j, v);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) sq = fmaf(v[i], v[i], sq);
+                    for (int i = 0; i < 8; ++i) sq = fmaf(v[i], v[i], sq);
+                }
+            } else {
+                for (int j = threadIdx.x; j < W; j += MOE_WARPS * 32) sq = fmaf(source[j], source[j], sq);
             }
-        } else {
-            for (int j = threadIdx.x; j < W; j += MOE_WARPS * 32) sq = fmaf(source[j], source[j], sq);
-        }
-        sq = warp_sum(sq);
-        if (lane == 0) square[warp] = sq;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float total = 0.f;
-            for (int w = 0; w < MOE_WARPS; ++w) total += square[w];
-            inv_shared = 1.0f / sqrtf(total / (float)W + eps);
-        }
-        __syncthreads();
-        const float inv = inv_shared;
-        if (by8) {
-            for (int j = 8 * threadIdx.x; j < W; j += 8 * MOE_WARPS * 32) {
-                float v[8], g[8];
-                load8(source + j, v);
-                load8(gain + j, g);
+            sq = warp_sum(sq);
+            if (lane == 0) square[warp] = sq;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                float total = 0.f;
+                for (int w = 0; w < MOE_WARPS; ++w) total += square[w];
+                inv_shared = 1.0f / sqrtf(total / (float)W + eps);
+            }
+            __syncthreads();
+            const float inv = inv_shared;
+            if (by8) {
+                for (int j = 8 * threadIdx.x; j < W; j += 8 * MOE_WARPS * 32) {
+                    float v[8], g[8];
+                    load8(source + j, v);
+                    load8(gain + j, g);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = v[i] * inv * g[i];
-                store8(target + j, v);
+                    for (int i = 0; i < 8; ++i) v[i] = v[i] * inv * g[i];
+                    store8(target + j, v);
+                }
+            } else {
+                for (int j = threadIdx.x; j < W; j += MOE_WARPS * 32) target[j] = from_float<T>(source[j] * inv * gain[j]);
             }
-        } else {
-            for (int j = threadIdx.x; j < W; j += MOE_WARPS * 32) target[j] = from_float<T>(source[j] * inv * gain[j]);
+            __syncthreads();
         }
-        __syncthreads();
         x = pdl_fresh(static_cast<const T*>(x_out));      // (a pointer the compiler cannot tie to the stores above)
     }
-    const T* row = x + (size_t)t * x_stride;
-    const int rows = E + (shared_gate_w ? 1 : 0);
-    for (int e0 = 0; e0 < rows; e0 += MOE_BATCH) {
-        float acc[MOE_BATCH];
+    const T* row[TOKENS];                                 // (rows past the last token read that one again)
 #pragma unroll
-        for (int b = 0; b < MOE_BATCH; ++b) acc[b] = 0.f;
+    for (int m = 0; m < TOKENS; ++m) row[m] = x + (size_t)min(t0 + m, tokens - 1) * x_stride;
+    const int rows = E + (shared_gate_w ? 1 : 0);
+    for (int e0 = 0; e0 < rows; e0 += BATCH) {
+        float acc[TOKENS][BATCH];
+#pragma unroll
+        for (int m = 0; m < TOKENS; ++m)
+#pragma unroll
+            for (int b = 0; b < BATCH; ++b) acc[m][b] = 0.f;
         if (by8) {
             for (int j = 8 * threadIdx.x; j < W; j += 8 * MOE_WARPS * 32) {
-                float xv[8];
-                load8(row + j, xv);
+                float xv[TOKENS][8];
 #pragma unroll
-                for (int b = 0; b < MOE_BATCH; ++b) {
+                for (int m = 0; m < TOKENS; ++m) load8(row[m] + j, xv[m]);
+#pragma unroll
+                for (int b = 0; b < BATCH; ++b) {
                     if (e0 + b < rows) {
                         const T* w = e0 + b < E ? router + (size_t)(e0 + b) * router_stride : shared_gate_w;
                         float wv[8];
                         load8(w + j, wv);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) acc[b] = fmaf(xv[i], wv[i], acc[b]);
+                        for (int m = 0; m < TOKENS; ++m)
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) acc[m][b] = fmaf(xv[m][i], wv[i], acc[m][b]);
                     }
                 }
             }
         } else {
             for (int j = threadIdx.x; j < W; j += MOE_WARPS * 32) {
-                const float xv = to_float(row[j]);
+                float xv[TOKENS];
 #pragma unroll
-                for (int b = 0; b < MOE_BATCH; ++b) {
+                for (int m = 0; m < TOKENS; ++m) xv[m] = to_float(row[m][j]);
+#pragma unroll
+                for (int b = 0; b < BATCH; ++b) {
                     if (e0 + b < rows) {
                         const T* w = e0 + b < E ? router + (size_t)(e0 + b) * router_stride : shared_gate_w;
-                        acc[b] = fmaf(xv, to_float(w[j]), acc[b]);
+                        const float wv = to_float(w[j]);
+#pragma unroll
+                        for (int m = 0; m < TOKENS; ++m) acc[m][b] = fmaf(xv[m], wv, acc[m][b]);
                     }
                 }
             }
         }
+        // the sums over the lanes by halving exchanges (the tree of a sum per output, a fifth of the exchanges): a lane
+        // keeps the upper or the lower half of its outputs by one bit of its number, in the end output lane / SHARE
+        constexpr int OUTS = TOKENS * BATCH, SHARE = 32 / OUTS;
+        static_assert(OUTS <= 32 && 32 % OUTS == 0, "a lane ends with the sum of one output");
+        float v[OUTS];
 #pragma unroll
-        for (int b = 0; b < MOE_BATCH; ++b) {
-            const float total = warp_sum(acc[b]);
-            if (lane == 0) partial[warp][b] = total;
+        for (int o = 0; o < OUTS; ++o) v[o] = acc[o / BATCH][o % BATCH];
+        int held = OUTS;
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) {
+            if (held > 1) {
+                held >>= 1;
+                const bool upper = lane & offset;
+#pragma unroll
+                for (int o = 0; o < OUTS / 2; ++o) {
+                    if (o < held) {
+                        const float give = upper ? v[o] : v[o + held], keep = upper ? v[o + held] : v[o];
+                        v[o] = keep + __shfl_xor_sync(0xffffffffu, give, offset);
+                    }
+                }
+            } else {
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], offset);
+            }
         }
+        if (lane % SHARE == 0) partial[lane / SHARE / BATCH][warp][lane / SHARE % BATCH] = v[0];
         __syncthreads();
-        if (threadIdx.x < MOE_BATCH && e0 + threadIdx.x < rows) {
+        if (threadIdx.x < TOKENS * BATCH && e0 + threadIdx.x % BATCH < rows) {
+            const int m = threadIdx.x / BATCH, b = threadIdx.x % BATCH;
             float total = 0.f;
 #pragma unroll
-            for (int w = 0; w < MOE_WARPS; ++w) total += partial[w][threadIdx.x];
-            score[e0 + threadIdx.x] = total;
+            for (int w = 0; w < MOE_WARPS; ++w) total += partial[m][w][b];
+            scores[m][e0 + b] = total;
         }
         __syncthreads();
     }
-    if (warp != 0) return;
+    if (warp >= here) return;
+    const int t = t0 + warp;
+    float* score = scores[warp];
     if (shared_gate_w && lane == 0) shared_gate[t] = 1.0f / (1.0f + expf(-score[E]));
-    // ---- the election, by the lanes of warp 0 together: lane l holds the experts l, l + 32, ...
+    // ---- the election, by the lanes of a warp together: lane l holds the experts l, l + 32, ...
     constexpr int PER_LANE = MOE_MAX_EXPERTS / 32;
     float mine[PER_LANE];
     float top_z = -INFINITY;
@@ -212,7 +255,8 @@ moe_route_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ ro
         // a group's mark is its largest score; groups - keep times the open group with the lowest mark is closed
         // (ties: the higher index goes, so that the lower index stays, as in the election below)
         const int per = E / groups;
-        __shared__ float group_mark[MOE_MAX_EXPERTS];
+        __shared__ float group_marks[TOKENS][MOE_MAX_EXPERTS];
+        float* group_mark = group_marks[warp];
         for (int g = lane; g < groups; g += 32) {
             float m = -INFINITY, second = -INFINITY;
             for (int j = 0; j < per; ++j) {
@@ -250,8 +294,10 @@ moe_route_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ ro
             if (e < E && group_mark[e / per] == INFINITY) mine[i] = -INFINITY;
         }
     }
-    __shared__ int winner[MOE_MAX_EXPERTS];
-    __shared__ float winner_score[MOE_MAX_EXPERTS];
+    __shared__ int winners[TOKENS][MOE_MAX_EXPERTS];
+    __shared__ float winner_scores[TOKENS][MOE_MAX_EXPERTS];
+    int* winner = winners[warp];
+    float* winner_score = winner_scores[warp];
     float total = 0.f;
     for (int k = 0; k < top; ++k) {
         float best = -INFINITY;
@@ -549,18 +595,22 @@ PS_EXPORT int ps_moe_route(const void* x, int x_stride, const void* router, int 
     if (score_kind < 0 || score_kind > 1) return PS_ERR_BAD_ARGUMENT;
     if (E > ps::MOE_MAX_EXPERTS) return PS_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    const dim3 grid(T), block(ps::MOE_WARPS * 32);
+    // Four tokens a CTA where one each would be more than one wave of 8 per SM: with fewer, SMs are idle that the single ones use.  Us, one / four
+    // (with the norm in front, which a CTA does token by token): 1,024 tokens x 1,024, 8 experts 6.3 / 6.0 (7.9 / 9.3), 2,048 11.4 / 7.3 (14.1 /
+    // 11.3), 1,200 x 2,048 14.9 / 8.5 (19.1 / 14.0), 4,099 x 2,048 27.1 / 17.5 (37.2 / 31.7), 64 experts, 600 37.8 / 42.0, 4,000 148 / 100.
+    const bool several = T > 8 * 148;
+    const dim3 grid(several ? (T + ps::MOE_TOKENS - 1) / ps::MOE_TOKENS : T), block(ps::MOE_WARPS * 32);
     // rows of the input and of the router in 32-byte units: eight numbers per access
     const int by8 = W % 8 == 0 && x_stride % 8 == 0 && router_stride % 8 == 0 && !((uintptr_t)x & 31) &&
                     !((uintptr_t)router & 31) && !((uintptr_t)shared_gate_w & 15) &&
                     (!raw || (raw_stride % 8 == 0 && !((uintptr_t)raw & 31) && !((uintptr_t)gain & 31)));
     if (dtype == PS_F32)
-        return ps::launch_pdl(ps::moe_route_kernel<float>, grid, block, 0, s, (const float*)x, x_stride,
+        return ps::launch_pdl(several ? ps::moe_route_kernel<float, ps::MOE_TOKENS> : ps::moe_route_kernel<float, 1>, grid, block, 0, s, (const float*)x, x_stride,
                               (const float*)router, router_stride, (const float*)shared_gate_w, dense, chosen,
                               chosen_w, shared_gate, T, W, E, top, groups, keep, by8, raw, raw_stride, gain, eps,
                               (float*)const_cast<void*>(x), score_kind, normalize, correction, mark_kind, weight_scale);
     if (dtype == PS_BF16)
-        return ps::launch_pdl(ps::moe_route_kernel<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16*)x,
+        return ps::launch_pdl(several ? ps::moe_route_kernel<__nv_bfloat16, ps::MOE_TOKENS> : ps::moe_route_kernel<__nv_bfloat16, 1>, grid, block, 0, s, (const __nv_bfloat16*)x,
                               x_stride, (const __nv_bfloat16*)router, router_stride,
                               (const __nv_bfloat16*)shared_gate_w, dense, chosen, chosen_w, shared_gate, T, W, E, top,
                               groups, keep, by8, raw, raw_stride, gain, eps, (__nv_bfloat16*)const_cast<void*>(x),
