@@ -139,6 +139,7 @@ _SIGNATURES = {
         "ps_gemm_skinny_grouped": [_P, _I, _L, _P, _I, _P, _P, _I, _L, _I, _I, _I, _I, _I, _I, _I, _P],
         "ps_paged_attention_decode_checked": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I,
                                               _F, _I, _I, _P, _P, _P, _P, _P],
+        "ps_attention_lanes": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _F, _P, _I, _I, _P],
         "ps_paged_attention_decode_ex": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I,
                                          _I, _I, _F, _I, _I, _I, _P, _P, _P, _P, _F, _P, _I, _I, _P],
         "ps_shared_position_attention": [_P, _I, _P, _I, _P, _P, _L, _P, _P, _I, _P, _I, _I, _I, _I, _I, _F, _P, _I, _P],
@@ -907,6 +908,33 @@ class Ops:
             page_size, window or 0, scale, split_tiles, n_splits, cluster,
             _ptr(part_acc), _ptr(part_ml), _ptr(counters), _ptr(status), float(softcap or 0.0), _ptr(sink),
             1 if all_values else 0, self._wide(out), _stream()), "paged_attention_decode")
+        return out
+
+    @staticmethod
+    def attention_lanes_ok(q, tokens, k_pool, v_pool, page_stride, head_dim, columns, max_kv_len):
+        """Whether the first ``tokens`` rows (``columns`` results each) run on :meth:`attention_lanes`: 16-byte pieces of rows, lanes that
+        hold a whole row (head sizes of 40 to 64, or 128), and contexts that one CTA walks through in the time that the split keys of
+        :meth:`paged_attention_decode` take, or pairs of token and result enough to fill the SMs.  Us, split / here: 12 heads of 64, 1
+        token, 1,200 keys 8.5 / 6.8, 4,000 7.9 / 19.0, 8 tokens 29.7 / 33.8, 32 tokens, 1,500 keys 66 / 38, 4,000 93.5 / 92.9; 16 heads of 128, 1
+        token, 1,200 keys 7.3 / 12.6, 8 tokens 23.7 / 15.3, 64 tokens 109 / 102; 8 heads of 80, 64 tokens, 300 keys 22.9 / 25.2."""
+        pairs = tokens * columns
+        return ((max_kv_len <= 1280 or pairs > 296) and (32 < head_dim <= 64 or (head_dim == 128 and pairs > 74)) and head_dim % 8 == 0
+                and q.stride(0) % 8 == 0 and q.stride(1) == 1 and page_stride % 8 == 0 and 0 < page_stride < 2 ** 31 and columns <= 65535
+                and all(t.data_ptr() % 16 == 0 for t in (q, k_pool, v_pool)))
+
+    def attention_lanes(self, q, out, k_pool, v_pool, page_stride, token_item, positions, block_table, n_heads, n_kv_heads, head_dim,
+                        page_size, window, scale, max_kv_len, q_start=None, kv_len=None, token_row=None, softcap=None, sink=None,
+                        all_values=False, warps=0):
+        """Attention of single tokens on CUDA cores, one CTA per token and head (csrc/attention_lanes.cu; bfloat16, head sizes that are
+        multiples of 8 up to 128).  Arguments as for :meth:`paged_attention_decode`; ``warps``: of a CTA, 4, 8 or 16 (0: by the count)."""
+        _require(q, "q", torch.bfloat16)
+        self.launches += 1
+        _check(self.fast.ps_attention_lanes(
+            _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_pool), _ptr(v_pool), page_stride, _ptr(token_item), _ptr(token_row),
+            _ptr(positions), _ptr(block_table), block_table.stride(0), _ptr(q_start), _ptr(kv_len), q.shape[0], n_heads, n_kv_heads,
+            head_dim, page_size, window or 0, scale, int(max_kv_len), warps, float(softcap or 0.0), _ptr(sink), 1 if all_values else 0,
+            self._wide(out),
+            _stream()), "attention_lanes")
         return out
 
     def prefill_attention(self, q, out, k_pool, v_pool, page_stride, q_start, kv_len, block_table, first_item,

@@ -98,6 +98,11 @@ def attention(ops, q, out, ctx, layer, n_heads, n_kv_heads, head_dim, window, sc
                            ctx.token_item[:short_tokens], ctx.positions[:short_tokens], layer.block_table, n_heads,
                            n_kv_heads, head_dim, layer.page_size, window, scale, ctx.max_kv_len, q_start=ctx.q_start,
                            kv_len=ctx.kv_len, token_row=ctx.token_slot[:short_tokens], softcap=softcap, sink=sink, mix=mix)
+    elif short_tokens and ops.attention_lanes_ok(q, short_tokens, layer.k_pool, layer.v_pool, layer.page_stride, head_dim, columns, ctx.max_kv_len):
+        ops.attention_lanes(q[:short_tokens], every[:short_tokens], layer.k_pool, layer.v_pool, layer.page_stride,
+                            ctx.token_item[:short_tokens], ctx.positions[:short_tokens], layer.block_table, n_heads, n_kv_heads, head_dim,
+                            layer.page_size, window, scale, ctx.max_kv_len, q_start=ctx.q_start, kv_len=ctx.kv_len,
+                            token_row=ctx.token_slot[:short_tokens], softcap=softcap, sink=sink, all_values=all_values)
     elif short_tokens:
         # The splits of a (token, head) pair merge through global memory. (With at most one pair per SM the
         # kernel makes one CTA of six teams per pair instead and merges in shared memory: batch 8, 278 -> 259 us
