@@ -569,23 +569,42 @@ gemm_f32_rows_walk_kernel(const float* __restrict__ A, int lda, const float* __r
     }
 }
 
+// CTAs of the walking form on an SM at once, by their registers
+constexpr int walkers_per_sm(int tokens, int warps) { return tokens == 2 ? (warps == 6 ? 4 : 3) : tokens == 4 ? (warps == 6 ? 3 : 2) : 2; }
+
+// K up to 1,024: CTAs that stay and walk over the groups where there are more of them than are resident at once (2 to 4 on an SM), each of
+// which would wait for its weights again; few rows leave room for enough (registers) to be as fast without.  Us, one CTA a group / walking: 8
+// rows 2,304 x 768 4.9 / 3.7, 3,072 x 768 6.6 / 4.7, 4,096 x 1,024 9.0 / 6.4, 768 x 768 (one wave) 2.3 / 2.5; 16 rows 768 x 768 5.8 / 3.3,
+// 2,304 x 768 10.7 / 5.3; 4 rows 3,072 x 768 5.0 / 3.6; 2 rows 2,304 x 768 2.2 / 2.8, 4,096 x 1,024 4.5 / 4.8.  As many walkers as are resident: 4 rows x
+// 50,257 x 768, 444 / 592 of them 29 / 37, 2 rows x 50,257 x 1,024 33 / 40.
+// Beyond: the steps whose weights a warp has on their way together, against the registers they take (with 8 rows and one step two CTAs are on
+// an SM, with three one).  Us, 1 / 2 / 3 steps: 2 rows 768 x 3,072 3.7 / 3.4 / 2.7, 4,800 x 1,600 8.1 / 7.3 / 9.1, 1,600 x 6,400 10.2 / 8.8 / 11.5; 4 rows
+// 4,800 x 1,600 12.0 / 9.5 / 9.9, 768 x 3,072 3.9 / 3.6 / 2.8; 8 rows 768 x 3,072 5.3 / 9.2 / 5.9, 1,024 x 4,096 7.0 / 12.7 / 8.7, 1,600 x 6,400 19.7 / 27 / 18.2;
+// 16 rows 768 x 3,072 13.8 / 10.0 / 12.4, 1,600 x 6,400 44 / 31 / 45.
 template <int TOKENS, int COLS>
 int launch_rows(const float* A, int lda, const float* W, int ldw, const float* bias, float* out, int ldo, int M, int N, int K,
                 int act, int accumulate, cudaStream_t s) {
     const int groups = (N + COLS - 1) / COLS;
     const dim3 grid(groups), block(ROWS_WARPS * 32);
-    // more groups than two rounds of CTAs (a vocabulary): CTAs that stay and walk over them
-    if (groups > 4 * 2 * 148 && K <= 128 * ROWS_WARPS) {
-        const dim3 walkers(2 * 2 * 148);
-        if (K <= 128 * 6)
-            return launch_pdl(gemm_f32_rows_walk_kernel<TOKENS, COLS, 6>, walkers, dim3(6 * 32), 0, s, A, lda, W, ldw, bias, out, ldo, M, N,
-                              K, act, accumulate);
-        return launch_pdl(gemm_f32_rows_walk_kernel<TOKENS, COLS, 8>, walkers, block, 0, s, A, lda, W, ldw, bias, out, ldo, M, N, K, act,
-                          accumulate);
+#define PS_ROWS(KERNEL, GRID, BLOCK) return launch_pdl(KERNEL, GRID, BLOCK, 0, s, A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate)
+    if (K <= 128 * ROWS_WARPS) {
+        if (groups > (TOKENS == 2 ? 1184 : 296)) {
+            const bool narrow = K <= 128 * 6;
+            const dim3 walkers(min(groups, 148 * walkers_per_sm(TOKENS, narrow ? 6 : 8)));
+            if (narrow) PS_ROWS((gemm_f32_rows_walk_kernel<TOKENS, COLS, 6>), walkers, dim3(6 * 32));
+            PS_ROWS((gemm_f32_rows_walk_kernel<TOKENS, COLS, 8>), walkers, block);
+        }
+        PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 1>), grid, block);
     }
-    if (K > 128 * ROWS_WARPS)
-        return launch_pdl(gemm_f32_rows_kernel<TOKENS, COLS, 3>, grid, block, 0, s, A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate);
-    return launch_pdl(gemm_f32_rows_kernel<TOKENS, COLS, 1>, grid, block, 0, s, A, lda, W, ldw, bias, out, ldo, M, N, K, act, accumulate);
+    if constexpr (TOKENS == 16) {
+        PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 2>), grid, block);
+    } else if constexpr (TOKENS == 8) {
+        if (K <= 4096) PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 1>), grid, block);
+    } else {
+        if (K <= 2048 || (TOKENS == 2 && K > 4096)) PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 2>), grid, block);
+    }
+    if constexpr (TOKENS < 16) PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 3>), grid, block);
+#undef PS_ROWS
 }
 
 }  // namespace f32
