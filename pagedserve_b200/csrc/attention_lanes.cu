@@ -210,7 +210,7 @@ PS_EXPORT int ps_attention_lanes(const void* q, int q_stride, void* out, int out
         return PS_ERR_UNSUPPORTED;
     if (page_size <= 0 || (page_size & (page_size - 1)) || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15)) return PS_ERR_UNSUPPORTED;
     if (warps != 0 && warps != 4 && warps != 8 && warps != 16) return PS_ERR_BAD_ARGUMENT;
-    // as many warps as leave all CTAs resident (16 heads a token, us with 16 / 8 / 4 warps: 8 tokens, 300 keys 3.7 / 4.7 / 7.5; 16 tokens 7.4 / 6.2 / 9.6;
+    // as many warps as leave all CTAs resident (12 heads a token, us with 16 / 8 / 4 warps: 8 tokens, 300 keys 3.7 / 4.7 / 7.5; 16 tokens 7.4 / 6.2 / 9.6;
     // 32 tokens, 160 keys 10.0 / 7.2 / 6.4; 64 tokens 19.5 / 11.6 / 8.3), more where contexts may be long (32 tokens, 4,000 keys 82 / 93 / 121)
     const long long pairs = (long long)T * n_heads * (all_values ? n_kv_heads : 1);
     if (warps == 0) warps = pairs <= 148 ? 16 : pairs <= (max_kv_len <= 1280 ? 296 : 592) ? 8 : 4;
