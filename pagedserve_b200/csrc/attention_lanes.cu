@@ -144,8 +144,7 @@ attention_lanes_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_b
         }
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-            if (s[u] == -INFINITY) continue;                      // (what is not seen stays out of the sums)
-            const float w = ex2(s[u] - base);
+            const float w = ex2(s[u] - base);                     // (what is not seen: a weight and a row of zeros)
             float x[8];
             unpack(value[u], x);
             l += w;
@@ -177,7 +176,8 @@ attention_lanes_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_b
             total = fmaf(l_s[w], weight, total);
             sum = fmaf(acc_s[w][i], weight, sum);
         }
-        store_result(out, (size_t)t * out_stride + column * head_dim + i, total > 0.f ? sum / total : 0.f, extras);
+        // (no weight at all: zero; a NaN in the total, from the query, a key or infinite scores, stays one)
+        store_result(out, (size_t)t * out_stride + column * head_dim + i, total == 0.f ? sum * 0.f : sum / total, extras);
     }
 }
 

@@ -77,3 +77,41 @@ def test_which_tokens_run_on_it():
     assert ok(1, 64, 8, 1280) and ok(64, 64, 8, 8192) and ok(16, 128, 8, 1024)
     assert not ok(1, 64, 8, 1281) and not ok(1, 128, 8, 1024) and not ok(64, 32, 8, 1024) and not ok(64, 96, 8, 1024)
     assert not ok(1, 64, 8, 1024, stride=16388) and not ok(1, 64, 8, 1024, stride=2 ** 31) and not ok(1, 64, 8, 1024, rows=q[:, 4:])
+
+
+@pytest.mark.parametrize("head_dim", [64, 48, 128])
+@pytest.mark.parametrize("warps", [4, 8, 16])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_numbers_that_are_not_finite(head_dim, warps, with_sink):
+    """A NaN in the query or in a key that it sees, infinite scores of either sign and infinite values give what the split-key kernel and the
+    equations give: NaN in every column, in one column, or an infinity; and other heads, tokens and unseen keys are not touched."""
+    from test_kernels_gpu import PagedCase, ops_for, rel_err
+
+    ops, heads, kv_heads, page = ops_for(torch.bfloat16), 4, 2, 16
+    lengths = [5, 90, 300, 301, 302, 303, 700]
+    case = PagedCase(ops, torch.bfloat16, lengths, heads, kv_heads, head_dim, page, seed=warps)
+    items = torch.arange(len(lengths), dtype=torch.int32, device=DEV)
+    last = torch.tensor(lengths, device=DEV) - 1
+    q = torch.randn(len(lengths), heads * head_dim, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).to(DEV)
+    q[1:, 3] = q[1:, head_dim + 3] = 1.0                         # (heads 0 and 1 read key head 0, heads 2 and 3 key head 1)
+    q[4, head_dim + 3] = -1.0
+    place = lambda item, key: (int(case.table[item, key // page]), 0, key % page)
+    q[0, 2 * head_dim + 1] = float("nan")                        # item 0, head 2
+    case.k_pool[place(1, 17)][3] = float("nan")                  # item 1, heads 0 and 1
+    case.k_pool[place(2, 290)][3] = float("inf")                 # scores of +infinity
+    case.v_pool[place(3, 64)][5] = float("inf")                  # one column
+    case.k_pool[place(4, 100)][3] = float("-inf")                # -infinity for head 0 (a weight of zero), +infinity for head 1
+    case.k_pool[place(5, 7)][3], case.v_pool[place(5, 7)][9] = float("-inf"), float("inf")        # zero times infinity
+    sink = torch.randn(heads, generator=torch.Generator().manual_seed(1)).to(DEV) if with_sink else None
+    arguments = (case.k_pool, case.v_pool, case.page_stride, items, last.to(torch.int32), case.table, heads, kv_heads, head_dim, page, None,
+                 head_dim ** -0.5, max(lengths))
+    out, other = (torch.full((len(lengths), heads * head_dim), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops.attention_lanes(q, out, *arguments, sink=sink, warps=warps)
+    ops.paged_attention_decode(q, other, *arguments, sink=sink)
+    assert torch.equal(out.isnan(), other.isnan()) and torch.equal(out.isinf(), other.isinf())
+    there = out.isfinite()
+    assert rel_err(torch.where(there, out, 0), torch.where(there, other, 0)) < 8e-3
+    rows = out.reshape(len(lengths), heads, head_dim)
+    assert bool(rows[0, 2].isnan().all()) and bool(rows[1, :2].isnan().all()) and bool(rows[2, :2].isnan().all()) and bool(rows[4, 1].isnan().all())
+    assert bool(rows[3, :2, 5].isinf().all()) and bool(rows[5, :2, 9].isnan().all())
+    assert int((~there).sum()) == head_dim * (1 + 2 + 2 + 1) + 2 + 2
