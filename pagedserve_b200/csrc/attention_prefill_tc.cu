@@ -398,7 +398,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     float big = 0.f;
 #pragma unroll
                     for (int j = c; j < c + 32; ++j) big = fmaxf(big, fabsf(__uint_as_float(sr[j])));
-                    if (extras.scale_over_cap >= TANH_LEAST_SCALE && __all_sync(0xffffffffu, big * extras.scale_over_cap <= TANH_RANGE)) {
+                    if (extras.scale_over_cap >= TANH_LEAST_SCALE && extras.scale_over_cap <= TANH_MOST_SCALE &&
+                        __all_sync(0xffffffffu, big * extras.scale_over_cap <= TANH_RANGE)) {
                         const CapPolynomial capped(extras);
 #pragma unroll
                         for (int j = c; j < c + 32; j += 2) {

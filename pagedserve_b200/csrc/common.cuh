@@ -214,7 +214,10 @@ __device__ __forceinline__ float tanh_ex2(float x) {
 // Capped scores on multiply-adds alone, for raw q.k products within TANH_RANGE of the cap (|raw * scale_over_cap|): cap * tanh(x) is raw
 // times a polynomial in raw^2, whose coefficients take up the scales.  Fitted to tanh(x) / x for the least relative error over the range (1.3e-8;
 // 1.1e-7 with the rounding of the steps).
-constexpr float TANH_RANGE = 0.5f, TANH_LEAST_SCALE = 1e-4f;                       // (below it the last coefficient could vanish)
+constexpr float TANH_RANGE = 0.5f;
+// The scales over the cap for which the coefficients are formed (the last one holds the ninth power): below, it could vanish, beyond, it could be
+// an infinity, which times a product of zero is a NaN.
+constexpr float TANH_LEAST_SCALE = 1e-4f, TANH_MOST_SCALE = 1e2f;
 struct CapPolynomial {
     unsigned long long c[5];
     __device__ __forceinline__ explicit CapPolynomial(const SoftmaxExtras& x) {
