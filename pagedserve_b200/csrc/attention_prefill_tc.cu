@@ -392,27 +392,33 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             if constexpr (!L::SHARED) mbar_arrive(s_free);        // the next tile's scores may overwrite S
             if constexpr (CAPPED) {
                 // Special functions are what capped scores wait for: three a score (16 a clock and SM), two of them tanh's.  Scores well
-                // within the cap, the ordinary case, get it from multiply-adds.  (32 at a time: the registers do for no more.)
+                // within the cap, the ordinary case, get it from multiply-adds.  Which of the two a score takes is a matter of its own size:
+                // the columns hold products with rows that no query here sees (left-over memory) as well, and other rows of the warp may be
+                // another entry's, so the warp's largest only says whether anyone needs the functions.  (32 at a time: the registers do for no more.)
+                // Us, one choice for all scores of a warp / a choice per score, two prompts of 1,024, 12 heads of 64, scores of 1 in size:
+                // cap 50 27.5 / 26.7, cap 4 (a score beyond in most warps) 33.7 / 36.4; 16 heads of 128 37.2 / 35.4 and 47.1 / 46.5.
 #pragma unroll
                 for (int c = 0; c < COLS; c += 32) {
+                    const CapPolynomial capped(extras);
                     float big = 0.f;
 #pragma unroll
                     for (int j = c; j < c + 32; ++j) big = fmaxf(big, fabsf(__uint_as_float(sr[j])));
-                    if (extras.scale_over_cap >= TANH_LEAST_SCALE && extras.scale_over_cap <= TANH_MOST_SCALE &&
-                        __all_sync(0xffffffffu, big * extras.scale_over_cap <= TANH_RANGE)) {
-                        const CapPolynomial capped(extras);
+                    const bool special = __any_sync(0xffffffffu, !(big <= extras.polynomial_to));
+                    auto each = [&](auto form) {
 #pragma unroll
                         for (int j = c; j < c + 32; j += 2) {
+                            const float a = __uint_as_float(sr[j]), b = __uint_as_float(sr[j + 1]);
                             float even, odd;
-                            pair_split(capped(pair_of(__uint_as_float(sr[j]), __uint_as_float(sr[j + 1]))), even, odd);
-                            sr[j] = __float_as_uint(even);
-                            sr[j + 1] = __float_as_uint(odd);
+                            pair_split(capped(pair_of(a, b)), even, odd);
+                            sr[j] = __float_as_uint(form(a, even));
+                            sr[j + 1] = __float_as_uint(form(b, odd));
                         }
-                    } else {
-#pragma unroll
-                        for (int j = c; j < c + 32; ++j)
-                            sr[j] = __float_as_uint(extras.cap_log2 * tanh_ex2(__uint_as_float(sr[j]) * extras.scale_over_cap));
-                    }
+                    };
+                    if (!special) each([](float, float polynomial) { return polynomial; });
+                    else each([&](float raw, float polynomial) {
+                        const float function = cap_special(raw, extras);
+                        return fabsf(raw) <= extras.polynomial_to ? polynomial : function;
+                    });
                 }
             }
             const bool need_mask = (key0 + COLS - 1 > pos0) || key0 < lo_all || rows < BQ;

@@ -173,14 +173,19 @@ __device__ __forceinline__ unsigned long long pair_fma(unsigned long long a, uns
 struct SoftmaxExtras {
     float cap_log2;
     float scale_over_cap;
+    float polynomial_to;      // raw products up to this size get their cap from CapPolynomial (negative: none do)
     const float* sink;
     int wide;
 };
+// The part of the cap up to which a polynomial forms tanh, and the scales over the cap for which there is one: its last coefficient holds
+// the ninth power of that number and could vanish below, and beyond could be an infinity, which times a product of zero is a NaN.
+constexpr float TANH_RANGE = 0.5f, TANH_LEAST_SCALE = 1e-4f, TANH_MOST_SCALE = 1e2f;
 __host__ __device__ inline SoftmaxExtras softmax_extras(float scale, float softcap, const float* sink, int wide = 0) {
     SoftmaxExtras e;
     e.wide = wide;
     e.cap_log2 = softcap > 0.f ? softcap * 1.4426950408889634f : 0.f;
     e.scale_over_cap = softcap > 0.f ? scale / softcap : 0.f;
+    e.polynomial_to = e.scale_over_cap >= TANH_LEAST_SCALE && e.scale_over_cap <= TANH_MOST_SCALE ? TANH_RANGE / e.scale_over_cap : -1.f;
     e.sink = sink;
     return e;
 }
@@ -211,13 +216,9 @@ __device__ __forceinline__ float tanh_ex2(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
     return fmaf(-2.0f, r, 1.0f);
 }
-// Capped scores on multiply-adds alone, for raw q.k products within TANH_RANGE of the cap (|raw * scale_over_cap|): cap * tanh(x) is raw
-// times a polynomial in raw^2, whose coefficients take up the scales.  Fitted to tanh(x) / x for the least relative error over the range (1.3e-8;
-// 1.1e-7 with the rounding of the steps).
-constexpr float TANH_RANGE = 0.5f;
-// The scales over the cap for which the coefficients are formed (the last one holds the ninth power): below, it could vanish, beyond, it could be
-// an infinity, which times a product of zero is a NaN.
-constexpr float TANH_LEAST_SCALE = 1e-4f, TANH_MOST_SCALE = 1e2f;
+// Capped scores on multiply-adds alone, for raw q.k products up to SoftmaxExtras::polynomial_to: cap * tanh(x) is raw times a polynomial in
+// raw^2, whose coefficients take up the scales.  Fitted to tanh(x) / x for the least relative error up to TANH_RANGE (1.3e-8; 1.1e-7 with
+// the rounding of the steps).
 struct CapPolynomial {
     unsigned long long c[5];
     __device__ __forceinline__ explicit CapPolynomial(const SoftmaxExtras& x) {
@@ -235,6 +236,10 @@ struct CapPolynomial {
         return pair_mul(raw, pair_fma(pair_fma(pair_fma(pair_fma(c[4], u, c[3]), u, c[2]), u, c[1]), u, c[0]));
     }
 };
+// one product's cap from the special functions, rounded on its own (no addition behind it is fused with it)
+__device__ __forceinline__ float cap_special(float raw, const SoftmaxExtras& x) {
+    return __fmul_rn(x.cap_log2, tanh_ex2(raw * x.scale_over_cap));
+}
 // a raw q.k product in log2 units, capped or not
 __device__ __forceinline__ float score_log2(float raw, float scale_log2, const SoftmaxExtras& x) {
     return x.cap_log2 > 0.f ? x.cap_log2 * tanh_ex2(raw * x.scale_over_cap) : raw * scale_log2;
