@@ -89,9 +89,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const bool two_sums = splits > 1 && splits < parts && rank > 0;    // this CTA's two parts are not added up here
     const int kb0 = part_start(first_part), stages = part_start(last_part) - kb0;
 
-    // the tile's bias (a vector of the weights: nothing of a step makes it)
-    __shared__ __align__(16) float columns[BN];
-    if (threadIdx.x < BN) columns[threadIdx.x] = bias && n0 + (int)threadIdx.x < N ? bias[n0 + threadIdx.x] : 0.f;
+    __shared__ __align__(16) float columns[BN];    // the tile's bias or factors
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         for (int s = 0; s < RAW; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], SPLITTERS / 2); }
@@ -179,6 +177,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         pdl_prologue();
         const int quarter = warp & 3, team = (warp - 4) >> 2;          // TMEM lanes 32 quarter.. (rows), k's 8 team.. and columns 32 team..
         const int row = 32 * quarter + lane;
+        // (behind the wait: the kernel in front may have made the vector; it is there long before the first operands are pieces)
+        if (team == 0) columns[row] = bias && n0 + row < N ? pdl_fresh(bias)[n0 + row] : 0.f;
         const uint32_t tmem_row = tmem + ((uint32_t)(32 * quarter) << 16);
         const int half = team >> 1, sub = team & 1;                    // slot of a stage, 16 k's of the slot
         unsigned long long sum[16], total[16];                         // pairs of columns: of the part, of the parts before it

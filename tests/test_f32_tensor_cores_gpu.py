@@ -114,6 +114,27 @@ def test_products_in_a_row():
         assert float((outs[i].double() - want).abs().max()) < 1e-5 * float(want.abs().max()), i
 
 
+@pytest.mark.parametrize("factor", [False, True])
+def test_vectors_that_the_kernel_in_front_makes(factor):
+    """A bias or a vector of factors may be the result of the kernel in front, which writes it late (K of 8,192), weights ready or not."""
+    ops, g = ops_for(), torch.Generator().manual_seed(4)
+    made, outs = torch.full((1, 700), float("nan"), device=DEV), torch.empty(12, 200, 700, device=DEV)
+    left, right = torch.randn(12, 1, 8192, generator=g).to(DEV), (torch.randn(700, 8192, generator=g) / 90).to(DEV)
+    a, w = torch.randn(200, 768, generator=g).to(DEV), (torch.randn(700, 768, generator=g) / 28).to(DEV)
+    torch.cuda.synchronize()
+    for i in range(12):
+        ops.linear_f32_tc(left[i], right, None, made)
+        if i % 2:
+            ops.linear_f32_tc(a, w, made[0], outs[i], accumulate=2 if factor else 0)
+        else:
+            ops.linear(a, w, None if factor else made[0], outs[i], factor=made[0] if factor else None)
+    for i in range(12):
+        vector = left[i].double() @ right.double().T
+        want = (a.double() @ w.double().T) * vector if factor else a.double() @ w.double().T + vector
+        # (the vector: a sum of 8,192 products)
+        assert float((outs[i].double() - want).abs().max()) < 2 * bound(8192) * size_of(want) * size_of(vector), i
+
+
 def test_refused():
     from pagedserve_b200.kernels.ops import KernelError
 
