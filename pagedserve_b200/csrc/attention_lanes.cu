@@ -55,9 +55,8 @@ attention_lanes_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_b
     const int first_new = (q_start && kv_len) ? kv_len[item] - (q_start[item + 1] - q_start[item]) : 0;
     const int* bt = block_table + (size_t)(token_row ? token_row[t] : item) * bt_stride;
     const int page_size = 1 << page_log2;
-    // from a key's numbers to its value's (which lie in the same pool), and where this lane's numbers of head g begin in a page
+    // from a key's place to its value's in the other pool
     const long long to_value = (all_values ? (long long)(column % n_kv_heads - g) * page_size * head_dim : 0);
-    const int in_page = (g << page_log2) * head_dim + d;
     const bool inside = d < head_dim;
     const int first = lo / SPAN * SPAN;
     auto key_of = [&](int round, int u) { return round + (u * WARPS + warp) * GROUPS + group; };
@@ -210,10 +209,13 @@ PS_EXPORT int ps_attention_lanes(const void* q, int q_stride, void* out, int out
         return PS_ERR_UNSUPPORTED;
     if (page_size <= 0 || (page_size & (page_size - 1)) || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15)) return PS_ERR_UNSUPPORTED;
     if (warps != 0 && warps != 4 && warps != 8 && warps != 16) return PS_ERR_BAD_ARGUMENT;
-    // as many warps as leave all CTAs resident (12 heads a token, us with 16 / 8 / 4 warps: 8 tokens, 300 keys 3.7 / 4.7 / 7.5; 16 tokens 7.4 / 6.2 / 9.6;
-    // 32 tokens, 160 keys 10.0 / 7.2 / 6.4; 64 tokens 19.5 / 11.6 / 8.3), more where contexts may be long (32 tokens, 4,000 keys 82 / 93 / 121)
+    // As many warps as leave all CTAs resident (heads of 64, us with 16 / 8 / 4 warps: 96 pairs of token and head, 300 keys each 5.3 / 5.6 / 7.5; 192
+    // pairs 9.9 / 6.4 / 7.7; 384 pairs, 150 keys 10.3 / 9.5 / 6.3; 768 pairs 20.0 / 14.8 / 8.5).  Where contexts may be long, one long one among
+    // short ones decides, which more warps walk faster: 300 to 592 pairs take 8 there (384 pairs, one context of 1,000 among 150s 14.6 / 15.5 / 19.4,
+    // a fourth of them 15.8 / 16.7 / 20.9, all of 1,000 25.2 / 26.1 / 23.4; 480 pairs 17.5 / 16.0 / 20.5, 19.1 / 17.6 / 25.2, 33.0 / 27.2 / 32.6), and heads
+    // of 128, whose round has half as many keys, from short contexts on (512 pairs, 300 keys 26.5 / 19.1 / 21.5, one of 500 among 60s 16.5 / 14.7 / 19.0).
     const long long pairs = (long long)T * n_heads * (all_values ? n_kv_heads : 1);
-    if (warps == 0) warps = pairs <= 148 ? 16 : pairs <= (max_kv_len <= 1280 ? 296 : 592) ? 8 : 4;
+    if (warps == 0) warps = pairs <= 148 ? 16 : pairs <= 296 || (pairs <= 592 && (max_kv_len > 512 || head_dim > 64)) ? 8 : 4;
 #define PS_LANES(HD, WARPS)                                                                                                               \
     return ps::lanes::launch<HD, WARPS>(q, q_stride, out, out_stride, k_pool, v_pool, page_stride, token_item, token_row, positions,      \
                                         block_table, bt_stride, q_start, kv_len, T, n_heads, n_kv_heads, head_dim, page_size, window,     \

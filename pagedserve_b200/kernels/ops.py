@@ -916,9 +916,14 @@ class Ops:
         hold a whole row (head sizes of 40 to 64, or 128), and contexts that one CTA walks through in the time that the split keys of
         :meth:`paged_attention_decode` take, or pairs of token and result enough to fill the SMs.  Us, split / here: 12 heads of 64, 1
         token, 1,200 keys 8.5 / 6.8, 4,000 7.9 / 19.0, 8 tokens 29.7 / 33.8, 32 tokens, 1,500 keys 66 / 38, 4,000 93.5 / 92.9; 16 heads of 128, 1
-        token, 1,200 keys 7.3 / 12.6, 8 tokens 23.7 / 15.3, 64 tokens 109 / 102; 8 heads of 80, 64 tokens, 300 keys 22.9 / 25.2."""
+        token, 1,200 keys 7.3 / 12.6, 8 tokens 23.7 / 15.3, 64 tokens 109 / 102; 8 heads of 80, 64 tokens, 300 keys 22.9 / 25.2.
+        One long context among short ones, which one CTA walks (32 tokens of 12 heads, one of 1,000 among 150s 15.1 / 15.5, 8,000 69 / 71): heads
+        of 128 with 149 to 296 pairs lose there what they gain where all are long (12 tokens of 16 heads, one of 1,000 among 60s 12.4 / 19.5,
+        all of 750 22.7 / 18.4) and run here to 512 keys only (6.7 / 6.9 with one of 240, 13.5 / 7.9 with all); with fewer the difference is
+        3 us against 8 (8 tokens 9.5 / 12.4, all of 750 19.2 / 11.7)."""
         pairs = tokens * columns
-        return ((max_kv_len <= 1280 or pairs > 296) and (32 < head_dim <= 64 or (head_dim == 128 and pairs > 74)) and head_dim % 8 == 0
+        heads = 32 < head_dim <= 64 or (head_dim == 128 and pairs > 74 and (max_kv_len <= 512 or not 148 < pairs <= 296))
+        return (heads and (max_kv_len <= 1280 or pairs > 296) and head_dim % 8 == 0
                 and q.stride(0) % 8 == 0 and q.stride(1) == 1 and page_stride % 8 == 0 and 0 < page_stride < 2 ** 31 and columns <= 65535
                 and all(t.data_ptr() % 16 == 0 for t in (q, k_pool, v_pool)))
 

@@ -115,3 +115,27 @@ def test_numbers_that_are_not_finite(head_dim, warps, with_sink):
     assert bool(rows[0, 2].isnan().all()) and bool(rows[1, :2].isnan().all()) and bool(rows[2, :2].isnan().all()) and bool(rows[4, 1].isnan().all())
     assert bool(rows[3, :2, 5].isinf().all()) and bool(rows[5, :2, 9].isnan().all())
     assert int((~there).sum()) == head_dim * (1 + 2 + 2 + 1) + 2 + 2
+
+
+def test_contexts_of_different_lengths():
+    """Which kernel and how many warps run where one context may be far longer than the others: heads of 128 with 149 to 296 pairs
+    leave it beyond 512 keys, and 297 to 592 pairs take 8 warps (a number of warps has bits of its own)."""
+    from test_kernels_gpu import PagedCase, ops_for
+
+    ops, pool = ops_for(torch.bfloat16), torch.empty(8, 2, 8, 16, 128, dtype=torch.bfloat16, device=DEV)
+    ok = lambda tokens, longest: ops.attention_lanes_ok(torch.empty(tokens, 1024, dtype=torch.bfloat16, device=DEV), tokens, pool[:, 0], pool[:, 1],
+                                                        16384, 128, 8, longest)
+    assert ok(18, 1024) and not ok(19, 1024) and not ok(37, 513) and ok(19, 512) and ok(37, 512) and ok(38, 1280) and ok(38, 8192) and not ok(37, 8192)
+    for heads, head_dim, longest, warps in ((1, 64, 1024, (16, 8, 8, 8, 4)), (1, 64, 512, (16, 8, 4, 4, 4)), (1, 128, 512, (16, 8, 8, 8, 4))):
+        lengths = [500] + [20] * 9
+        case = PagedCase(ops, torch.bfloat16, lengths, heads, 1, head_dim, 16, seed=1)
+        for tokens, expected in zip((148, 149, 297, 592, 593), warps):
+            item = torch.arange(tokens, dtype=torch.int32, device=DEV) % len(lengths)
+            positions = torch.tensor(lengths, dtype=torch.int32, device=DEV)[item.long()] - 1
+            q = torch.randn(tokens, head_dim, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).to(DEV)
+            outs = []
+            for count in (0, expected) + tuple({4, 8, 16} - {expected}):
+                outs.append(torch.empty(tokens, head_dim, dtype=torch.float32, device=DEV))
+                ops.attention_lanes(q, outs[-1], case.k_pool, case.v_pool, case.page_stride, item, positions, case.table, heads, 1, head_dim, 16,
+                                    None, head_dim ** -0.5, longest, warps=count)
+            assert torch.equal(outs[0], outs[1]) and not torch.equal(outs[0], outs[2]) and not torch.equal(outs[0], outs[3]), (longest, tokens)
