@@ -20,9 +20,13 @@
 // The order of a row's sums depends on its position alone (reference: src/model/paged_attention.py:262-295).
 //
 // What bounds a tile: the chain of softmax (the workers), P V and the next S (72 MMAs, 74 clocks and more each), which follow one another; a CTA
-// fills an SM, so only cutting into pieces overlaps.  Us, multiply-adds (attention_f32.cu) / here, 12 heads of 64: 2 x 1,024 tokens 172 / 57,
-// 5 x 128 18 / 15, 8 x 20 tokens behind 280 39 / 23, 2 x 16 behind 984 115 / 48; a portion with nothing before it pays for its fixed part,
-// 16 tokens 9.4 / 10.4, 4 x 64 10.9 / 12.7.  Error against 64 bits: 2 x 16 behind 984 6.0e-7 / 2.7e-7, 5 x 128 1.6e-7 / 1.4e-7.
+// fills an SM, so only cutting into pieces overlaps.  In the last tile the products stop at the last key (in steps of 16), and a warp whose rows
+// see none of its 32 keys forms no weights (16 tokens 10.4 -> 6.3 us, 4 x 64 12.6 -> 9.9, 5 x 128 14.7 -> 13.8).  Us, multiply-adds (as
+// attention_f32.cu's, for heads of 64) / here, 12 heads of 64: 2 x 1,024 tokens 187 / 51, 5 x 128 18.4 / 13.8, 8 x 20 tokens behind 280
+// 39.5 / 20.4, 2 x 16 behind 984 116 / 48, 16 tokens 9.8 / 6.3, 64 10.5 / 9.6, 4 x 64 10.9 / 9.9.  Error against 64 bits: 2 x 16 behind 984
+// 6.0e-7 / 2.7e-7, 5 x 128 1.6e-7 / 1.4e-7.
+#include <type_traits>
+
 #include "f32_pieces.cuh"
 
 namespace ps {
@@ -159,15 +163,18 @@ prompt_attention_f32_tc_kernel(const float* __restrict__ q, int q_stride, float*
 
     if (warp == WORKERS / 32) {
         if (elect_one()) {
-            // D = f32, A = B = bf16, M = 128; keys K-major, N = 128; values MN-major (bit 16), N = 64
+            // D = f32, A = B = bf16, M = 128; keys K-major, N = 128 or what is left of the last tile; values MN-major (bit 16), N = 64
             constexpr uint32_t kind = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 4) << 24);
-            constexpr uint32_t idesc_s = kind | ((uint32_t)(BKEY >> 3) << 17), idesc_o = kind | (1u << 16) | ((uint32_t)(HD >> 3) << 17);
+            constexpr uint32_t idesc_o = kind | (1u << 16) | ((uint32_t)(HD >> 3) << 17);
             // the six products, the small ones first: pieces of the first and of the second operand
             constexpr int piece_a[6] = {2, 1, 0, 1, 0, 0}, piece_b[6] = {0, 1, 2, 0, 1, 0};
             const uint64_t keys = umma_desc(smem_u32(base + K_OPS));
             for (int it = 0; it <= last - first; ++it) {
                 if (!mbar_wait(k_ready, it & 1, abort_flag)) { atomicExch(status, 61); break; }
                 tc_fence_after();
+                // 16-key steps that anyone sees: the others' scores are masked whatever they are, and their weights and values are zeros
+                const int steps = (min(BKEY, hi - (first + it) * BKEY + 1) + 15) / 16;
+                const uint32_t idesc_s = kind | ((uint32_t)(2 * steps) << 17);
 #pragma unroll
                 for (int product = 0; product < 6; ++product)
 #pragma unroll
@@ -178,12 +185,21 @@ prompt_attention_f32_tc_kernel(const float* __restrict__ q, int q_stride, float*
                 if (!mbar_wait(p_ready, it & 1, abort_flag)) { atomicExch(status, 62); break; }
                 tc_fence_after();
                 const uint64_t values = umma_desc(smem_u32(base + V_OPS + (it & 1) * OPS_BYTES));
+                auto step = [&](int product, int k) {            // 16 keys: 2,048 bytes of values
+                    umma_ts(tmem + O_COL, tmem + P_COL + 64 * piece_a[product] + 8 * k, values + piece_b[product] * (PLANE >> 4) + 128 * k, idesc_o,
+                            (product | k) ? 1u : 0u);
+                };
+                if (steps == BKEY / 16) {
 #pragma unroll
-                for (int product = 0; product < 6; ++product)
+                    for (int product = 0; product < 6; ++product)
 #pragma unroll
-                    for (int k = 0; k < BKEY / 16; ++k)          // 16 keys: 2,048 bytes of values
-                        umma_ts(tmem + O_COL, tmem + P_COL + 64 * piece_a[product] + 8 * k, values + piece_b[product] * (PLANE >> 4) + 128 * k, idesc_o,
-                                (product | k) ? 1u : 0u);
+                        for (int k = 0; k < BKEY / 16; ++k) step(product, k);
+                } else {
+#pragma unroll
+                    for (int product = 0; product < 6; ++product)
+#pragma unroll 1
+                        for (int k = 0; k < steps; ++k) step(product, k);
+                }
                 umma_commit(o_full);
             }
         }
@@ -224,10 +240,11 @@ prompt_attention_f32_tc_kernel(const float* __restrict__ q, int q_stride, float*
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto cut = [&](int raw, unsigned char* to, bool values) {    // the older of the two groups on their way has come
+    auto cut = [&](int tile, int raw, unsigned char* to, bool values) {          // the older of the two groups on their way has come
         asm volatile("cp.async.wait_group 1;" ::: "memory");
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
+            if (tile * BKEY + 64 * i > hi) break;                // (no step of the products reads these rows)
             float4 v[2];
 #pragma unroll
             for (int half = 0; half < 2; ++half) v[half] = *reinterpret_cast<const float4*>(base + raw + ((2 * i + half) * WORKERS + tid) * 16);
@@ -278,10 +295,10 @@ prompt_attention_f32_tc_kernel(const float* __restrict__ q, int q_stride, float*
         for (int p = 0; p < 3; ++p) tmem_st8(tmem_row + Q_COL + 32 * p + 8 * team, piece[p]);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
-    cut(K_RAW, base + K_OPS, false);
+    cut(first, K_RAW, base + K_OPS, false);
     arrive(k_ready);
     bring(first + 1, k_pool, 0, K_RAW);
-    cut(V_RAW, base + V_OPS, true);
+    cut(first, V_RAW, base + V_OPS, true);
     bring(first + 1, v_pool, to_value, V_RAW);
 
     float o[16], m = -INFINITY, l = 0.f;                         // l: of this thread's keys
@@ -295,32 +312,36 @@ prompt_attention_f32_tc_kernel(const float* __restrict__ q, int q_stride, float*
 #pragma unroll
         for (int d = 0; d < 16; ++d) o[d] += __uint_as_float(r[d]);
     };
-    for (int tile = first; tile <= last; ++tile) {
+    // A tile.  LAST: the last one, of whose keys a warp's rows may see none (a team's keys begin beyond the diagonal or the end): it forms no
+    // weights then and stores zeros.  (Every rounding is written out, so that both forms have the same bits.)
+    auto work = [&](int tile, auto last_tile) {
+        constexpr bool LAST = decltype(last_tile)::value;
         const int it = tile - first;
         if (it > 0) drain(it - 1);
         await(s_full, it & 1, 63);
         float s[32], top = -INFINITY;
-        {
+        const int key0 = tile * BKEY + 32 * team;
+        const bool seen = !LAST || key0 <= min(pos0 + 32 * quarter + 31, hi);
+        if (seen) {
             uint32_t r[16];
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 tmem_ld16(tmem_row + S_COL + 32 * team + 16 * half, r);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int j = 0; j < 16; ++j) s[16 * half + j] = __uint_as_float(r[j]) * scale;
+                for (int j = 0; j < 16; ++j) s[16 * half + j] = __fmul_rn(__uint_as_float(r[j]), scale);
             }
-        }
-        if (softcap > 0.f) {
+            if (softcap > 0.f) {
 #pragma unroll 4
-            for (int j = 0; j < 32; ++j) s[j] = capped(s[j], softcap);
-        }
-        const int key0 = tile * BKEY + 32 * team;
-        if (key0 + 31 > pos || key0 < low) {
+                for (int j = 0; j < 32; ++j) s[j] = capped(s[j], softcap);
+            }
+            if (key0 + 31 > pos || key0 < low) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) s[j] = key0 + j <= pos && key0 + j >= low ? s[j] : -INFINITY;
-        }
+                for (int j = 0; j < 32; ++j) s[j] = key0 + j <= pos && key0 + j >= low ? s[j] : -INFINITY;
+            }
 #pragma unroll
-        for (int j = 0; j < 32; ++j) top = fmaxf(top, s[j]);
+            for (int j = 0; j < 32; ++j) top = fmaxf(top, s[j]);
+        }
         float* shared_top = exchange + (it & 1) * 4 * BQ + row;  // (two buffers: one barrier a tile is enough)
         shared_top[team * BQ] = top;
         asm volatile("bar.sync %0, 128;" ::"r"(2 + quarter) : "memory");
@@ -330,32 +351,41 @@ prompt_attention_f32_tc_kernel(const float* __restrict__ q, int q_stride, float*
         const float m_base = m_new == -INFINITY ? 0.f : m_new;   // a row that sees no key of this tile or before it
         const float shrink = expf(m - m_base);
         m = m_new;
-        l *= shrink;
+        if (!seen) l = __fmul_rn(l, shrink);
 #pragma unroll
-        for (int d = 0; d < 16; ++d) o[d] *= shrink;
+        for (int d = 0; d < 16; ++d) o[d] = __fmul_rn(o[d], shrink);
+        if (seen) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            uint32_t piece[3][8];
+            for (int half = 0; half < 2; ++half) {
+                uint32_t piece[3][8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float even = expf(s[16 * half + 2 * j] - m_base), odd = expf(s[16 * half + 2 * j + 1] - m_base);
-                l += even;
-                l += odd;
-                split(even, odd, piece[0][j], piece[1][j], piece[2][j]);
+                for (int j = 0; j < 8; ++j) {
+                    const float even = expf(__fsub_rn(s[16 * half + 2 * j], m_base)), odd = expf(__fsub_rn(s[16 * half + 2 * j + 1], m_base));
+                    l = half == 0 && j == 0 ? fmaf(l, shrink, even) : l + even;
+                    l += odd;
+                    split(even, odd, piece[0][j], piece[1][j], piece[2][j]);
+                }
+#pragma unroll
+                for (int p = 0; p < 3; ++p) tmem_st8(tmem_row + P_COL + 64 * p + 16 * team + 8 * half, piece[p]);
             }
-#pragma unroll
-            for (int p = 0; p < 3; ++p) tmem_st8(tmem_row + P_COL + 64 * p + 16 * team + 8 * half, piece[p]);
+        } else if (key0 <= hi) {
+            const uint32_t none[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll 1
+            for (int i = 0; i < 6; ++i) tmem_st8(tmem_row + P_COL + 64 * (i >> 1) + 16 * team + 8 * (i & 1), none);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         arrive(p_ready);
-        if (tile < last) {
-            cut(K_RAW, base + K_OPS, false);
+        if constexpr (!LAST) {
+            cut(tile + 1, K_RAW, base + K_OPS, false);
             arrive(k_ready);
             bring(tile + 2, k_pool, 0, K_RAW);
-            cut(V_RAW, base + V_OPS + ((it + 1) & 1) * OPS_BYTES, true);
+            cut(tile + 1, V_RAW, base + V_OPS + ((it + 1) & 1) * OPS_BYTES, true);
             bring(tile + 2, v_pool, to_value, V_RAW);
         }
-    }
+    };
+#pragma unroll 1
+    for (int tile = first; tile < last; ++tile) work(tile, std::false_type());
+    work(last, std::true_type());
     drain(last - first);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     // the row's sum is that of its four threads, in order; both buffers of the exchange are free behind the barrier

@@ -170,6 +170,28 @@ def test_prompt_attention(head_dim, all_values, window, softcap, with_sink):
     assert int(ops.status.item()) == 0
 
 
+@pytest.mark.parametrize("before", [0, 70, 128])
+@pytest.mark.parametrize("softcap", [0.0, 5.0])
+def test_prompt_attention_of_part_of_a_tile(before, softcap):
+    """The last tile's products are formed for the keys that are there, in steps of 16: a portion that ends at each edge of a step has the
+    bits of those rows of a longer one."""
+    from test_f32_kernels_gpu import Step, plain
+
+    ops, outs = ops_for(), {}
+    for end in [before + 160] + [before + n for n in (16, 17, 31, 32, 33, 48, 58, 59, 64, 65, 80, 96, 112, 113, 127, 128, 129, 144)]:
+        step = Step([(before + 160, 160)], 2, 1, 64, page=16, seed=9)
+        count = end - before
+        step.ctx.q_start[1], step.ctx.kv_len[0], step.ctx.num_long_blocks = count, end, (count + 63) // 64
+        q = step.q[0].reshape(160, -1)[:count].to(DEV)
+        outs[count] = torch.full((count, 128), float("nan"), device=DEV)
+        ops.attention_f32(q, outs[count], step.ctx, step.layer, 2, 1, 64, 0, 0.125, softcap or None)
+    want = plain(step, 0.125, 0, softcap, None, False)
+    assert float((outs[160].cpu().double() - want).norm() / want.norm()) < 1e-6
+    for count, out in outs.items():
+        assert torch.equal(out, outs[160][:count]), count
+    assert int(ops.status.item()) == 0
+
+
 def test_prompt_attention_of_infinities():
     """Scores and values that are not finite reach the rows that see them, as they do term by term, and no others."""
     from test_f32_kernels_gpu import Step
