@@ -579,7 +579,8 @@ constexpr int walkers_per_sm(int tokens, int warps) { return tokens == 2 ? (warp
 // 50,257 x 768, 444 / 592 of them 29 / 37, 2 rows x 50,257 x 1,024 33 / 40.
 // Beyond: the steps whose weights a warp has on their way together, against the registers they take (with 8 rows and one step two CTAs are on
 // an SM, with three one).  Us, 1 / 2 / 3 steps: 2 rows 768 x 3,072 3.7 / 3.4 / 2.7, 4,800 x 1,600 8.1 / 7.3 / 9.1, 1,600 x 6,400 10.2 / 8.8 / 11.5; 4 rows
-// 4,800 x 1,600 12.0 / 9.5 / 9.9, 768 x 3,072 3.9 / 3.6 / 2.8; 8 rows 768 x 3,072 5.3 / 9.2 / 5.9, 1,024 x 4,096 7.0 / 12.7 / 8.7, 1,600 x 6,400 19.7 / 27 / 18.2;
+// 4,800 x 1,600 12.0 / 9.5 / 9.9, 768 x 3,072 3.9 / 3.6 / 2.8; 8 rows 768 x 3,072 5.3 / 9.2 / 5.9, 1,024 x 4,096 7.0 / 12.7 / 8.7, 1,600 x 6,400 19.7 / 27 / 18.2,
+// but where each CTA has an SM to itself one step leaves it waiting: 592 x 3,072 (148 CTAs) 4.3 with one, 3.0 with three, 600 x 3,072 4.2 / 5.0;
 // 16 rows 768 x 3,072 13.8 / 10.0 / 12.4, 1,600 x 6,400 44 / 31 / 45.
 template <int TOKENS, int COLS>
 int launch_rows(const float* A, int lda, const float* W, int ldw, const float* bias, float* out, int ldo, int M, int N, int K,
@@ -599,7 +600,7 @@ int launch_rows(const float* A, int lda, const float* W, int ldw, const float* b
     if constexpr (TOKENS == 16) {
         PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 2>), grid, block);
     } else if constexpr (TOKENS == 8) {
-        if (K <= 4096) PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 1>), grid, block);
+        if (K <= 4096 && groups > 148) PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 1>), grid, block);
     } else {
         if (K <= 2048 || (TOKENS == 2 && K > 4096)) PS_ROWS((gemm_f32_rows_kernel<TOKENS, COLS, 2>), grid, block);
     }
