@@ -102,20 +102,23 @@ def bench_attention(args):
     pool = torch.randn(B * pages_per + 1, layers, 2, H, page, D, device="cuda").to(torch.bfloat16)
     table = torch.randperm(B * pages_per, device="cuda").to(torch.int32).view(B, pages_per)
     q = torch.randn(B, H * D, device="cuda").to(torch.bfloat16)
-    out = torch.empty_like(q, dtype=torch.float32 if wide else None)
+    out = torch.empty_like(q)
     token_item = torch.arange(B, dtype=torch.int32, device="cuda")
     positions = torch.full((B,), ctx - 1, dtype=torch.int32, device="cuda")
     stride = layers * 2 * H * page * D
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
 
+    longest = args.max_context or ctx
+    attend, kernel = _token_attention(ops, q, pool, stride, H, H, D, longest)
+
     def run(i):
         layer = i % layers
-        ops.paged_attention_decode(q, out, pool[:, layer, 0], pool[:, layer, 1], stride, token_item, positions, table,
-                                   H, H, D, page, None, D ** -0.5, args.max_context or ctx, status=status)
+        attend(q, out, pool[:, layer, 0], pool[:, layer, 1], stride, token_item, positions, table, H, H, D, page, None, D ** -0.5, longest,
+               status=status)
 
     seconds = _time(run, args.iters, graph=args.graph)
     nbytes = B * ctx * H * D * 2 * 2
-    print(f"decode attention B={B} ctx={ctx} heads={H} hd={D} page={page}: {seconds * 1e6:.2f} us, "
+    print(f"decode attention ({kernel}) B={B} ctx={ctx} heads={H} hd={D} page={page}: {seconds * 1e6:.2f} us, "
           f"{nbytes / seconds / 1e9:.0f} GB/s of K+V, status {int(status.item())}")
 
 
@@ -131,10 +134,21 @@ def _paged_inputs(items, context, kv_heads, head_dim, page, rotate_mb=200, plane
     return pool, table, layers, layers * planes * kv_heads * page * head_dim
 
 
+def _token_attention(ops, q, pool, stride, heads, kv_heads, head_dim, longest, every_value=False):
+    """What :func:`pagedserve_b200.kernels.tensorcore.attention` runs for these single tokens where the heads of a group are not the rows
+    of a tile, and its name."""
+    from pagedserve_b200.kernels.tensorcore import ROWS_FROM_HEADS
+
+    columns = heads * kv_heads if every_value else heads
+    if heads < ROWS_FROM_HEADS * kv_heads and ops.attention_lanes_ok(q, q.shape[0], pool, pool, stride, head_dim, columns, longest):
+        return lambda *arguments, status=None, **options: ops.attention_lanes(*arguments, **options), "lanes"
+    return ops.paged_attention_decode, "split keys"
+
+
 def time_decode_attention(batch, context, heads, kv_heads, head_dim, page=16, window=None, softcap=None,
                           sink=False, iters=20, planes=2, chunk=None, mixed=False, as_rows=False, splits=None, wide=False):
-    """One decode token per request over ``context`` keys (bfloat16 split-key kernel); GB/s over the K and V
-    bytes a token may see (with one plane: over the rows once).  ``mixed``: a layer whose heads' weights are mixed
+    """One decode token per request over ``context`` keys (bfloat16; the kernel that the engine takes for these sizes, named in
+    the result); GB/s over the K and V bytes a token may see (with one plane: over the rows once).  ``mixed``: a layer whose heads' weights are mixed
     across heads (every query head meets all values, then the mixing kernel).  ``as_rows``: the kernel with the heads of a
     group (mixed: all heads) as the rows of a tile, a token's keys shared out over ``splits`` CTAs (None: its own rule).
     ``wide``: the result is left as float32."""
@@ -143,25 +157,28 @@ def time_decode_attention(batch, context, heads, kv_heads, head_dim, page=16, wi
     ops = Ops(torch.bfloat16)
     pool, table, layers, stride = _paged_inputs(batch, context, kv_heads, head_dim, page, planes=planes)
     q = torch.randn(batch, heads * head_dim, device="cuda").to(torch.bfloat16)
-    out = torch.empty_like(q)
+    out = torch.empty_like(q, dtype=torch.float32 if wide else None)
     token_item = torch.arange(batch, dtype=torch.int32, device="cuda")
     positions = torch.full((batch,), context - 1, dtype=torch.int32, device="cuda")
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     sinks = torch.randn(heads, device="cuda") if sink else None
-    every = torch.empty(batch, heads * kv_heads * head_dim, dtype=torch.bfloat16, device="cuda") if mixed else out
+    every = torch.empty(batch, heads * kv_heads * head_dim, dtype=out.dtype, device="cuda") if mixed else out
     mix = torch.eye(heads, device="cuda")
     if chunk:                                           # a chunked mask travels as a negative window
         window = -chunk
 
+    attend, kernel = _token_attention(ops, q, pool, stride, heads, kv_heads, head_dim, context, mixed)
+
     def run(i):
         layer = i % layers
-        ops.paged_attention_decode(q, every, pool[:, layer, 0], pool[:, layer, planes - 1], stride, token_item, positions,
-                                   table, heads, kv_heads, head_dim, page, window, head_dim ** -0.5, context,
-                                   status=status, softcap=softcap, sink=sinks, all_values=mixed)
+        attend(q, every, pool[:, layer, 0], pool[:, layer, planes - 1], stride, token_item, positions, table, heads, kv_heads, head_dim,
+               page, window, head_dim ** -0.5, context, status=status, softcap=softcap, sink=sinks, all_values=mixed)
         if mixed:
             ops.head_mix(every, mix, out, heads, kv_heads, head_dim)
 
     if as_rows:
+        kernel = "heads as rows"
+
         def run(i):
             layer = i % layers
             ops.attention_rows(q, out, pool[:, layer, 0], pool[:, layer, planes - 1], stride, token_item, positions, table,
@@ -173,7 +190,7 @@ def time_decode_attention(batch, context, heads, kv_heads, head_dim, page=16, wi
     if chunk:
         seen = (context - 1) % chunk + 1
     nbytes = batch * seen * kv_heads * head_dim * 2 * planes
-    return {"us": seconds * 1e6, "gbs": nbytes / seconds / 1e9, "status": int(status.item())}
+    return {"us": seconds * 1e6, "gbs": nbytes / seconds / 1e9, "kernel": kernel, "status": int(status.item())}
 
 
 def time_prefill_attention(prompts, prompt_len, heads, kv_heads, head_dim, page=16, window=None, softcap=None,
