@@ -2,7 +2,7 @@
 // of 4; smaller than 64 are filled up with zeros).  Cache layout, masks, cap, sink and all_values as in attention_f32.cu, whose kernels take
 // the other sizes and the single tokens.
 //
-// Queries, keys, values and weights are cut into three bfloat16 pieces each (an exact sum), and six of the nine products of two numbers'
+// Queries, keys, values and weights are cut into three bfloat16 pieces each, and six of the nine products of two numbers'
 // pieces are formed, the small ones first, as in gemm_f32_tc.cu (which says what the terms left out and the sums that tcgen05 cuts off amount to).
 // One CTA per (128 queries of an entry, head), key tiles of 128 aligned to absolute positions:
 //
@@ -15,7 +15,7 @@
 // tile's keys and values are cut into pieces; its scores are queued behind.
 //
 // Infinities and NaNs: a value that is not finite counts as zero in the product (0 * infinity would reach rows that do not see it), and a row
-// that sees one, or whose sums are not finite, is computed again at the end, term by term.
+// that sees one, or whose results are not finite or below 2^-80, is computed again at the end, term by term.
 //
 // The order of a row's sums depends on its position alone (reference: src/model/paged_attention.py:262-295).
 //
@@ -409,7 +409,7 @@ prompt_attention_f32_tc_kernel(const float* __restrict__ q, int q_stride, float*
 #pragma unroll
         for (int d = 0; d < 16; ++d) {
             o[d] *= scale_out;
-            again |= !finite(o[d]);
+            again |= doubtful(o[d]);
         }
         if (again || *infinities) {
             const Call call{q, k_pool, v_pool, sink_h, out, page_stride, to_value, bt, q_stride, out_stride, head_dim, shift, g, scale, softcap};

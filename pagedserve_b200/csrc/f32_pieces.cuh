@@ -1,4 +1,4 @@
-// Float32 operands on the tensor cores: numbers as exact sums of three bfloat16 numbers, and what their kernels (gemm_f32_tc.cu,
+// Float32 operands on the tensor cores: numbers as sums of three bfloat16 numbers, and what their kernels (gemm_f32_tc.cu,
 // attention_f32_tc.cu) need of barriers, tensor memory and tcgen05.
 #pragma once
 #include <cuda.h>
@@ -90,9 +90,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Two numbers as three pairs of bfloat16 numbers that add up to them exactly.  The first pieces are cut off, not rounded (a number near the
-// largest float would round to an infinity); what is left has 16 bits, the second pieces are rounded to 8 of them, with
-// what is left then of 8 bits and either sign: the terms that the products leave out have no sign in common.
+// Two numbers as three pairs of bfloat16 numbers that add up to them: exactly from 2^-110 on; of a smaller one the third piece loses what is
+// below 2^-133, the smallest bfloat16 number.  The first pieces are cut off, not rounded (a number near the largest float would round to an
+// infinity); what is left has 16 bits, the second pieces are rounded to 8 of them, with what is left then of 8 bits and either sign: the terms
+// that the products leave out have no sign in common.  A second piece is at most 2^-7 of its number's power of two, a third one 2^-16, so
+// that those terms (second by third and third by third) are below 2^-22 of a product (the worst found is 3.9 * 2^-24).
 __device__ __forceinline__ void split(float x, float y, uint32_t& first, uint32_t& second, uint32_t& third) {
     const unsigned long long minus = pair_of(-1.f, -1.f);
     const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
@@ -104,6 +106,14 @@ __device__ __forceinline__ void split(float x, float y, uint32_t& first, uint32_
     rest = pair_fma(pair_of(__uint_as_float(second << 16), __uint_as_float(second & 0xffff0000u)), minus, rest);
     pair_split(rest, x, y);
     third = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
+
+// Whether a result has to be formed again term by term: one that is not finite (an infinity or a NaN among the operands, or an overflow), and one
+// so small that the third pieces behind it may have lost bits (products of numbers below 2^-110 by ones up to 2^19, sums of up to 2^11 of them;
+// on their own such sums were up to 1.4e-4 off at 2^-122, and from 2^-114 down further than multiply-adds).
+__device__ __forceinline__ bool doubtful(float v) {
+    const float size = fabsf(v);
+    return !(size <= 3.402823466e38f) || (size < 8.2718061e-25f /* 2^-80 */ && size > 0.f);
 }
 
 }  // namespace f32tc

@@ -1,7 +1,7 @@
 // float32 products of many rows on the tensor cores, to float32 accuracy: out[M,N] = epilogue(A[M,K] W[N,K]^T + bias).
 //
-// A float32 number is the sum of three bfloat16 numbers (24 bits of mantissa: 8 + 8 + 8), a = a0 + a1 + a2 exactly, and a product
-// of two is a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a1 b1 + a2 b0) but for terms below 2^-24 of it.  tcgen05.mma forms the six
+// A float32 number is the sum of three bfloat16 numbers (24 bits of mantissa: 8 + 8 + 8), a = a0 + a1 + a2, and a product
+// of two is a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a1 b1 + a2 b0) but for terms below 2^-22 of it, of either sign (f32_pieces.cuh).  tcgen05.mma forms the six
 // bfloat16 products exactly and adds them up in float32.  It cuts its sums off instead of rounding them (64 x 64 x 16 terms after
 // one another: 1 + 0.75 * 2^-23 gives 1), an error that grows with every MMA on one accumulator: over K = 768 of normal numbers 7.4e-7 of the
 // result's size, where float32 additions one after the other are off by 2.1e-7.  So an accumulator takes 64 k's only, the small
@@ -23,8 +23,8 @@
 // 152 / 51, 2,048 x 768 x 3,072 259 / 80 (121 TFLOP/s), 384 x 2,304 x 768 41 / 17, 651 x 1,024 x 1,024 53 / 20, 17 x 768 x 768 10.4 / 9.3.  With stages
 // of 32 k's (half as much work between barriers, twice the additions of accumulators) 70 / 112 in the first two.
 //
-// Infinities and NaNs: the pieces of an infinity are an infinity and NaNs.  A result that is not finite is computed again, term by term,
-// from the operands themselves.
+// Infinities and NaNs: the pieces of an infinity are an infinity and NaNs.  A result that is not finite, or below 2^-80, is computed again, term by
+// term, from the operands themselves.
 //
 // Stands where the reference has cuBLAS nn.Linear calls in float32 (src/model/paged_decoder.py:49-50, 178-179, 295-299).
 #include "f32_pieces.cuh"
@@ -37,7 +37,8 @@ constexpr int SLOT = 32;                                         // k's of a slo
 constexpr int RAW = 4, OPS = 2;                                  // slots of float32 operands, stages of pieces
 constexpr int SPLITTERS = 16;                                    // warps that form pieces and sums
 constexpr int THREADS = 128 + 32 * SPLITTERS;
-// Registers: 96 a thread at launch (five warps a scheduler), of which the first warps, which only issue, hand most to the splitters.
+// Registers: 96 a thread at launch (five warps a scheduler), of which the first warps, which only issue, hand most to the splitters.  (The
+// compiler keeps to the 96 all the same and spills 17 words.)
 constexpr int REGS = 96, FEW_REGS = 32, MANY_REGS = 112;
 static_assert(128 * FEW_REGS + 32 * SPLITTERS * MANY_REGS <= THREADS * REGS, "no more than the block was launched with");
 constexpr int OPERAND = BM * SLOT * 4, RAW_BYTES = 2 * OPERAND;
@@ -49,12 +50,12 @@ static_assert(2 * RESULTS * 4 <= RAW * RAW_BYTES + OPS * OPS_BYTES, "results lie
 constexpr float FIXED = 7.f, PER_SPLIT = .3f, PER_STAGE = 1.44f;  // microseconds of a CTA, measured
 constexpr int TMEM_COLS = 512, TMEM_A = 256;                     // accumulators at columns 0 and 128, pieces of A from 256, 128 a stage
 
-// the sums of up to `count` of four neighbouring columns that are not finite again, one product after the other
+// the doubtful ones among the sums of up to `count` of four neighbouring columns again, one product after the other
 __device__ __noinline__ float4 plain_dots(float4 sums, const float* a, const float* w, int ldw, int K, int count) {
     float v[4] = {sums.x, sums.y, sums.z, sums.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (j >= count || fabsf(v[j]) <= 3.402823466e38f) continue;
+        if (j >= count || !doubtful(v[j])) continue;
         v[j] = 0.f;
 #pragma unroll 1
         for (int k = 0; k < K; ++k) v[j] = fmaf(a[k], w[(size_t)j * ldw + k], v[j]);
@@ -306,9 +307,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     if (q > 0 && splits < parts) add(ld_cluster_f32x4(results + RESULTS + r * PITCH, q));
                 }
             }
-            // an infinity or a NaN among the operands, or an overflow
-            const float size = fmaxf(fmaxf(fabsf(sums.x), fabsf(sums.y)), fmaxf(fabsf(sums.z), fabsf(sums.w)));
-            if (!(size <= 3.402823466e38f) || sums.x != sums.x || sums.y != sums.y || sums.z != sums.z || sums.w != sums.w)
+            if (doubtful(sums.x) || doubtful(sums.y) || doubtful(sums.z) || doubtful(sums.w))
                 sums = plain_dots(sums, pdl_fresh(A) + (size_t)(m0 + r) * lda, W + (size_t)n * ldw, ldw, K, N - n);
             if (bias && (accumulate & PS_COLUMN_FACTOR)) { sums.x *= column.x; sums.y *= column.y; sums.z *= column.z; sums.w *= column.w; }
             else if (bias) { sums.x += column.x; sums.y += column.y; sums.z += column.z; sums.w += column.w; }

@@ -100,6 +100,34 @@ def test_infinities_and_nans():
         assert torch.allclose(out[20][finite[20]], plain[20][finite[20]], rtol=1e-3)
 
 
+@pytest.mark.parametrize("power", [-60, -100, -108, -112, -116, -120, -124])
+def test_small_numbers(power):
+    """Rows whose third pieces end below the smallest bfloat16 number: no further from 64 bits than multiply-adds, rows of zeros stay zeros."""
+    from test_f32_kernels_gpu import Step, plain
+
+    ops, g = ops_for(), torch.Generator().manual_seed(1)
+    a, w = torch.randn(140, 768, generator=g).to(DEV) * 2.0 ** power, torch.randn(130, 768, generator=g).to(DEV)
+    a[7], a[8] = 0.0, a[8] * 2.0 ** 30
+    want, errors = a.double() @ w.double().T, []
+    size = want.abs().amax(1, keepdim=True).clamp_min(1e-300)
+    for run in (ops.linear_f32_tc, ops.linear_simt):
+        out = torch.empty(140, 130, device=DEV)
+        run(a, w, None, out)
+        errors.append(float(((out.double() - want) / size).norm()))
+        assert bool((out[7] == 0).all())
+    assert errors[0] <= errors[1], errors
+    step, errors = Step([(200, 200)], 2, 2, 64, page=16, seed=7), []
+    step.layer.v_pool.mul_(2.0 ** power)
+    step.v = [v * 2.0 ** power for v in step.v]
+    q, want = step.q[0].reshape(200, -1).to(DEV), plain(step, 0.125, 0, 0.0, None, False)
+    for heads in (ops.F32_TC_HEADS, (1, 0)):
+        ops.F32_TC_HEADS = heads
+        out = torch.empty(200, 128, device=DEV)
+        ops.attention_f32(q, out, step.ctx, step.layer, 2, 2, 64, 0, 0.125)
+        errors.append(float((out.cpu().double() - want).norm() / want.norm()))
+    assert errors[0] <= 1.5 * errors[1], errors
+
+
 def test_products_in_a_row():
     """Products launched one behind the other, each reading what the one before wrote: the weights among it where they may be."""
     ops, g = ops_for(), torch.Generator().manual_seed(2)
