@@ -196,7 +196,8 @@ struct Layout {
     __host__ __device__ static constexpr int p_col(int half) { return P_COL + half * (SHARED ? COLS : COLS / 2); }
 };
 
-// CAPPED: scores go through the cap (instances of their own: the others would spill registers)
+// CAPPED: scores go through the cap (instances of their own, so that the others hold none of its code).  With two CTAs on an SM, 168 or 96 registers
+// a thread, all of them spill a little: 13 and 9 words without a cap (heads of 128, 64), 33 and 17 with one.
 template <int HD, int SPLIT, bool CAPPED, int RESIDENT>
 __global__ void __launch_bounds__(64 + 128 * SPLIT, RESIDENT)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,

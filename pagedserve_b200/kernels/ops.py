@@ -399,8 +399,8 @@ class Ops:
     F32_FEW_ROWS = 16             # most rows of a float32 product that run on the kernel that streams the weights once
 
     def linear_f32_rows(self, a, w, bias, out, act=None, accumulate=False):
-        """The float32 product of at most F32_FEW_ROWS rows (csrc/gemm_simt.cu: gemm_f32_rows_kernel).  ``w`` must have been
-        complete before the kernel in front began: it is read before that one has ended."""
+        """The float32 product of at most F32_FEW_ROWS rows (csrc/gemm_simt.cu: gemm_f32_rows_kernel).  ``w`` and ``bias`` must have
+        been complete before the kernel in front began: they are read before that one has ended."""
         M, K = a.shape
         N = w.shape[0]
         if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
@@ -450,7 +450,9 @@ class Ops:
     def _f32_tc_ok(a, w, out):
         """Whether a float32 product of more than F32_FEW_ROWS rows runs on the tensor cores.  By the shape of ``w`` and alignment, not by
         the rows: a row's bits are then those of the row alone in any larger step.  From 17 rows on it is the faster one at K of 768
-        (17 x 768 x 768: 9.3 us, multiply-adds 10.4); the multiply-adds' time falls with K, here 7 us stay."""
+        (17 x 768 x 768: 9.3 us, multiply-adds 10.4); the multiply-adds' time falls with K, here 7 us stay.  At the line itself, K of 640,
+        products of a tile or a few lose (128 x 592 x 640 10.6, multiply-adds 9.3; 40 x 768 x 640 9.6 / 9.0) what many tiles gain several times over.
+        (Below it products of thousands of rows stay on multiply-adds; the kernel takes K from 256 on.)"""
         return (a.shape[1] >= 640 and w.shape[0] >= 64 and a.shape[1] % 4 == 0 and a.dtype == w.dtype == out.dtype == torch.float32
                 and a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1 and a.stride(0) % 4 == 0
                 and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -913,10 +915,11 @@ class Ops:
     @staticmethod
     def attention_lanes_ok(q, tokens, k_pool, v_pool, page_stride, head_dim, columns, max_kv_len):
         """Whether the first ``tokens`` rows (``columns`` results each) run on :meth:`attention_lanes`: 16-byte pieces of rows, lanes that
-        hold a whole row (head sizes of 40 to 64, or 128), and contexts that one CTA walks through in the time that the split keys of
-        :meth:`paged_attention_decode` take, or pairs of token and result enough to fill the SMs.  Us, split / here: 12 heads of 64, 1
-        token, 1,200 keys 8.5 / 6.8, 4,000 7.9 / 19.0, 8 tokens 29.7 / 33.8, 32 tokens, 1,500 keys 66 / 38, 4,000 93.5 / 92.9; 16 heads of 128, 1
-        token, 1,200 keys 7.3 / 12.6, 8 tokens 23.7 / 15.3, 64 tokens 109 / 102; 8 heads of 80, 64 tokens, 300 keys 22.9 / 25.2.
+        hold a whole row (head sizes of 40 to 64, of which the engine sends 48 and 64 here, or 128), and contexts that one CTA walks
+        through in the time that the split keys of :meth:`paged_attention_decode` take, or pairs of token and result enough to fill the
+        SMs.  Us, split / here: 12 heads of 64, 1 token, 1,200 keys 8.5 / 6.8, 4,000 7.9 / 19.0, 8 tokens 29.7 / 33.8, 32 tokens, 1,500 keys
+        66 / 38, 4,000 93.5 / 92.9; 16 heads of 128, 1 token, 1,200 keys 7.3 / 12.6, 8 tokens 23.7 / 15.3, 64 tokens 109 / 102; 8 heads of 80,
+        64 tokens, 300 keys 22.9 / 25.2.
         One long context among short ones, which one CTA walks (32 tokens of 12 heads, one of 1,000 among 150s 15.1 / 15.5, 8,000 69 / 71): heads
         of 128 with 149 to 296 pairs lose there what they gain where all are long (12 tokens of 16 heads, one of 1,000 among 60s 12.4 / 19.5,
         all of 750 22.7 / 18.4) and run here to 512 keys only (6.7 / 6.9 with one of 240, 13.5 / 7.9 with all); with fewer the difference is

@@ -119,6 +119,10 @@ def attention(ops, q, out, ctx, layer, n_heads, n_kv_heads, head_dim, window, sc
         if ops.prefill_tc_ok(head_dim, layer.page_size, q, every, getattr(layer, "pool", None)):
             # Two threads per query row halve the chain of each 128-key tile but leave one CTA per SM: worth it
             # when all blocks are resident at once, or nearly so while some block runs over many tiles.
+            # Us, two CTAs / one: 128 blocks of heads of 128, 1,024 keys 21.7 / 19.7, with a cap 30.6 / 23.9; 256 blocks 25.7 / 25.4 and 35.6 / 29.0;
+            # 384 blocks 30.6 / 39.0 and 41.6 / 47.1; 256 keys, 192 blocks 13.9 / 16.3 and 16.8 / 17.5.  Over 48 to 432 blocks, 256 to 2,048 keys, heads
+            # of 64 and 128, with and without a cap the choice is within 8 % of the better one but for 288 blocks of 768 and more keys
+            # (heads of 64 19.5 / 25.0, 128 24.1 / 28.2) and heads of 128 with a cap, 160 to 192 blocks of 512 keys (20.2 / 17.2).
             # (an entry of b blocks of 64 queries has at most (b + 1) / 2 of 128)
             most_blocks = (ctx.num_long_blocks + long_items) // 2
             blocks = -(-ctx.num_long_blocks // 2) * columns          # near enough the 128-query blocks of all heads
