@@ -37,8 +37,8 @@ __device__ __forceinline__ void unpack(const uint4& raw, float (&x)[8]) {
     }
 }
 
-template <int HD, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : 1)
+template <int HD, int WARPS, int RESIDENT>
+__global__ void __launch_bounds__(WARPS * 32, RESIDENT)
 attention_lanes_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_bfloat16* __restrict__ out, int out_stride,
                        const __nv_bfloat16* __restrict__ k_pool, const __nv_bfloat16* __restrict__ v_pool, long long page_stride,
                        const int* __restrict__ token_item, const int* __restrict__ token_row, const int* __restrict__ positions,
@@ -180,12 +180,12 @@ attention_lanes_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_b
     }
 }
 
-template <int HD, int WARPS>
+template <int HD, int WARPS, int RESIDENT>
 int launch(const void* q, int q_stride, void* out, int out_stride, const void* k_pool, const void* v_pool, long long page_stride,
            const int* token_item, const int* token_row, const int* positions, const int* block_table, int bt_stride, const int* q_start,
            const int* kv_len, int T, int n_heads, int n_kv_heads, int head_dim, int page_size, int window, float scale, float softcap,
            const float* sink, int all_values, int wide, cudaStream_t s) {
-    return launch_pdl(attention_lanes_kernel<HD, WARPS>, dim3(T, all_values ? n_heads * n_kv_heads : n_heads), dim3(WARPS * 32), 0, s,
+    return launch_pdl(attention_lanes_kernel<HD, WARPS, RESIDENT>, dim3(T, all_values ? n_heads * n_kv_heads : n_heads), dim3(WARPS * 32), 0, s,
                       (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, (const __nv_bfloat16*)k_pool,
                       (const __nv_bfloat16*)v_pool, page_stride, token_item, token_row, positions, block_table, bt_stride, q_start, kv_len,
                       n_heads, n_kv_heads, head_dim, 31 - __builtin_clz(page_size), window, scale * 1.4426950408889634f,
@@ -210,20 +210,33 @@ PS_EXPORT int ps_attention_lanes(const void* q, int q_stride, void* out, int out
     if (page_size <= 0 || (page_size & (page_size - 1)) || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15)) return PS_ERR_UNSUPPORTED;
     if (warps != 0 && warps != 4 && warps != 8 && warps != 16) return PS_ERR_BAD_ARGUMENT;
     // As many warps as leave all CTAs resident (heads of 64, us with 16 / 8 / 4 warps: 96 pairs of token and head, 300 keys each 5.3 / 5.6 / 7.5; 192
-    // pairs 9.9 / 6.4 / 7.7; 384 pairs, 150 keys 10.3 / 9.5 / 6.3; 768 pairs 20.0 / 14.8 / 8.5).  Where contexts may be long, one long one among
-    // short ones decides, which more warps walk faster: 300 to 592 pairs take 8 there (384 pairs, one context of 1,000 among 150s 14.6 / 15.5 / 19.4,
-    // a fourth of them 15.8 / 16.7 / 20.9, all of 1,000 25.2 / 26.1 / 23.4; 480 pairs 17.5 / 16.0 / 20.5, 19.1 / 17.6 / 25.2, 33.0 / 27.2 / 32.6), and heads
-    // of 128, whose round has half as many keys, from short contexts on (512 pairs, 300 keys 26.5 / 19.1 / 21.5, one of 500 among 60s 16.5 / 14.7 / 19.0).
+    // pairs 9.9 / 6.4 / 7.7; 768 pairs, 150 keys 20.0 / 14.8 / 8.5).  Where contexts may be long, one long one among short ones decides, which more
+    // warps walk faster.
+    // 297 to 444 pairs take 8 beyond 256 keys, three CTAs on an SM.  384 pairs, us with three / with two on an SM / 4 warps: 30 keys each 3.0 / - / 2.2,
+    // 60 keys 3.4 / 5.0 / 3.7, 300 keys 8.5 / 12.7 / 9.1, all of 1,000 18.8 / 26.1 / 23.5; one of 500 among 60s 7.7 / 9.2 / 10.8, one of 1,000 among 60s
+    // 12.1 / 14 / 19.0, a fourth of 1,000 among 100s 16.6 / 16.7 / 20.8.  Beyond 1,280 keys two: a third takes more from the long ones than it gives (a
+    // fourth of 4,000 among 100s 57 / 45).
+    // 445 to 592 pairs take 4 where contexts end at 1,280 (480 pairs, 60 keys 5.7 with 8 warps, 4.3 with 4, 300 keys 13.2 / 12.0, one of 1,000 among 60s 14 / 19.3).
+    // Heads of 128, whose round has half as many keys, take 8 up to 592 pairs from short contexts on (384 pairs, 300 keys 12.6 / 17.8 / 15.1, one of 1,000
+    // among 60s 21.4 / 22 / 33.0; 512 pairs, two on an SM, 300 keys 19.1, with 4 warps 21.5, one of 500 among 60s 14.7 / 19.0).
     const long long pairs = (long long)T * n_heads * (all_values ? n_kv_heads : 1);
-    if (warps == 0) warps = pairs <= 148 ? 16 : pairs <= 296 || (pairs <= 592 && (max_kv_len > 512 || head_dim > 64)) ? 8 : 4;
-#define PS_LANES(HD, WARPS)                                                                                                               \
-    return ps::lanes::launch<HD, WARPS>(q, q_stride, out, out_stride, k_pool, v_pool, page_stride, token_item, token_row, positions,      \
+    const bool three = pairs > 296 && pairs <= 444 && max_kv_len <= 1280;
+    if (warps == 0) {
+        const bool large = head_dim > 64;
+        if (pairs <= 148) warps = 16;
+        else if (pairs <= 296) warps = 8;
+        else if (pairs <= 444) warps = large || max_kv_len > 256 ? 8 : 4;
+        else warps = pairs <= 592 && (large || max_kv_len > 1280) ? 8 : 4;
+    }
+#define PS_LANES(HD, WARPS, RESIDENT)                                                                                                     \
+    return ps::lanes::launch<HD, WARPS, RESIDENT>(q, q_stride, out, out_stride, k_pool, v_pool, page_stride, token_item, token_row, positions,      \
                                         block_table, bt_stride, q_start, kv_len, T, n_heads, n_kv_heads, head_dim, page_size, window,     \
                                         scale, softcap, sink, all_values, wide, (cudaStream_t)stream)
 #define PS_LANES_HEADS(HD)                                                                                                                \
-    if (warps == 16) PS_LANES(HD, 16);                                                                                                    \
-    if (warps == 8) PS_LANES(HD, 8);                                                                                                      \
-    PS_LANES(HD, 4)
+    if (warps == 16) PS_LANES(HD, 16, 1);                                                                                                 \
+    if (warps == 8 && three) PS_LANES(HD, 8, 3);                                                                                          \
+    if (warps == 8) PS_LANES(HD, 8, 2);                                                                                                   \
+    PS_LANES(HD, 4, 6)
     if (head_dim <= 64) { PS_LANES_HEADS(64); }
     PS_LANES_HEADS(128);
 #undef PS_LANES_HEADS

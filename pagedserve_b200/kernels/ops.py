@@ -920,7 +920,7 @@ class Ops:
         SMs.  Us, split / here: 12 heads of 64, 1 token, 1,200 keys 8.5 / 6.8, 4,000 7.9 / 19.0, 8 tokens 29.7 / 33.8, 32 tokens, 1,500 keys
         66 / 38, 4,000 93.5 / 92.9; 16 heads of 128, 1 token, 1,200 keys 7.3 / 12.6, 8 tokens 23.7 / 15.3, 64 tokens 109 / 102; 8 heads of 80,
         64 tokens, 300 keys 22.9 / 25.2.
-        One long context among short ones, which one CTA walks (32 tokens of 12 heads, one of 1,000 among 150s 15.1 / 15.5, 8,000 69 / 71): heads
+        One long context among short ones, which one CTA walks (32 tokens of 12 heads, one of 1,000 among 60s 13.7 / 12.1, 8,000 among 150s 69 / 71): heads
         of 128 with 149 to 296 pairs lose there what they gain where all are long (12 tokens of 16 heads, one of 1,000 among 60s 12.4 / 19.5,
         all of 750 22.7 / 18.4) and run here to 512 keys only (6.7 / 6.9 with one of 240, 13.5 / 7.9 with all); with fewer the difference is
         3 us against 8 (8 tokens 9.5 / 12.4, all of 750 19.2 / 11.7)."""

@@ -119,17 +119,18 @@ def test_numbers_that_are_not_finite(head_dim, warps, with_sink):
 
 def test_contexts_of_different_lengths():
     """Which kernel and how many warps run where one context may be far longer than the others: heads of 128 with 149 to 296 pairs
-    leave it beyond 512 keys, and 297 to 592 pairs take 8 warps (a number of warps has bits of its own)."""
+    leave it beyond 512 keys, and 297 and more pairs take 8 warps where contexts may be long (a number of warps has bits of its own)."""
     from test_kernels_gpu import PagedCase, ops_for
 
     ops, pool = ops_for(torch.bfloat16), torch.empty(8, 2, 8, 16, 128, dtype=torch.bfloat16, device=DEV)
     ok = lambda tokens, longest: ops.attention_lanes_ok(torch.empty(tokens, 1024, dtype=torch.bfloat16, device=DEV), tokens, pool[:, 0], pool[:, 1],
                                                         16384, 128, 8, longest)
     assert ok(18, 1024) and not ok(19, 1024) and not ok(37, 513) and ok(19, 512) and ok(37, 512) and ok(38, 1280) and ok(38, 8192) and not ok(37, 8192)
-    for heads, head_dim, longest, warps in ((1, 64, 1024, (16, 8, 8, 8, 4)), (1, 64, 512, (16, 8, 4, 4, 4)), (1, 128, 512, (16, 8, 8, 8, 4))):
+    for heads, head_dim, longest, warps in ((1, 64, 1024, (16, 8, 8, 8, 8, 4, 4, 4)), (1, 64, 512, (16, 8, 8, 8, 8, 4, 4, 4)), (1, 64, 256, (16, 8, 8, 4, 4, 4, 4, 4)),
+                                            (1, 64, 2048, (16, 8, 8, 8, 8, 8, 8, 4)), (1, 128, 512, (16, 8, 8, 8, 8, 8, 8, 4))):
         lengths = [500] + [20] * 9
         case = PagedCase(ops, torch.bfloat16, lengths, heads, 1, head_dim, 16, seed=1)
-        for tokens, expected in zip((148, 149, 297, 592, 593), warps):
+        for tokens, expected in zip((148, 149, 296, 297, 444, 445, 592, 593), warps):
             item = torch.arange(tokens, dtype=torch.int32, device=DEV) % len(lengths)
             positions = torch.tensor(lengths, dtype=torch.int32, device=DEV)[item.long()] - 1
             q = torch.randn(tokens, head_dim, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).to(DEV)
